@@ -62,15 +62,17 @@ template <class R> size_t fast_smem_bytes(int stride, int worlds_per_cta);
 // queue (two device ints, zero between launches) one wave of resident CTAs
 // takes groups of 32 worlds from it until none is left. tile in
 // 1 .. substeps - 1 (with tile_q: 13 x 4 floats per world): the control step
-// as launches of `tile` substeps each, the same worlds bit for bit.
+// as launches of `tile` substeps each, the same worlds bit for bit. alone
+// (false: the launch runs beside others, as a part of a control step in
+// parts): small batches may spread over more CTAs of fewer worlds each.
 cudaError_t launch_step_warps(const DevModel<float>& M, const Worlds<float>& W, const Actuation& A, float* spill,
                               int spill_per_lane, int lane_cap, const int* ids, int n_items, int* queue,
-                              cudaStream_t stream, int tile = 0, float* tile_q = nullptr);
+                              cudaStream_t stream, bool alone = true, int tile = 0, float* tile_q = nullptr);
 // The same step in FP64 (arc_step_warps64.cu): two CTAs per SM (its bodies
 // take twice the shared memory), the whole control step in one launch.
 cudaError_t launch_step_warps64(const DevModel<double>& M, const Worlds<double>& W, const Actuation& A,
                                 double* spill, int spill_per_lane, int lane_cap, const int* ids, int n_items,
-                                int* queue, cudaStream_t stream);
+                                int* queue, cudaStream_t stream, bool alone = true);
 constexpr int kFastOnChipContacts = 2;
 constexpr int kWarpsOnChipContacts = 1;  // keeps four CTAs of the warp-per-leg kernel per SM
 // the fewest on-chip records of any kernel: a spill area of lane_cap minus

@@ -581,20 +581,20 @@ template <> const DevModel<double>& dev_model<double>(const arc_sim* s) { return
 // the warp-per-leg step in the sim's precision (FP64: the whole control
 // step in one launch; substep tiles are FP32 only)
 template <class R> cudaError_t launch_warps(arc_sim*, const DevModel<R>&, const Worlds<R>&, const Actuation&,
-                                           const int*, int, int*, cudaStream_t);
+                                           const int*, int, int*, cudaStream_t, bool alone);
 template <> cudaError_t launch_warps<float>(arc_sim* s, const DevModel<float>& M, const Worlds<float>& W,
                                             const Actuation& A, const int* ids, int n_items, int* queue,
-                                            cudaStream_t st)
+                                            cudaStream_t st, bool alone)
 {
     return launch_step_warps(M, W, A, static_cast<float*>(s->spill), s->spill_per_lane, s->lane_cap, ids, n_items,
-                             queue, st, s->substep_tile, s->tile_q);
+                             queue, st, alone, s->substep_tile, s->tile_q);
 }
 template <> cudaError_t launch_warps<double>(arc_sim* s, const DevModel<double>& M, const Worlds<double>& W,
                                              const Actuation& A, const int* ids, int n_items, int* queue,
-                                             cudaStream_t st)
+                                             cudaStream_t st, bool alone)
 {
     return launch_step_warps64(M, W, A, static_cast<double*>(s->spill), s->spill_per_lane, s->lane_cap, ids,
-                               n_items, queue, st);
+                               n_items, queue, st, alone);
 }
 
 // ids: device list of n_ids distinct worlds to step (NULL: all worlds).
@@ -611,7 +611,7 @@ template <class R> int step_impl(arc_sim* s, const Actuation& A, cudaStream_t st
     const bool warps_ok = M.leaper && s->substeps <= kFastMaxSubsteps;
     cudaError_t e;
     if (warps_ok && (s->kernel == ARC_KERNEL_WARPS || (ids && s->kernel == ARC_KERNEL_LEGS)))
-        e = launch_warps<R>(s, M, W, A, ids, n_items, queue, st);
+        e = launch_warps<R>(s, M, W, A, ids, n_items, queue, st, part < 0);
     else if (!ids && s->kernel == ARC_KERNEL_LEGS && M.leaper && s->substeps <= kFastMaxSubsteps)
         e = launch_step_fast<R>(M, W, A, static_cast<R*>(s->spill), s->spill_per_lane, s->lane_cap, s->wpc, st);
     else
@@ -1494,14 +1494,14 @@ bool fused_applies(const arc_sim* s)
 // worlds into O's list (O.done_count zeroed first) and reset in the kernel
 // (fused == 2) or by the reset kernel after it (fused == 1).
 int env_control_step(arc_sim* s, const float* actions, const TaskOut& O, const int* ids, int n, int* queue,
-                     cudaStream_t st)
+                     cudaStream_t st, bool alone = true)
 {
     const bool resets = s->fused >= 2;
     if (check(s, cudaMemsetAsync(O.done_count, 0, sizeof(int), st), "memset done_count") ||
         check(s,
               launch_control_step(s->mf, s->rm, view<float>(s), (TerrainGeom<float>*)s->tg, s->tgd, s->grid_of,
                                   s->cell, s->tp, s->ts, O, actions, static_cast<float*>(s->spill),
-                                  s->spill_per_lane, s->lane_cap, ids, n, queue, resets, st),
+                                  s->spill_per_lane, s->lane_cap, ids, n, queue, resets, st, alone),
               "control step kernel"))
         return ARC_ERR_CUDA;
     if (resets)
@@ -1802,7 +1802,7 @@ template <class R> int env_step_chunk(arc_sim* s, int first, int count, int c, c
         return ARC_ERR_CUDA;
     if (fused_applies(s)) {
         int* queue = !s->use_queue ? nullptr : (part >= 0 ? s->part_queue + 2 * part : s->queue);
-        return env_control_step(s, s->actions, O, ids, count, queue, st);
+        return env_control_step(s, s->actions, O, ids, count, queue, st, part < 0);
     }
     Actuation A{nullptr, s->actions};
     if (int rc = step_any(s, A, st, ids, count, part))

@@ -205,7 +205,7 @@ __device__ __forceinline__ void joint_positions(P& bp, const BodyK<F>& kp, P& bc
 // the positional correction against the static world (solve_pos with no
 // second body and alpha = 0, :226-242). Returns 1 when the sphere touched.
 template <class Rec>
-__device__ __forceinline__ int collide(P& b, const BodyK<F>& k, V xprev, Q qprev, const SphereK<F>& sk,
+__device__ __forceinline__ int collide(P& b, const BodyK<F>& k, Ref body, const SphereK<F>& sk,
                                        SphereState<F>& ss, const TerrainView<F>& t, F inv_cell, const StepK<F>& st,
                                        Rec&& record)
 {
@@ -245,21 +245,47 @@ __device__ __forceinline__ int collide(P& b, const BodyK<F>& k, V xprev, Q qprev
     F ln = F(0), depth_max = F(0);
     V n_max{F(0), F(0), F(1)};
     int touched = 0, ix = ix0, iy = iy0;
+    // a box of at most 2 x 2 columns is scanned through the bits of `left`
+    // (column dx + 2 dy), a wider one column by column. The bits give the
+    // columns higher than the sphere's bottom at once: of the 9 columns that
+    // a lane's spheres span in a substep 0.6 are, and testing one per
+    // iteration cost a warp 22 iterations where 6 find them all (4,096
+    // worlds: 504 us against 527)
+    const bool wide = ix1 - ix0 > 1 || iy1 - iy0 > 1;
+    int left = 1 | (ix1 > ix0 ? 2 : 0) | (iy1 > iy0 ? 4 : 0) | (ix1 > ix0 && iy1 > iy0 ? 8 : 0);
 #pragma unroll 1
     for (;;) {
         V r, d, n{F(0), F(0), F(1)};
         F depth = F(0);
         bool contact = false;
 #pragma unroll 1
-        while (!contact && iy <= iy1) {
-            const int cx = ix, cy = iy;
-            if (++ix > ix1) {
-                ix = ix0;
-                ++iy;
+        while (!contact) {
+            int cx, cy;
+            F top;
+            if (wide) {
+                if (iy > iy1)
+                    break;
+                cx = ix;
+                cy = iy;
+                if (++ix > ix1) {
+                    ix = ix0;
+                    ++iy;
+                }
+                top = height(cx, cy);
+                if (c.z - rad >= top)
+                    continue;
+            } else {
+                const F low = c.z - rad;
+                const int below = left & ((low >= h00 ? 0 : 1) | (low >= h10 ? 0 : 2) | (low >= h01 ? 0 : 4) | (low >= h11 ? 0 : 8));
+                if (!below)
+                    break;
+                const int bit = below & -below;
+                left &= ~(2 * bit - 1);
+                const int dx = (bit & 10) ? 1 : 0, dy = (bit & 12) ? 1 : 0;
+                cx = ix0 + dx;
+                cy = iy0 + dy;
+                top = dy ? (dx ? h11 : h01) : (dx ? h10 : h00);
             }
-            const F top = height(cx, cy);
-            if (c.z - rad >= top)
-                continue;
             const F x0 = t.ox + F(cx) * t.cell, x1 = x0 + t.cell;
             const F y0 = t.oy + F(cy) * t.cell, y1 = y0 + t.cell;
             // edges and corners buried by an equal or higher neighbour
@@ -295,7 +321,7 @@ __device__ __forceinline__ int collide(P& b, const BodyK<F>& k, V xprev, Q qprev
             // friction, once, after the scan; c is the current centre
             const V p = madd(c, n_max, -rad);
             if (!ss.anchored || dot(n_max, ss.anchor_n) < F(0.9)) {
-                const V c0 = xprev + qrotate(qprev, sk.pos);
+                const V c0 = getv(body, kXP) + qrotate(getq(body, kQP), sk.pos);
                 ss.anchor = madd(c0, n_max, -rad);
                 ss.anchor_n = n_max;
                 ss.anchored = 1;
@@ -363,11 +389,30 @@ enum : uint32_t { OP_END = 0, OP_INT, OP_JNT, OP_COL, OP_UPD, OP_DMP, OP_CVL, OP
 // order. Warp 0 runs ahead of the others in issue priority: the torso's
 // work there makes the step 5% faster than the same lists with the torso
 // on warp 3.
-#define ARC_LEG_OPS(k)                                                                                         \
-    {ARC_OP(OP_INT, 1, 4, 0, 0), ARC_OP(OP_JNT, 0, 1, k, (k) + 1), ARC_OP(OP_JNT, 1, 2, 0, 0),                  \
-     ARC_OP(OP_UPD, 1, 2, 0, 0), ARC_OP(OP_DMP, 0, 1, 4 + (k), 5 + (k)), ARC_OP(OP_JNT, 2, 3, 0, 0),            \
-     ARC_OP(OP_COL, 1, 2, 0, 0), ARC_OP(OP_COL, 2, 6, 0, 0), ARC_OP(OP_UPD, 2, 4, 0, 0), ARC_OP(OP_DMP, 1, 3, 0, 0), \
-     ARC_OP(OP_CVL, 0, 0, 0, 0), OP_END}
+//
+// Two such lists, the same work in another order. While the chain is with
+// the later legs, a leg that is done with its torso joint has time to spare:
+// joints 3, 6 and 9 take 3.7k cycles each, a leg's third joint 3.9k, its
+// femur sphere 2.1k and its tibia's four spheres 13k (32 worlds, one CTA on
+// the SM, of 47k cycles a substep). kListLatency fills that wait: legs 0 and
+// 1 solve their third joint and collide the femur before their damping
+// joint, leg 2 its third joint, leg 3, whose damping joint comes at once,
+// nothing. It pays while an SM holds one or two CTAs (4,096 worlds: 527 us
+// against 579; 8,000: 509 against 531); with three or four the other CTAs
+// fill the waits and the damping chain's earlier start wins (16,384 worlds:
+// 945 against 984 us), so kListThroughput leaves all of it for later.
+#define ARC_LEG_HEAD(k)                                                                                        \
+    ARC_OP(OP_INT, 1, 4, 0, 0), ARC_OP(OP_JNT, 0, 1, k, (k) + 1), ARC_OP(OP_JNT, 1, 2, 0, 0),                   \
+        ARC_OP(OP_UPD, 1, 2, 0, 0)
+#define ARC_TORSO_HEAD                                                                                         \
+    ARC_OP(OP_INT, 0, 4, 0, 0), ARC_OP(OP_JNT, 0, 1, 0, 1), ARC_OP(OP_JNT, 1, 2, 0, 0), ARC_OP(OP_UPD, 1, 2, 0, 0)
+#define ARC_TORSO_DAMP ARC_OP(OP_COL, 0, 1, 4, 0), ARC_OP(OP_UPD, 0, 1, 0, 0), ARC_OP(OP_DMP, 0, 1, 0, 5)
+#define ARC_LEG_DAMP(k) ARC_OP(OP_DMP, 0, 1, 4 + (k), 5 + (k))
+#define ARC_JOINT3 ARC_OP(OP_JNT, 2, 3, 0, 0)
+#define ARC_FEMUR ARC_OP(OP_COL, 1, 2, 0, 0)
+#define ARC_LEG_TAIL                                                                                           \
+    ARC_OP(OP_COL, 2, 6, 0, 0), ARC_OP(OP_UPD, 2, 4, 0, 0), ARC_OP(OP_DMP, 1, 3, 0, 0), ARC_OP(OP_CVL, 0, 0, 0, 0)
+#define ARC_TORSO_TAIL ARC_OP(OP_CVL, 1, 0, 8, 0)
 // Capped lists: warp 0 owns the torso, whose sphere's contacts lead the
 // list as sphere 0 leads the reference's, and every lane's count is
 // published before any contact velocity.
@@ -377,27 +422,66 @@ enum : uint32_t { OP_END = 0, OP_INT, OP_JNT, OP_COL, OP_UPD, OP_DMP, OP_CVL, OP
      ARC_OP(OP_DMP, 0, 1, 4 + k, 5 + k), ARC_OP(OP_DMP, 1, 3, 0, 0), ARC_OP(OP_CVL, 0, 0, 0, 0), OP_END}
 
 constexpr int kMaxOps = 20;
-__constant__ uint32_t kOps[2][kWarps][kMaxOps] = {
-    {{ARC_OP(OP_INT, 0, 4, 0, 0), ARC_OP(OP_JNT, 0, 1, 0, 1), ARC_OP(OP_JNT, 1, 2, 0, 0), ARC_OP(OP_UPD, 1, 2, 0, 0),
-      ARC_OP(OP_COL, 0, 1, 4, 0), ARC_OP(OP_UPD, 0, 1, 0, 0), ARC_OP(OP_DMP, 0, 1, 0, 5), ARC_OP(OP_JNT, 2, 3, 0, 0),
-      ARC_OP(OP_COL, 1, 2, 0, 0), ARC_OP(OP_COL, 2, 6, 0, 0), ARC_OP(OP_UPD, 2, 4, 0, 0), ARC_OP(OP_DMP, 1, 3, 0, 0),
-      ARC_OP(OP_CVL, 0, 0, 0, 0), ARC_OP(OP_CVL, 1, 0, 8, 0), OP_END},
-     ARC_LEG_OPS(1), ARC_LEG_OPS(2), ARC_LEG_OPS(3)},
+enum : int { kListThroughput = 0, kListLatency = 1, kListCapped = 2 };
+__constant__ uint32_t kOps[3][kWarps][kMaxOps] = {
+    {{ARC_TORSO_HEAD, ARC_TORSO_DAMP, ARC_JOINT3, ARC_FEMUR, ARC_LEG_TAIL, ARC_TORSO_TAIL, OP_END},
+     {ARC_LEG_HEAD(1), ARC_LEG_DAMP(1), ARC_JOINT3, ARC_FEMUR, ARC_LEG_TAIL, OP_END},
+     {ARC_LEG_HEAD(2), ARC_LEG_DAMP(2), ARC_JOINT3, ARC_FEMUR, ARC_LEG_TAIL, OP_END},
+     {ARC_LEG_HEAD(3), ARC_LEG_DAMP(3), ARC_JOINT3, ARC_FEMUR, ARC_LEG_TAIL, OP_END}},
+    {{ARC_TORSO_HEAD, ARC_JOINT3, ARC_FEMUR, ARC_TORSO_DAMP, ARC_LEG_TAIL, ARC_TORSO_TAIL, OP_END},
+     {ARC_LEG_HEAD(1), ARC_JOINT3, ARC_FEMUR, ARC_LEG_DAMP(1), ARC_LEG_TAIL, OP_END},
+     {ARC_LEG_HEAD(2), ARC_JOINT3, ARC_LEG_DAMP(2), ARC_FEMUR, ARC_LEG_TAIL, OP_END},
+     {ARC_LEG_HEAD(3), ARC_LEG_DAMP(3), ARC_JOINT3, ARC_FEMUR, ARC_LEG_TAIL, OP_END}},
     {{ARC_OP(OP_INT, 0, 2, 0, 0), ARC_OP(OP_JNT, 0, 1, 0, 1), ARC_OP(OP_INT, 2, 4, 0, 0), ARC_OP(OP_JNT, 1, 3, 0, 0),
       ARC_OP(OP_COL, 0, 1, 4, 0), ARC_OP(OP_UPD, 0, 1, 0, 0), ARC_OP(OP_COL, 1, 2, 0, 0), ARC_OP(OP_COL, 2, 6, 0, 0),
       ARC_OP(OP_UPD, 1, 4, 0, 0), ARC_OP(OP_CNT, 0, 0, 0, 0), ARC_OP(OP_DMP, 0, 1, 0, 5), ARC_OP(OP_DMP, 1, 3, 0, 0),
       ARC_OP(OP_CVL, 0, 0, 0, 0), ARC_OP(OP_CVL, 1, 0, 8, 0), OP_END},
      ARC_CAPPED_OPS(1), ARC_CAPPED_OPS(2), ARC_CAPPED_OPS(3)}};
-#undef ARC_LEG_OPS
+#undef ARC_LEG_HEAD
+#undef ARC_TORSO_HEAD
+#undef ARC_TORSO_DAMP
+#undef ARC_LEG_DAMP
+#undef ARC_JOINT3
+#undef ARC_FEMUR
+#undef ARC_LEG_TAIL
+#undef ARC_TORSO_TAIL
 #undef ARC_CAPPED_OPS
 #undef ARC_OP
 
 // ---------------------------------------------------------------------------
 
 
-// One control step of the 32 worlds of group `group` (items group * 32 ..
-// group * 32 + 31: worlds ids[item], or item itself without ids) by a CTA of
-// kThreads threads, thread tid = lane j of warp `leg`. On return the
+// How a launch over n_items worlds is split: worlds per group (one CTA's
+// lanes) and the operation list.
+//   Worlds per group. A group's time is that of the longest path over its
+// worlds' contacts, so with fewer groups than SMs smaller groups are faster:
+// 64 worlds take 353 us one per group and 408 us as two groups of 32, 1,000
+// worlds 404-418 us in groups of 7-14 and 443 us in groups of 32. Groups
+// beyond about half the SMs gain little more and crowd out what runs beside
+// the step, so the split stops there; and a launch that shares the GPU with
+// others (`alone` false) keeps groups of 32.
+//   Operation list: kListLatency up to two groups per SM in FP32, up to one
+// in FP64, whose SMs hold two (4,096 worlds: 758 us against 848; 7,000:
+// 1,119 against 1,069).
+struct GroupPlan {
+    int per_group, groups, list;
+};
+inline GroupPlan group_plan(int n_items, int sms, bool alone)
+{
+    const int spread = sms / 2 > 0 ? sms / 2 : 1;
+    GroupPlan p;
+    p.per_group = kWorlds;
+    if (alone && n_items < spread * kWorlds)
+        p.per_group = (n_items + spread - 1) / spread;
+    p.groups = (n_items + p.per_group - 1) / p.per_group;
+    p.list = alone && p.groups <= (sizeof(F) == 4 ? 2 : 1) * sms ? kListLatency : kListThroughput;
+    return p;
+}
+
+// One control step of the worlds of group `group` (items group * per_group
+// .. + per_group - 1, at most 32: worlds ids[item], or item itself without
+// ids) by a CTA of kThreads threads, thread tid = lane j of warp `leg`, in
+// the order of the operation list `list`. On return the
 // worlds' records, flags, time and unstable marks are written and every
 // thread of the CTA has passed the group's last barrier.
 //
@@ -411,12 +495,12 @@ __constant__ uint32_t kOps[2][kWarps][kMaxOps] = {
 __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const Worlds<F>& W, const Actuation& A,
                                            F* __restrict__ spill, int spill_per_lane, int lane_cap,
                                            const int* __restrict__ ids, int n_items, int group, int tid, int leg,
-                                           int j, int sub0, int sub1, F* __restrict__ tile_q)
+                                           int j, int sub0, int sub1, F* __restrict__ tile_q, int per_group, int list)
 {
     (void)tid;
     const bool first_tile = sub0 == 0, last_tile = sub1 >= M.substeps;
-    const int item = group * kWorlds + j;
-    const int world = item < n_items ? (ids ? ids[item] : item) : -1;
+    const int item = group * per_group + j;
+    const int world = j < per_group && item < n_items ? (ids ? ids[item] : item) : -1;
     const bool valid = world >= 0 && world < W.n;
     const int wi = valid ? world : 0;
 
@@ -496,7 +580,7 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
         if (leg == 0)
             touches |= (unsigned long long)(sphr[0] & 1023u) << 50;
     }
-    const uint32_t* ops = &kOps[capped ? 1 : 0][leg][0];
+    const uint32_t* ops = &kOps[capped ? (int)kListCapped : list][leg][0];
     int last_nc = 0;  // this lane's contact records in the last substep
     __syncthreads();
 
@@ -583,14 +667,12 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
                     const BodyK<F>& k = M.body[bid];
                     P pose;
                     load_pose(r, k, pose);
-                    const V xp = getv(r, kXP);
-                    const Q qp = getq(r, kQP);
 #pragma unroll 1
                     for (int s = a; s < b; ++s) {
                         const int bit = s == 0 ? 5 : s - 1;
                         const Ref ra{s == 0 ? &sm.torso[kBodyF][j] : &sm.anch[leg][6 * (s - 1)][j]};
                         SphereState<F> ss{getv(ra, 0), getv(ra, 3), (int)((anch >> bit) & 1u)};
-                        const int t = collide(pose, k, xp, qp, M.sphere[s == 0 ? 0 : 5 * leg + s], ss, T, inv_cell, st,
+                        const int t = collide(pose, k, r, M.sphere[s == 0 ? 0 : 5 * leg + s], ss, T, inv_cell, st,
                                                      [&](V l, V n) { record(bid, l, n); });
                         touches += (unsigned long long)t << (10 * bit);
                         anch = (anch & ~(1u << bit)) | ((uint32_t)(ss.anchored != 0) << bit);

@@ -22,12 +22,13 @@ struct Smem64 {
 
 __global__ void __launch_bounds__(wl::kThreads, 2)
 k_step_warps64(const __grid_constant__ DevModel<double> M, Worlds<double> W, Actuation A, double* __restrict__ spill,
-               int spill_per_lane, int lane_cap, const int* __restrict__ ids, int n_items, int* queue)
+               int spill_per_lane, int lane_cap, const int* __restrict__ ids, int n_items, int* queue,
+               int per_group, int list)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem64& sm = *reinterpret_cast<Smem64*>(smem_raw);
     const int tid = threadIdx.x, leg = tid / wl::kWorlds, j = tid % wl::kWorlds;
-    const int n_groups = (n_items + wl::kWorlds - 1) / wl::kWorlds;
+    const int n_groups = (n_items + per_group - 1) / per_group;
     // with a queue every group, the first included, is taken from it
     int first = blockIdx.x;
     if (queue) {
@@ -39,7 +40,7 @@ k_step_warps64(const __grid_constant__ DevModel<double> M, Worlds<double> W, Act
 #pragma unroll 1
     for (int group = first; group < n_groups;) {
         wl::step_group(sm.step, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, group, tid, leg, j, 0,
-                       M.substeps, nullptr);
+                       M.substeps, nullptr, per_group, list);
         if (!queue)
             break;
         __syncthreads();
@@ -66,7 +67,7 @@ k_step_warps64(const __grid_constant__ DevModel<double> M, Worlds<double> W, Act
 
 cudaError_t launch_step_warps64(const DevModel<double>& M, const Worlds<double>& W, const Actuation& A,
                                 double* spill, int spill_per_lane, int lane_cap, const int* ids, int n_items,
-                                int* queue, cudaStream_t stream)
+                                int* queue, cudaStream_t stream, bool alone)
 {
     if (W.n <= 0 || n_items <= 0)
         return cudaSuccess;
@@ -76,7 +77,7 @@ cudaError_t launch_step_warps64(const DevModel<double>& M, const Worlds<double>&
     // per device: the shared-memory attribute, and how many CTAs are resident
     // at once (the work queue's wave)
     static std::atomic<unsigned long long> configured{0};
-    static int resident[64] = {};
+    static int resident[64] = {}, sm_count[64] = {};
     cudaError_t e = once_per_device(configured, [&](int dev) {
         cudaError_t r = cudaFuncSetAttribute(k_step_warps64, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int sms = 0, per_sm = 0;
@@ -85,21 +86,19 @@ cudaError_t launch_step_warps64(const DevModel<double>& M, const Worlds<double>&
         if (r == cudaSuccess)
             r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_warps64, wl::kThreads, smem);
         if (r == cudaSuccess)
-            resident[dev] = sms * (per_sm > 0 ? per_sm : 1);
+            resident[dev] = sms * (per_sm > 0 ? per_sm : 1), sm_count[dev] = sms;
         return r;
     });
     if (e != cudaSuccess)
         return e;
-    const int groups = (n_items + wl::kWorlds - 1) / wl::kWorlds;
-    int grid = groups;
-    if (queue) {
-        int dev = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess)
-            return e;
-        grid = groups < resident[dev] ? groups : resident[dev];  // one wave of resident CTAs
-    }
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess)
+        return e;
+    const wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone);
+    // with a queue, one wave of resident CTAs
+    const int grid = queue && plan.groups > resident[dev] ? resident[dev] : plan.groups;
     k_step_warps64<<<grid, wl::kThreads, smem, stream>>>(M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
-                                                         queue);
+                                                         queue, plan.per_group, plan.list);
     return cudaGetLastError();
 }
 

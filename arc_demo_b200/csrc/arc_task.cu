@@ -801,12 +801,12 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
                TerrainGeom<float>* tg, TerrainGeomD* tgd, const int* __restrict__ grid_of, double cell,
                const __grid_constant__ TaskParams P, TaskState S, TaskOut O, Actuation A,
                float* __restrict__ spill, int spill_per_lane, int lane_cap, const int* __restrict__ ids, int n_items,
-               int* queue, int sub0, int sub1, float* __restrict__ tile_q)
+               int* queue, int sub0, int sub1, float* __restrict__ tile_q, int per_group, int list)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ControlSmem& cs = *reinterpret_cast<ControlSmem*>(smem_raw);
     const int tid = threadIdx.x, leg = tid / wl::kWorlds, j = tid % wl::kWorlds;
-    const int n_groups = (n_items + wl::kWorlds - 1) / wl::kWorlds;
+    const int n_groups = (n_items + per_group - 1) / per_group;
     auto world_of = [&](int item) {
         const int w = item < n_items ? (ids ? ids[item] : item) : -1;
         return w >= 0 && w < W.n ? w : -1;
@@ -825,7 +825,7 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
 #pragma unroll 1
     for (int group = first; group < n_groups;) {
         wl::step_group(cs.step, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, group, tid, leg, j, sub0, sub1,
-                       tile_q);
+                       tile_q, per_group, list);
         if constexpr (kMode != kPhysics) {
             if (tid == 0)
                 cs.n_ended = 0;
@@ -878,13 +878,13 @@ cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Wo
                         TerrainGeom<float>* tg, TerrainGeomD* tgd, const int* grid_of, double cell,
                         const TaskParams& P, const TaskState& S, const TaskOut& O, const Actuation& A, float* spill,
                         int spill_per_lane, int lane_cap, const int* ids, int n_items, int* queue, int sub0, int sub1,
-                        float* tile_q, cudaStream_t stream)
+                        float* tile_q, cudaStream_t stream, bool alone)
 {
     const int smem = (int)sizeof(ControlSmem);
     // per device and form: the shared-memory attribute, and how many CTAs are
     // resident at once (the work queue's wave)
     static std::atomic<unsigned long long> configured{0};
-    static int resident[64] = {};
+    static int resident[64] = {}, sm_count[64] = {};
     cudaError_t e = once_per_device(configured, [&](int dev) {
         cudaError_t r = cudaFuncSetAttribute(k_control_step<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int sms = 0, per_sm = 0;
@@ -893,22 +893,22 @@ cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Wo
         if (r == cudaSuccess)
             r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_control_step<kMode>, wl::kThreads, smem);
         if (r == cudaSuccess)
-            resident[dev] = sms * (per_sm > 0 ? per_sm : 1);
+            resident[dev] = sms * (per_sm > 0 ? per_sm : 1), sm_count[dev] = sms;
         return r;
     });
     if (e != cudaSuccess)
         return e;
-    const int groups = (n_items + wl::kWorlds - 1) / wl::kWorlds;
-    int grid = groups;
-    if (queue) {
-        int dev = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess)
-            return e;
-        grid = groups < resident[dev] ? groups : resident[dev];  // one wave of resident CTAs
-    }
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess)
+        return e;
+    wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone);
+    if (kMode != kPhysics)  // the fused forms' task work takes whole groups of 32
+        plan = wl::GroupPlan{wl::kWorlds, (n_items + wl::kWorlds - 1) / wl::kWorlds, plan.list};
+    // with a queue, one wave of resident CTAs
+    const int grid = queue && plan.groups > resident[dev] ? resident[dev] : plan.groups;
     k_control_step<kMode><<<grid, wl::kThreads, smem, stream>>>(M, RM, W, tg, tgd, grid_of, cell, P, S, O, A, spill,
                                                                 spill_per_lane, lane_cap, ids, n_items, queue, sub0,
-                                                                sub1, tile_q);
+                                                                sub1, tile_q, plan.per_group, plan.list);
     return cudaGetLastError();
 }
 
@@ -916,18 +916,18 @@ cudaError_t control_launch(const DevModel<float>& M, const ResetModel& RM, const
                            TerrainGeom<float>* tg, TerrainGeomD* tgd, const int* grid_of, double cell,
                            const TaskParams& P, const TaskState& S, const TaskOut& O, const Actuation& A,
                            float* spill, int spill_per_lane, int lane_cap, const int* ids, int n_items, int* queue,
-                           int mode, int sub0, int sub1, float* tile_q, cudaStream_t stream)
+                           int mode, int sub0, int sub1, float* tile_q, cudaStream_t stream, bool alone)
 {
     switch (mode) {
     case kPhysics:
         return launch_form<kPhysics>(M, RM, W, tg, tgd, grid_of, cell, P, S, O, A, spill, spill_per_lane, lane_cap,
-                                     ids, n_items, queue, sub0, sub1, tile_q, stream);
+                                     ids, n_items, queue, sub0, sub1, tile_q, stream, alone);
     case kWithTask:
         return launch_form<kWithTask>(M, RM, W, tg, tgd, grid_of, cell, P, S, O, A, spill, spill_per_lane, lane_cap,
-                                      ids, n_items, queue, sub0, sub1, tile_q, stream);
+                                      ids, n_items, queue, sub0, sub1, tile_q, stream, alone);
     case kWithResets:
         return launch_form<kWithResets>(M, RM, W, tg, tgd, grid_of, cell, P, S, O, A, spill, spill_per_lane,
-                                        lane_cap, ids, n_items, queue, sub0, sub1, tile_q, stream);
+                                        lane_cap, ids, n_items, queue, sub0, sub1, tile_q, stream, alone);
     default:
         return cudaErrorInvalidValue;
     }
@@ -1071,7 +1071,7 @@ cudaError_t launch_control_step(const DevModel<float>& M, const ResetModel& RM, 
                                 TerrainGeom<float>* tg, TerrainGeomD* tgd, const int* grid_of, double cell,
                                 const TaskParams& P, const TaskState& S, const TaskOut& O, const float* actions,
                                 float* spill, int spill_per_lane, int lane_cap, const int* ids, int n_items, int* queue,
-                                bool resets, cudaStream_t stream)
+                                bool resets, cudaStream_t stream, bool alone)
 {
     if (W.n <= 0 || n_items <= 0)
         return cudaSuccess;
@@ -1079,12 +1079,12 @@ cudaError_t launch_control_step(const DevModel<float>& M, const ResetModel& RM, 
         return cudaErrorInvalidValue;
     return control_launch(M, RM, W, tg, tgd, grid_of, cell, P, S, O, Actuation{nullptr, actions}, spill,
                           spill_per_lane, lane_cap, ids, n_items, queue, resets ? kWithResets : kWithTask, 0,
-                          M.substeps, nullptr, stream);
+                          M.substeps, nullptr, stream, alone);
 }
 
 cudaError_t launch_step_warps(const DevModel<float>& M, const Worlds<float>& W, const Actuation& A, float* spill,
                               int spill_per_lane, int lane_cap, const int* ids, int n_items, int* queue,
-                              cudaStream_t stream, int tile, float* tile_q)
+                              cudaStream_t stream, bool alone, int tile, float* tile_q)
 {
     if (W.n <= 0 || n_items <= 0)
         return cudaSuccess;
@@ -1099,7 +1099,7 @@ cudaError_t launch_step_warps(const DevModel<float>& M, const Worlds<float>& W, 
         const int sub1 = sub0 + tile < M.substeps ? sub0 + tile : M.substeps;
         cudaError_t e = control_launch(M, RM, W, nullptr, nullptr, nullptr, 0.0, P, TaskState{}, TaskOut{}, A, spill,
                                        spill_per_lane, lane_cap, ids, n_items, queue, kPhysics, sub0, sub1, tile_q,
-                                       stream);
+                                       stream, alone);
         if (e != cudaSuccess)
             return e;
     }

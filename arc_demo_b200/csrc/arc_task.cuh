@@ -105,7 +105,7 @@ cudaError_t launch_control_step(const DevModel<float>& M, const ResetModel& RM, 
                                 TerrainGeom<float>* tg, TerrainGeomD* tgd, const int* grid_of, double cell,
                                 const TaskParams& P, const TaskState& S, const TaskOut& O, const float* actions,
                                 float* spill, int spill_per_lane, int lane_cap, const int* ids, int n_items, int* queue,
-                                bool resets, cudaStream_t stream);
+                                bool resets, cudaStream_t stream, bool alone);
 
 // Starts worlds ids[0 .. n) (device arrays) afresh as new tenants of their
 // slots: level and difficulty, RNG key and RNG counters set, then a task
