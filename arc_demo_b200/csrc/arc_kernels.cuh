@@ -37,6 +37,7 @@ struct ResetModel {
     Q4<double> q_rel0[kMaxJoints];
     double default_angles[kMaxJoints], lo[kMaxJoints], hi[kMaxJoints];
     double stand_height, footprint;
+    int legs;  // joints in this many equal chains that start at body 0, in order (0: any tree)
 };
 
 // ----- stepping

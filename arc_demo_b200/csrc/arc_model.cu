@@ -377,6 +377,7 @@ ResetModel make_reset_model(const ModelHost& m)
         r.hi[i] = m.j[i].hi;
     }
     r.stand_height = m.stand_height;
+    r.legs = m.leaper ? kNumLegs : 0;
     r.footprint = m.footprint;
     return r;
 }

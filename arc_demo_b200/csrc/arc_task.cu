@@ -1,5 +1,5 @@
 // arc_task.cu - task layer kernels (arc/task.py on the device) and the
-// warp-cooperative world reset (csrc/arc_sim.c:88-110).
+// cooperative world reset (csrc/arc_sim.c:88-110).
 #include "arc_task.cuh"
 #include "arc_step_warps.cuh"
 
@@ -36,48 +36,67 @@ struct Xorshift {
 };
 
 // Jumping ahead in the stream. xorshift128 is linear over GF(2): one step
-// is a 128 x 128 bit matrix M acting on the state (s0 s1 s2 s3). Column b
-// of M^(2^k), for k < kJumpBits, is g_jump[k][b] (built once per device by
-// k_jump_init), so skipping d draws costs one XOR of a column per set state
-// bit, for each set bit of d; the draws that follow are the stream's own,
-// bit for bit.
-constexpr int kJumpBits = 13;  // skips below 8,192 draws (a 64 x 64 terrain takes 4,742)
-__device__ uint4 g_jump[kJumpBits][128];
+// is a 128 x 128 bit matrix M acting on the state (s0 s1 s2 s3). A reset's
+// draws are cut into 32 slices of kSlice, one per lane of a warp, and row b
+// of g_skip holds column b of M^(kSlice * lane) for every lane (built once
+// per device by k_skip_init), so all lanes jump to their slices by XORing the
+// rows of the state bits that are set: the same rows for every lane, 512
+// coalesced bytes each, sixteen loads in flight. Row 128 is zero. The draws
+// that follow are the stream's own, bit for bit. (Skipping each lane by
+// powers of two, M^(2^k), took three times the loads and diverged.)
+constexpr int kSlice = 149;  // 32 slices hold the 4,742 draws of a 64 x 64 terrain and its stance
+__device__ uint4 g_skip[129][32];
 
-__global__ void k_jump_init()
+__global__ void k_skip_init()
 {
-    const int k = blockIdx.x, b = threadIdx.x;
+    const int lane = blockIdx.x, b = threadIdx.x;
     Xorshift r;
     for (int w = 0; w < 4; ++w)
         r.s[w] = (b >> 5) == w ? 1u << (b & 31) : 0u;
-    for (int it = 0; it < (1 << k); ++it)
+    for (int it = 0; it < kSlice * lane; ++it)
         r.next();
-    g_jump[k][b] = make_uint4(r.s[0], r.s[1], r.s[2], r.s[3]);
+    g_skip[b][lane] = make_uint4(r.s[0], r.s[1], r.s[2], r.s[3]);
 }
 
-__device__ __forceinline__ void rng_skip(Xorshift& r, uint32_t d)
+// Moves a state that all lanes of a warp share to the start of the lane's
+// slice. rows: kSkipRows bytes of shared memory for the warp.
+constexpr int kSkipRows = 128 + 16;
+__device__ __forceinline__ void rng_to_slice(Xorshift& r, int lane, unsigned char* rows)
 {
-    for (int k = 0; d; ++k, d >>= 1) {
-        if (!(d & 1u))
-            continue;
-        uint32_t o[4] = {0u, 0u, 0u, 0u};
+    // the rows of the set bits, listed by the lanes: lane l looks at bits 4l .. 4l + 3
+    const int word = lane >> 3, bit0 = 4 * lane;
+    const uint32_t mine = (word == 0 ? r.s[0] : word == 1 ? r.s[1] : word == 2 ? r.s[2] : r.s[3]) >> (bit0 & 31) & 15u;
+    int at = 0, n = 0;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            uint32_t bits = r.s[w];
-            while (bits) {
-                const int b = __ffs(bits) - 1;
-                bits &= bits - 1u;
-                const uint4 c = g_jump[k][w * 32 + b];
-                o[0] ^= c.x;
-                o[1] ^= c.y;
-                o[2] ^= c.z;
-                o[3] ^= c.w;
-            }
-        }
-#pragma unroll
-        for (int w = 0; w < 4; ++w)
-            r.s[w] = o[w];
+    for (int w = 0; w < 4; ++w) {
+        at += w < word ? __popc(r.s[w]) : (w == word ? __popc(r.s[w] & ((1u << (bit0 & 31)) - 1u)) : 0);
+        n += __popc(r.s[w]);
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if ((mine >> u) & 1u)
+            rows[at++] = (unsigned char)(bit0 + u);
+    if (lane < 16)
+        rows[n + lane] = 128;
+    __syncwarp();
+    uint4 o = make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < n; k += 16) {
+        uint4 c[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            c[u] = g_skip[rows[k + u]][lane];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            o.x ^= c[u].x;
+            o.y ^= c[u].y;
+            o.z ^= c[u].z;
+            o.w ^= c[u].w;
+        }
+    }
+    r.s[0] = o.x;
+    r.s[1] = o.y;
+    r.s[2] = o.z;
+    r.s[3] = o.w;
 }
 
 // rng_range(lo, hi) of a raw draw u (csrc/arc_rng.h:45-53)
@@ -176,49 +195,108 @@ __device__ __forceinline__ V3<double> rt_mul(const M3<double>& r, V3<double> a)
                       a.x * r.m[0][2] + a.y * r.m[1][2] + a.z * r.m[2][2]};
 }
 
+constexpr int kHeightsAt = 9 + 3 * kNumJoints + 3;  // offset of the heights in an observation row
+
 __device__ __forceinline__ float obs_value(double v)
 {
     float f = (float)v;
     return isfinite(f) ? f : 0.0f;
 }
 
-// arc/task.py:231-259: writes the 195 observation values of world i
-// Observation entries m_begin .. m_end - 1 of the 143 terrain heights in the
-// heading frame (csrc/arc_sim.c:185-203), written to dst[m - m_begin], kChunk
-// samples at a time: their terrain loads are all issued before any is used.
+// The heading frame of the terrain heights (csrc/arc_sim.c:185-203).
+__device__ __forceinline__ void heading_of(Q4<double> q, double& cy, double& sy)
+{
+    const V3<double> f = qrotate(q, V3<double>{1.0, 0.0, 0.0});
+    const double yaw = atan2(f.y, f.x);
+    cy = cos(yaw);
+    sy = sin(yaw);
+}
+
+// Sample m of the 143 terrain heights around x in the heading frame; th, g:
+// world i's columns.
+template <class R>
+__device__ __forceinline__ double sample_height(const TaskParams& P, const Worlds<R>& W, int i, const TerrainGeomD& g,
+                                                const R* th, V3<double> x, double cy, double sy, int m)
+{
+    const double fo = P.offsets[m][0], lo = P.offsets[m][1];
+    const double px = x.x + cy * fo - sy * lo, py = x.y + sy * fo + cy * lo;
+    // csrc/arc_terrain.h:42-50
+    const double fx = floor((px - g.ox) / g.cell), fy = floor((py - g.oy) / g.cell);
+    const bool in = fx >= 0.0 && fy >= 0.0 && fx < g.nx && fy < g.ny &&
+                    terrain_column_ok(W, i, (int)fx + (long long)(int)fy * g.nx, kCheckHeightsRead);
+    const int idx = in ? (int)fx + (int)fy * g.nx : 0;
+    const double top = (double)th[idx];
+    return in ? top : g.outside;
+}
+
+// The observation's entry of a terrain height.
+__device__ __forceinline__ float height_value(const TaskParams& P, V3<double> x, double h)
+{
+    const double rel = x.z - P.stand_height - h;
+    return obs_value(rel < -1.0 ? -1.0 : (rel > 1.0 ? 1.0 : rel));
+}
+
+// Observation entries m_begin .. m_end - 1 of the 143 terrain heights,
+// written to dst[m - m_begin], kChunk samples at a time: their terrain loads
+// are all issued before any is used.
 template <int kChunk, class R>
 __device__ void write_heights(const TaskParams& P, const Worlds<R>& W, int i, V3<double> x, Q4<double> q, float* dst,
                               int m_begin, int m_end)
 {
-    V3<double> f = qrotate(q, V3<double>{1.0, 0.0, 0.0});
-    const double yaw = atan2(f.y, f.x), cy = cos(yaw), sy = sin(yaw);
+    double cy, sy;
+    heading_of(q, cy, sy);
     const TerrainGeomD g = W.tgd[i];
     const R* th = W.th + W.toff[i];
     int k = 0;
     for (int m0 = m_begin; m0 < m_end; m0 += kChunk) {
         double h[kChunk];
 #pragma unroll
-        for (int u = 0; u < kChunk; ++u) {
-            const int m = m0 + u < m_end ? m0 + u : m_end - 1;
-            const double fo = P.offsets[m][0], lo = P.offsets[m][1];
-            const double px = x.x + cy * fo - sy * lo, py = x.y + sy * fo + cy * lo;
-            // csrc/arc_terrain.h:42-50
-            const double fx = floor((px - g.ox) / g.cell), fy = floor((py - g.oy) / g.cell);
-            const bool in = fx >= 0.0 && fy >= 0.0 && fx < g.nx && fy < g.ny &&
-                            terrain_column_ok(W, i, (int)fx + (long long)(int)fy * g.nx, kCheckHeightsRead);
-            const int idx = in ? (int)fx + (int)fy * g.nx : 0;
-            const double top = (double)__ldg(th + idx);
-            h[u] = in ? top : g.outside;
-        }
+        for (int u = 0; u < kChunk; ++u)
+            h[u] = sample_height(P, W, i, g, th, x, cy, sy, m0 + u < m_end ? m0 + u : m_end - 1);
 #pragma unroll
         for (int u = 0; u < kChunk; ++u) {
             if (m0 + u >= m_end)
                 break;
-            double rel = x.z - P.stand_height - h[u];
-            rel = rel < -1.0 ? -1.0 : (rel > 1.0 ? 1.0 : rel);
-            dst[k++] = obs_value(rel);
+            dst[k++] = height_value(P, x, h[u]);
         }
     }
+}
+
+// arc/task.py:231-259: writes the 195 observation values of world i
+// The parts of an observation row (arc/task.py:231-259): entries 0..8 the
+// torso's, 9..44 the joints', 45..47 the checkpoint's, then the heights and
+// the feet's contacts.
+__device__ __forceinline__ void obs_torso(const M3<double>& r, V3<double> v, V3<double> w, float* row)
+{
+    row[0] = obs_value(-r.m[2][0]);
+    row[1] = obs_value(-r.m[2][1]);
+    row[2] = obs_value(-r.m[2][2]);
+    const V3<double> lin = rt_mul(r, v), ang = rt_mul(r, w);
+    row[3] = obs_value(lin.x);
+    row[4] = obs_value(lin.y);
+    row[5] = obs_value(lin.z);
+    row[6] = obs_value(0.25 * ang.x);
+    row[7] = obs_value(0.25 * ang.y);
+    row[8] = obs_value(0.25 * ang.z);
+}
+
+__device__ __forceinline__ void obs_joint(const TaskParams& P, int j, double angle, double rate, double action,
+                                          float* row)
+{
+    row[9 + j] = obs_value(angle - P.default_angles[j]);
+    row[9 + kNumJoints + j] = obs_value(0.1 * rate);
+    row[9 + 2 * kNumJoints + j] = obs_value(action);
+}
+
+// c, s: cosine and sine of the heading
+__device__ __forceinline__ void obs_target(double c, double s, double dx, double dy, float* row)
+{
+    const double fwd = c * dx + s * dy, left = -s * dx + c * dy;
+    double dist = hypot(fwd, left);
+    dist = dist > 1e-6 ? dist : 1e-6;
+    row[kHeightsAt - 3] = obs_value(fwd / dist);
+    row[kHeightsAt - 2] = obs_value(left / dist);
+    row[kHeightsAt - 1] = obs_value((dist < 6.0 ? dist : 6.0) / 6.0);
 }
 
 template <class R>
@@ -226,37 +304,16 @@ __device__ void write_obs(const TaskParams& P, const Worlds<R>& W, const TaskSta
                           float* dst, bool heights = true)
 {
     const M3<double>& r = o.rot;
-    int k = 0;
-    dst[k++] = obs_value(-r.m[2][0]);
-    dst[k++] = obs_value(-r.m[2][1]);
-    dst[k++] = obs_value(-r.m[2][2]);
-    V3<double> lin = rt_mul(r, o.v), ang = rt_mul(r, o.w);
-    dst[k++] = obs_value(lin.x);
-    dst[k++] = obs_value(lin.y);
-    dst[k++] = obs_value(lin.z);
-    dst[k++] = obs_value(0.25 * ang.x);
-    dst[k++] = obs_value(0.25 * ang.y);
-    dst[k++] = obs_value(0.25 * ang.z);
+    obs_torso(r, o.v, o.w, dst);
     for (int j = 0; j < kNumJoints; ++j)
-        dst[k++] = obs_value(o.angle[j] - P.default_angles[j]);
-    for (int j = 0; j < kNumJoints; ++j)
-        dst[k++] = obs_value(0.1 * o.rate[j]);
-    for (int j = 0; j < kNumJoints; ++j)
-        dst[k++] = obs_value((double)S.prev_action[(size_t)i * kNumJoints + j]);
+        obs_joint(P, j, o.angle[j], o.rate[j], (double)S.prev_action[(size_t)i * kNumJoints + j], dst);
     const double heading = atan2(r.m[1][0], r.m[0][0]);
     const double dx = S.target[2 * i] - o.x.x, dy = S.target[2 * i + 1] - o.x.y;
-    const double c = cos(heading), s = sin(heading);
-    const double fwd = c * dx + s * dy, left = -s * dx + c * dy;
-    double dist = hypot(fwd, left);
-    dist = dist > 1e-6 ? dist : 1e-6;
-    dst[k++] = obs_value(fwd / dist);
-    dst[k++] = obs_value(left / dist);
-    dst[k++] = obs_value((dist < 6.0 ? dist : 6.0) / 6.0);
+    obs_target(cos(heading), sin(heading), dx, dy, dst);
     if (heights)
-        write_heights<8>(P, W, i, o.x, o.q, dst + k, 0, kNumOffsets);
-    k += kNumOffsets;
+        write_heights<8>(P, W, i, o.x, o.q, dst + kHeightsAt, 0, kNumOffsets);
     for (int l = 0; l < kNumLegs; ++l)
-        dst[k++] = obs_value(o.contact[l]);
+        dst[kHeightsAt + kNumOffsets + l] = obs_value(o.contact[l]);
 }
 
 // Checkpoint 3-6 m away inside the terrain (arc/task.py:127-151), drawn
@@ -412,7 +469,6 @@ __global__ void k_task_step(const __grid_constant__ DevModel<R> M, Worlds<R> W, 
 // their terminal observation too.
 constexpr int kHeightsPer = 16;
 constexpr int kHeightParts = (kNumOffsets + kHeightsPer - 1) / kHeightsPer;
-constexpr int kHeightsAt = 9 + 3 * kNumJoints + 3;  // offset of the heights in a row
 
 constexpr int kHeightThreads = 128;
 constexpr int kHeightBlocks = 8;
@@ -462,15 +518,38 @@ __global__ void k_task_observe(const __grid_constant__ DevModel<R> M, Worlds<R> 
 }
 
 // ---------------------------------------------------------------------------
-// warp-cooperative reset (csrc/arc_sim.c:88-110, csrc/arc_terrain.c:35-71):
-// each lane draws one consecutive slice of the world's RNG stream (skipping
-// ahead to it), all lanes build the terrain columns, lane 0 poses the robot.
-// The columns' jitter draws go straight into the world's own terrain array,
-// each to the slot its height later overwrites, so a warp needs only ~7 KB
-// of shared memory and dozens of worlds reset side by side on every SM.
+// cooperative reset (csrc/arc_sim.c:88-110, csrc/arc_terrain.c:35-71): a CTA
+// of four warps resets one world at a time. Warp 0 draws the world's RNG
+// stream (each lane one slice) into shared memory while the others tabulate
+// the lattice coordinates; the warps build the terrain in blocks of 32 x 8
+// cells, a lane walking down eight cells of a column, while warp 0 first
+// turns the joints (a lane per leg), which needs no ground; then the bodies
+// are placed on the ground, and the warps share the task state, the
+// checkpoint and the observation.
+//
+// In a control step a few worlds end and the step waits for the slowest of
+// them, so one world's latency counts as much as the throughput of a whole
+// batch. One warp per world spent 200 us on a world: 128 columns a lane with
+// both noises' four lattice values and two FP64 divisions each, 143 heights
+// and the stance in one lane. Here a thread walks down its column of cells
+// and keeps the two x-interpolations of each noise until the lattice row
+// changes (3 FP64 operations a noise and cell instead of 10), the division by
+// the constant step is a multiplication with a correcting FMA pair, and
+// no lane is left with more than a leg's joints or the checkpoint. (Code that
+// one lane runs once costs most in fetching it: the task state and
+// observation of a new world by one thread took 46k cycles.) The reset of
+// the 470 worlds that end in a step of 65,536: 217 -> 33 us; of 26 in one of
+// 4,096: 200 -> 28 us; of 16,384 worlds at once 2,001 -> 543 us (268 MB of
+// terrain written: 41 us at the copy rate), bound by instruction issue (59 %
+// of cycles) and the barriers between the phases.
 
+constexpr int kResetThreads = 128;
+constexpr int kResetWarps = kResetThreads / 32;
+constexpr int kResetPerSm = 8;                                   // 26 KB of shared memory each
 constexpr int kLat1 = (kGridMax / 8 + 2) * (kGridMax / 8 + 2);   // 100
 constexpr int kLat2 = (kGridMax / 3 + 2) * (kGridMax / 3 + 2);   // 529
+constexpr int kMaxDraws = kLat1 + kLat2 + kGridMax * kGridMax + kMaxJoints + 1;
+static_assert(kMaxDraws <= 32 * kSlice, "a world's draws fit 32 slices");
 
 struct ResetSmem {
     double lat[kLat1 + kLat2];
@@ -478,7 +557,17 @@ struct ResetSmem {
     // integer part and smoothed fraction (csrc/arc_terrain.c:41-45)
     double frac[2][kGridMax];
     int whole[2][kGridMax];
-    uint32_t pose[kMaxJoints + 1];  // the stance noise and yaw draws
+    uint32_t draw[kMaxDraws];       // the raw draws: lattices, jitter, stance noise and yaw
+    double top[kResetWarps];        // highest column under the robot, per warp
+    unsigned long long under;       // columns (of either axis) under the robot
+    int outside;                    // the robot's footprint leaves the grid
+    int next;                       // the next block of cells
+    uint32_t seed;
+    unsigned char rows[kSkipRows];
+    double angle[kMaxJoints];
+    V3<double> up[kMaxJoints], down[kMaxJoints];  // parent -> joint, joint -> child, in the world
+    V3<double> x[kMaxBodies];
+    Q4<double> q[kMaxBodies];
 };
 
 // The generator's arithmetic is written with explicitly rounded FP64
@@ -536,11 +625,67 @@ __device__ __forceinline__ unsigned long long scan_cells(double reach, double st
     return mask;
 }
 
-template <class R>
-__device__ void reset_world_warp(ResetSmem& sm, const ResetModel& RM, const Worlds<R>& W, TerrainGeom<R>* tg,
-                                 TerrainGeomD* tgd, int i, uint32_t seed, double diff, int n, double cell)
+// a / 0.03 correctly rounded: the quotient from the reciprocal, corrected
+// twice by its exact remainder (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990).
+__device__ __forceinline__ double over_step(double a)
 {
-    const int lane = threadIdx.x & 31;
+    constexpr double b = 0.03, y = 1.0 / 0.03;
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// A lattice's interpolation along x at row gy, and between two rows: the
+// operations of noise_at.
+__device__ __forceinline__ double noise_row(const double* lat, int m, int gy, double tx)
+{
+    const double a = lat[gy * m], b = lat[gy * m + 1];
+    return __dadd_rn(a, __dmul_rn(__dsub_rn(b, a), tx));
+}
+__device__ __forceinline__ double noise_between(double top, double bot, double ty)
+{
+    return __dadd_rn(__dmul_rn(top, __dsub_rn(1.0, ty)), __dmul_rn(bot, ty));
+}
+
+// Forward kinematics of joints j0 .. j1 - 1, whose parents are turned
+// (csrc/arc_phys.c:749-782, with the stance noise of csrc/arc_sim.c:99-103):
+// everything but the positions, which wait for the ground.
+__device__ __forceinline__ void turn_joints(ResetSmem& sm, const ResetModel& RM, const uint32_t* draw, int j0, int j1)
+{
+#pragma unroll 1
+    for (int j = j0; j < j1; ++j) {
+        double a = RM.default_angles[j] + range_of(draw[j], -0.1, 0.1);
+        a = a < RM.lo[j] ? RM.lo[j] : (a > RM.hi[j] ? RM.hi[j] : a);
+        sm.angle[j] = a;
+        const int p = RM.parent[j];
+        const Q4<double> qp = p >= 0 ? sm.q[p] : q_identity<double>();
+        sm.up[j] = qrotate(qp, RM.r1[j]);
+        const double s = sin(0.5 * a), ca = cos(0.5 * a);
+        const Q4<double> qa{ca, RM.a1[j].x * s, RM.a1[j].y * s, RM.a1[j].z * s};
+        const Q4<double> qc = qnormalize(qmul(qp, qmul(qa, RM.q_rel0[j])));
+        sm.q[RM.child[j]] = qc;
+        sm.down[j] = qrotate(qc, RM.r2[j]);
+    }
+}
+
+__device__ __forceinline__ void place_joints(ResetSmem& sm, const ResetModel& RM, int j0, int j1)
+{
+    for (int j = j0; j < j1; ++j) {
+        const int p = RM.parent[j];
+        const V3<double> anchor = (p >= 0 ? sm.x[p] : V3<double>{0.0, 0.0, 0.0}) + sm.up[j];
+        sm.x[RM.child[j]] = anchor - sm.down[j];
+    }
+}
+
+// Resets world i; called by all kResetThreads threads of a CTA. When it
+// returns every thread has passed a barrier after the world's last write.
+template <class R>
+__device__ __forceinline__ void reset_world(ResetSmem& sm, const ResetModel& RM, const Worlds<R>& W,
+                                            TerrainGeom<R>* tg, TerrainGeomD* tgd, int i, uint32_t seed, double diff,
+                                            int n, double cell)
+{
+    const int tid = threadIdx.x, lane = tid & 31;
     n = n < kGridMax ? n : kGridMax;
     const bool rough = diff > 0.0;
     const int m1 = n / 8 + 2, m2 = n / 3 + 2;
@@ -548,185 +693,243 @@ __device__ void reset_world_warp(ResetSmem& sm, const ResetModel& RM, const Worl
     const int J = rough ? n * n : 0;
     R* h = W.th + W.toff[i];
     if (!terrain_column_ok(W, i, (long long)n * n - 1, kCheckTerrainWrite))
-        return;  // the whole warp: n and the slice are the world's
-    // the raw jitter draw of column c sits in the low word of h[c] until the
-    // column's height replaces it
-    uint32_t* hdraw = reinterpret_cast<uint32_t*>(h);
-    constexpr int kStep = sizeof(R) / sizeof(uint32_t);
-    {
-        // slices of 2^kSliceBits draws: a lane skips by its index times a
-        // power of two, a few columns of five tables
-        constexpr int kSliceBits = 8;
-        const int total = L + J + RM.nj + 1;
-        const int per = total <= 32 << kSliceBits ? 1 << kSliceBits : (total + 31) / 32;
-        const int first = lane * per, last = first + per < total ? first + per : total;
-        Xorshift rng;
-        rng.seed(seed);
-        if (first < last)
-            rng_skip(rng, (uint32_t)first);
-        for (int k = first; k < last; ++k) {
-            const uint32_t u = rng.next();
-            if (k < L)
-                sm.lat[k] = __dadd_rn(-1.0, __dmul_rn(2.0, __dmul_rn((double)u, 1.0 / 4294967296.0)));
-            else if (k < L + J)
-                hdraw[(k - L) * kStep] = u;
-            else
-                sm.pose[k - L - J] = u;
-        }
-    }
-    for (int c = lane; c < 2 * kGridMax; c += 32)
-        lattice_coord(c < kGridMax ? 8 : 3, c % kGridMax, sm.whole[c / kGridMax][c % kGridMax],
-                      sm.frac[c / kGridMax][c % kGridMax]);
-    __syncwarp();
-
+        return;  // the whole CTA: n and the slice are the world's
     TerrainGeomD g;
     g.nx = g.ny = n;
     g.cell = cell;
     g.ox = -0.5 * n * cell;
     g.oy = -0.5 * n * cell;
     g.outside = -100.0;
-    if (lane == 0) {
-        tgd[i] = g;
-        tg[i] = TerrainGeom<R>{n, n, (R)g.cell, (R)g.ox, (R)g.oy, (R)g.outside};
+    if (tid < 32) {
+        const int total = L + J + RM.nj + 1;
+        const int first = lane * kSlice, last = first + kSlice < total ? first + kSlice : total;
+        Xorshift rng;
+        rng.seed(seed);
+        rng_to_slice(rng, lane, sm.rows);
+        for (int k = first; k < last; ++k)
+            sm.draw[k] = rng.next();
+    } else {
+        for (int c = tid - 32; c < 2 * kGridMax; c += kResetThreads - 32)
+            lattice_coord(c < kGridMax ? 8 : 3, c % kGridMax, sm.whole[c / kGridMax][c % kGridMax],
+                          sm.frac[c / kGridMax][c % kGridMax]);
+        if (tid == 32) {
+            // the grid is square and centred: x and y scan the same columns
+            bool out = false;
+            sm.under = scan_cells(RM.footprint + 0.1, 0.5 * cell, g.ox, cell, n, out);
+            sm.outside = out;
+            sm.next = 0;
+            tgd[i] = g;
+            tg[i] = TerrainGeom<R>{n, n, (R)g.cell, (R)g.ox, (R)g.oy, (R)g.outside};
+        }
     }
-    const double reach = RM.footprint + 0.1, step = 0.5 * cell;
-    bool out_x = false, out_y = false;
-    const unsigned long long mx = scan_cells(reach, step, g.ox, cell, n, out_x);
-    const unsigned long long my = scan_cells(reach, step, g.oy, cell, n, out_y);
-    double ground = (out_x || out_y) ? g.outside : -1e30;
+    __syncthreads();
+    for (int k = tid; k < L; k += kResetThreads)
+        sm.lat[k] = __fma_rn((double)sm.draw[k], 2.0 / 4294967296.0, -1.0);  // -1 + 2 u: the product is exact
+    __syncthreads();
+
+    // the joints, a lane per leg
+    const int lanes = RM.legs > 0 ? RM.legs : 1, per = RM.nj / lanes;
+    if (tid < 32) {
+        const uint32_t* draw = sm.draw + L + J;
+        if (lane == 0) {
+            const double yaw = range_of(draw[RM.nj], -kPi, kPi);
+            const double sy = sin(0.5 * yaw), cyw = cos(0.5 * yaw);
+            sm.q[0] = qnormalize(Q4<double>{cyw, 0.0 * sy, 0.0 * sy, 1.0 * sy});
+        }
+        __syncwarp();
+        if (lane < lanes)
+            turn_joints(sm, RM, draw, lane * per, (lane + 1) * per);
+        __syncwarp();
+    }
+    const unsigned long long under = sm.under;
+    double gmax = rough ? -1e300 : 0.0;
     if (!rough) {
-        for (int c = lane; c < n * n; c += 32)
+        for (int c = tid; c < n * n; c += kResetThreads)
             h[c] = R(0);
-        if (mx && my)
-            ground = ground > 0.0 ? ground : 0.0;
     } else {
         const double amp1 = __dmul_rn(0.45, diff), amp2 = __dmul_rn(0.12, diff), ampj = __dmul_rn(0.06, diff);
         const double* lat1 = sm.lat;
         const double* lat2 = sm.lat + m1 * m1;
+        const uint32_t* draw = sm.draw + L;
         const double f0x = floor((0.0 - g.ox) / g.cell), f0y = floor((0.0 - g.oy) / g.cell);
         double base = g.outside;
         if (f0x >= 0.0 && f0y >= 0.0 && f0x < n && f0y < n) {
             const int ix = (int)f0x, iy = (int)f0y;
-            base = column_height(sm, lat1, m1, lat2, m2, ix, iy, amp1, amp2, ampj, hdraw[(ix + iy * n) * kStep]);
+            base = column_height(sm, lat1, m1, lat2, m2, ix, iy, amp1, amp2, ampj, draw[ix + iy * n]);
         }
-        __syncwarp();  // every lane has read the base column's draw
-        double gmax = -1e300;
-        for (int c = lane; c < n * n; c += 32) {
-            const int ix = c % n, iy = c / n;
-            const double hf =
-                __dsub_rn(column_height(sm, lat1, m1, lat2, m2, ix, iy, amp1, amp2, ampj, hdraw[c * kStep]), base);
-            h[c] = (R)hf;
-            if (((mx >> ix) & 1) && ((my >> iy) & 1))
-                gmax = gmax > hf ? gmax : hf;
+        // blocks of 32 x 8 cells (two of 16 x 4 for at most 16 columns) to the
+        // warps as they come: a lane walks down its column. The rows of a
+        // block share the coarse noise's lattice row.
+        const int wide = n > 16 ? 32 : 16, rows = n > 16 ? 8 : 4, over = (n + wide - 1) / wide;
+        const int blocks = over * ((n + 7) / 8);
+        for (;;) {
+            int block = 0;
+            if (lane == 0)
+                block = atomicAdd(&sm.next, 1);
+            block = __shfl_sync(0xffffffffu, block, 0);
+            if (block >= blocks)
+                break;
+            const int ix = block % over * wide + (lane & (wide - 1));
+            const int iy0 = block / over * 8 + (n > 16 ? 0 : lane / 16 * 4);
+            if (ix >= n || iy0 >= n)
+                continue;
+            const double* c1 = lat1 + sm.whole[0][ix];
+            const double* c2 = lat2 + sm.whole[1][ix];
+            const double tx1 = sm.frac[0][ix], tx2 = sm.frac[1][ix];
+            const int g1 = sm.whole[0][iy0];
+            const double top1 = noise_row(c1, m1, g1, tx1), bot1 = noise_row(c1, m1, g1 + 1, tx1);
+            int g2 = sm.whole[1][iy0];
+            double top2 = noise_row(c2, m2, g2, tx2), bot2 = noise_row(c2, m2, g2 + 1, tx2);
+            const uint32_t below = ((under >> ix) & 1) ? (uint32_t)(under >> iy0) : 0u;
+            const int count = n - iy0 < rows ? n - iy0 : rows;
+            const uint32_t* dr = draw + ix + iy0 * n;
+            R* col = h + ix + iy0 * n;
+#pragma unroll 1
+            for (int k = 0; k < count; ++k, dr += n, col += n) {
+                if (sm.whole[1][iy0 + k] != g2) {
+                    ++g2;
+                    top2 = bot2;
+                    bot2 = noise_row(c2, m2, g2 + 1, tx2);
+                }
+                // column_height, operation by operation
+                const double v = __dadd_rn(__dmul_rn(amp1, noise_between(top1, bot1, sm.frac[0][iy0 + k])),
+                                           __dmul_rn(amp2, noise_between(top2, bot2, sm.frac[1][iy0 + k])));
+                const double jitter = __fma_rn((double)*dr, 2.0 / 4294967296.0, -1.0);
+                const double hj = __dadd_rn(v, __dmul_rn(ampj, jitter));
+                const double top = __dmul_rn(0.03, floor(__dadd_rn(over_step(hj), 0.5)));
+                const double hf = __dsub_rn(top, base);
+                *col = (R)hf;
+                if ((below >> k) & 1)
+                    gmax = gmax > hf ? gmax : hf;
+            }
         }
         for (int off = 16; off > 0; off >>= 1) {
-            double o = __shfl_xor_sync(0xffffffffu, gmax, off);
+            const double o = __shfl_xor_sync(0xffffffffu, gmax, off);
             gmax = gmax > o ? gmax : o;
         }
-        if (mx && my)
-            ground = ground > gmax ? ground : gmax;
     }
-    if (lane != 0)
-        return;
+    if (lane == 0)
+        sm.top[tid / 32] = gmax;
+    __syncthreads();
 
-    // noisy stance, yaw, forward kinematics (csrc/arc_sim.c:99-109, csrc/arc_phys.c:749-782)
-    double angles[kMaxJoints];
-    for (int j = 0; j < RM.nj; ++j) {
-        double a = RM.default_angles[j] + range_of(sm.pose[j], -0.1, 0.1);
-        angles[j] = a < RM.lo[j] ? RM.lo[j] : (a > RM.hi[j] ? RM.hi[j] : a);
-    }
-    const double yaw = range_of(sm.pose[RM.nj], -kPi, kPi);
-    V3<double> xs[kMaxBodies];
-    Q4<double> qs[kMaxBodies];
-    const double sy = sin(0.5 * yaw), cyw = cos(0.5 * yaw);
-    xs[0] = V3<double>{0.0, 0.0, ground + RM.stand_height + 0.03};
-    qs[0] = qnormalize(Q4<double>{cyw, 0.0 * sy, 0.0 * sy, 1.0 * sy});
-    for (int j = 0; j < RM.nj; ++j) {
-        const int p = RM.parent[j], c = RM.child[j];
-        V3<double> xp = p >= 0 ? xs[p] : V3<double>{0.0, 0.0, 0.0};
-        Q4<double> qp = p >= 0 ? qs[p] : q_identity<double>();
-        V3<double> anchor = xp + qrotate(qp, RM.r1[j]);
-        const double s = sin(0.5 * angles[j]), ca = cos(0.5 * angles[j]);
-        Q4<double> qa{ca, RM.a1[j].x * s, RM.a1[j].y * s, RM.a1[j].z * s};
-        qs[c] = qnormalize(qmul(qp, qmul(qa, RM.q_rel0[j])));
-        xs[c] = anchor - qrotate(qs[c], RM.r2[j]);
-    }
     R* rec = W.rec + (size_t)i * W.stride;
-    for (int b = 0; b < RM.nb; ++b) {
+    R* sr = rec + W.off_sphere;
+    R* jr = rec + W.off_joint;
+    if (tid < 32) {
+        // on the ground (csrc/arc_sim.c:104-109)
+        double ground = sm.outside ? g.outside : -1e30;
+        if (under)
+            for (int w = 0; w < kResetWarps; ++w)
+                ground = ground > sm.top[w] ? ground : sm.top[w];
+        if (lane == 0)
+            sm.x[0] = V3<double>{0.0, 0.0, ground + RM.stand_height + 0.03};
+        __syncwarp();
+        if (lane < lanes)
+            place_joints(sm, RM, lane * per, (lane + 1) * per);
+    } else {
+        for (int c = tid - 32; c < RM.ns * kSphereRec; c += kResetThreads - 32)
+            sr[c] = R(0);
+        for (int c = tid - 32; c < RM.ns; c += kResetThreads - 32)
+            W.sph[(size_t)i * RM.ns + c] = 0;
+        for (int j = tid - 32; j < RM.nj; j += kResetThreads - 32) {
+            jr[j * kJointRec + 0] = (R)sm.angle[j];
+            jr[j * kJointRec + 1] = (R)sm.angle[j];
+            jr[j * kJointRec + 2] = R(0);
+            jr[j * kJointRec + 3] = R(0);
+        }
+        if (tid == 32) {
+            W.unstable[i] = 0;
+            W.time[i] = 0.0;
+        }
+    }
+    __syncthreads();
+    for (int b = tid; b < RM.nb; b += kResetThreads) {
         R* r = rec + b * kBodyRec;
-        r[0] = (R)xs[b].x; r[1] = (R)xs[b].y; r[2] = (R)xs[b].z;
-        r[3] = (R)qs[b].w; r[4] = (R)qs[b].x; r[5] = (R)qs[b].y; r[6] = (R)qs[b].z;
+        const V3<double> x = sm.x[b];
+        const Q4<double> q = sm.q[b];
+        r[0] = (R)x.x; r[1] = (R)x.y; r[2] = (R)x.z;
+        r[3] = (R)q.w; r[4] = (R)q.x; r[5] = (R)q.y; r[6] = (R)q.z;
         for (int c = 7; c < 13; ++c)
             r[c] = R(0);
     }
-    R* sr = rec + W.off_sphere;
-    uint32_t* sph = W.sph + (size_t)i * RM.ns;
-    for (int s = 0; s < RM.ns; ++s) {
-        for (int c = 0; c < kSphereRec; ++c)
-            sr[s * kSphereRec + c] = R(0);
-        sph[s] = 0;
-    }
-    R* jr = rec + W.off_joint;
-    for (int j = 0; j < RM.nj; ++j) {
-        jr[j * kJointRec + 0] = (R)angles[j];
-        jr[j * kJointRec + 1] = (R)angles[j];
-        jr[j * kJointRec + 2] = R(0);
-        jr[j * kJointRec + 3] = R(0);
-    }
-    W.unstable[i] = 0;
-    W.time[i] = 0.0;
+    __syncthreads();
 }
 
 template <class R>
-__global__ void __launch_bounds__(32)
-k_reset_warp(const __grid_constant__ ResetModel RM, Worlds<R> W, TerrainGeom<R>* tg, TerrainGeomD* tgd,
-             const int* __restrict__ ids, int n_ids, const unsigned* __restrict__ seeds,
-             const double* __restrict__ difficulty, const int* __restrict__ grid_of, double cell)
+__global__ void __launch_bounds__(kResetThreads, kResetPerSm)
+k_reset(const __grid_constant__ ResetModel RM, Worlds<R> W, TerrainGeom<R>* tg, TerrainGeomD* tgd,
+        const int* __restrict__ ids, int n_ids, const unsigned* __restrict__ seeds,
+        const double* __restrict__ difficulty, const int* __restrict__ grid_of, double cell)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ResetSmem& sm = *reinterpret_cast<ResetSmem*>(smem_raw);
     for (int k = blockIdx.x; k < n_ids; k += gridDim.x) {
         const int i = ids[k];
-        reset_world_warp(sm, RM, W, tg, tgd, i, seeds[k], difficulty[k], grid_of ? grid_of[i] : kGridMax, cell);
-        __syncwarp();
+        reset_world(sm, RM, W, tg, tgd, i, seeds[k], difficulty[k], grid_of ? grid_of[i] : kGridMax, cell);
     }
 }
 
 // ArcTask.reset (arc/task.py:113-125) + the observation of the new episode,
-// by the 32 lanes of one warp (compiled once, as task_step_world).
+// by the kResetThreads threads of a CTA (compiled once, as task_step_world).
 template <class R>
 __device__ __noinline__ void task_reset_world(ResetSmem& sm, const DevModel<R>& M, const ResetModel& RM, const Worlds<R>& W,
                                  TerrainGeom<R>* tg, TerrainGeomD* tgd, const int* __restrict__ grid_of, double cell,
                                  const TaskParams& P, const TaskState& S, float* obs, int i)
 {
-    const int lane = threadIdx.x & 31;
-    uint32_t seed = 0;
-    if (lane == 0) {
+    const int tid = threadIdx.x;
+    if (tid == 0) {
         const unsigned e = S.episode[i]++;
-        seed = (uint32_t)stream_u64(P.seed, key_of(S, i), 2u, e);
+        sm.seed = (uint32_t)stream_u64(P.seed, key_of(S, i), 2u, e);
         S.difficulty[i] = S.level[i];
     }
-    seed = __shfl_sync(0xffffffffu, seed, 0);
-    __syncwarp();
-    reset_world_warp(sm, RM, W, tg, tgd, i, seed, S.difficulty[i], grid_of ? grid_of[i] : kGridMax, cell);
-    __syncwarp();
-    if (lane == 0) {
-        for (int j = 0; j < kNumJoints; ++j)
+    __syncthreads();
+    reset_world(sm, RM, W, tg, tgd, i, sm.seed, S.level[i], grid_of ? grid_of[i] : kGridMax, cell);
+    // warp 0: the checkpoint; warp 1: the task state and the rest of the row
+    // but the heights; warps 2, 3: the heights
+    float* row = obs ? obs + (size_t)i * kObsSize : nullptr;
+    const R* b0 = W.rec + (size_t)i * W.stride;
+    const V3<double> x{(double)b0[0], (double)b0[1], (double)b0[2]};
+    const Q4<double> q{(double)b0[3], (double)b0[4], (double)b0[5], (double)b0[6]};
+    if (tid < 32) {
+        const M3<double> rot = m3_from_quat(q);
+        if (tid == 0)
+            place_target(P, W, S, i, x, rot);
+        __syncwarp();
+        if (tid == 0 && row) {
+            const double heading = atan2(rot.m[1][0], rot.m[0][0]);
+            obs_target(cos(heading), sin(heading), S.target[2 * i] - x.x, S.target[2 * i + 1] - x.y, row);
+        }
+    } else if (tid < 64) {
+        const int j = tid - 32;
+        const R* jr = b0 + W.off_joint;
+        if (j < kNumJoints) {
             S.prev_action[(size_t)i * kNumJoints + j] = 0.0f;
-        S.torso_steps[i] = 0;
-        S.steps[i] = 0;
-        S.checkpoints[i] = 0;
-        Obs64 o;
-        read_world(M, W, i, o);
-        place_target(P, W, S, i, o.x, o.rot);
-        if (obs)
-            write_obs(P, W, S, i, o, obs + (size_t)i * kObsSize);
+            if (row)
+                obs_joint(P, j, (double)jr[j * kJointRec + 1], (double)jr[j * kJointRec + 2], 0.0, row);
+        } else if (j < kNumJoints + kNumLegs) {
+            if (row)  // no sphere has touched yet
+                row[kHeightsAt + kNumOffsets + j - kNumJoints] = 0.0f;
+        } else if (j == kNumJoints + kNumLegs) {
+            S.torso_steps[i] = 0;
+            S.steps[i] = 0;
+            S.checkpoints[i] = 0;
+            if (row)
+                obs_torso(m3_from_quat(q), V3<double>{(double)b0[7], (double)b0[8], (double)b0[9]},
+                          V3<double>{(double)b0[10], (double)b0[11], (double)b0[12]}, row);
+        }
+    } else if (row) {
+        double cy, sy;
+        heading_of(q, cy, sy);
+        const TerrainGeomD g = W.tgd[i];
+        const R* th = W.th + W.toff[i];
+        for (int m = tid - 64; m < kNumOffsets; m += kResetThreads - 64)
+            row[kHeightsAt + m] = height_value(P, x, sample_height(P, W, i, g, th, x, cy, sy, m));
     }
-    __syncwarp();
+    __syncthreads();  // the next world's reset reuses sm
 }
 
 template <class R>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kResetThreads, kResetPerSm)
 k_task_reset(const __grid_constant__ DevModel<R> M, const __grid_constant__ ResetModel RM, Worlds<R> W,
              TerrainGeom<R>* tg, TerrainGeomD* tgd, const int* __restrict__ grid_of, double cell,
              const __grid_constant__ TaskParams P, TaskState S, float* obs, const int* __restrict__ ids,
@@ -773,7 +976,7 @@ __global__ void k_task_set_targets(Worlds<R> W, const __grid_constant__ TaskPara
 //                 ended worlds go to the ended-world list, which a separate
 //                 reset launch then takes;
 //   kWithResets   the same, and the group's ended worlds are reset in the
-//                 kernel too, one warp each.
+//                 kernel too, one after the other by the whole CTA.
 // The task functions are compiled once (not inlined) and called both from
 // the fused forms and from the separate task kernels, so their outputs do
 // not depend on the form. The physics is inlined into each instantiation:
@@ -783,12 +986,13 @@ __global__ void k_task_set_targets(Worlds<R> W, const __grid_constant__ TaskPara
 // physics source in another context and agree with it to FP32 rounding
 // rather than bit for bit. The ended-world list is filled in completion
 // order, as the separate task kernel fills it.
+static_assert(kResetThreads == wl::kThreads, "the fused form's CTA resets worlds");
 enum : int { kPhysics = 0, kWithTask = 1, kWithResets = 2 };
 
 struct ControlSmem {
     union {
         wl::Smem step;
-        ResetSmem reset[wl::kWarps];  // one per warp, after the group's step
+        ResetSmem reset;  // after the group's step
     };
     int ended[wl::kWorlds];  // worlds of the group whose episode ended
     int n_ended;
@@ -847,8 +1051,8 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
             if constexpr (kMode == kWithResets) {
                 __syncthreads();
 #pragma unroll 1
-                for (int e = leg; e < cs.n_ended; e += wl::kWarps)
-                    task_reset_world(cs.reset[leg], M, RM, W, tg, tgd, grid_of, cell, P, S, O.obs, cs.ended[e]);
+                for (int e = 0; e < cs.n_ended; ++e)
+                    task_reset_world(cs.reset, M, RM, W, tg, tgd, grid_of, cell, P, S, O.obs, cs.ended[e]);
             }
         }
         if (!queue)
@@ -953,7 +1157,7 @@ int reset_grid(int n)
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int cap = sms * 32;  // one warp per world, up to 32 resident per SM
+    const int cap = sms * kResetPerSm;
     return n < cap ? (n > 0 ? n : 1) : cap;
 }
 
@@ -1010,8 +1214,8 @@ cudaError_t launch_task_reset(const DevModel<R>& M, const ResetModel& RM, const 
     });
     if (e != cudaSuccess)
         return e;
-    k_task_reset<R><<<reset_grid(max_n), 32, sizeof(ResetSmem), stream>>>(M, RM, W, tg, tgd, grid_of, cell, P, S, obs,
-                                                                       ids, count_dev, max_n);
+    k_task_reset<R><<<reset_grid(max_n), kResetThreads, sizeof(ResetSmem), stream>>>(M, RM, W, tg, tgd, grid_of, cell, P,
+                                                                                  S, obs, ids, count_dev, max_n);
     return cudaGetLastError();
 }
 
@@ -1027,7 +1231,7 @@ cudaError_t launch_task_set_targets(const Worlds<R>& W, const TaskParams& P, con
 
 cudaError_t init_reset_tables(cudaStream_t stream)
 {
-    k_jump_init<<<kJumpBits, 128, 0, stream>>>();
+    k_skip_init<<<32, 128, 0, stream>>>();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
 }
@@ -1041,12 +1245,12 @@ cudaError_t launch_reset_warp(const ResetModel& RM, const Worlds<R>& W, TerrainG
         return cudaSuccess;
     static std::atomic<unsigned long long> configured{0};
     cudaError_t e = once_per_device(configured, [](int) {
-        return cudaFuncSetAttribute(k_reset_warp<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ResetSmem));
+        return cudaFuncSetAttribute(k_reset<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ResetSmem));
     });
     if (e != cudaSuccess)
         return e;
-    k_reset_warp<R><<<reset_grid(n_ids), 32, sizeof(ResetSmem), stream>>>(RM, W, tg, tgd, ids, n_ids, seeds,
-                                                                        difficulty, grid_of, cell);
+    k_reset<R><<<reset_grid(n_ids), kResetThreads, sizeof(ResetSmem), stream>>>(RM, W, tg, tgd, ids, n_ids, seeds,
+                                                                                 difficulty, grid_of, cell);
     return cudaGetLastError();
 }
 
