@@ -1466,11 +1466,8 @@ template <class R> int env_task_step(arc_sim* s, const float* actions, bool writ
     const Worlds<R> W = view<R>(s);
     if (check(s, cudaMemsetAsync(s->to.done_count, 0, sizeof(int), st), "memset done_count"))
         return ARC_ERR_CUDA;
-    if (check(s, launch_task_step<R>(dev_model<R>(s), W, s->tp, s->ts, s->to, actions, write_obs ? 2 : 0, st),
-              "task step kernel"))
-        return ARC_ERR_CUDA;
-    return write_obs ? check(s, launch_task_heights<R>(dev_model<R>(s), W, s->tp, s->to, st), "task heights kernel")
-                     : ARC_OK;
+    return check(s, launch_task_step<R>(dev_model<R>(s), W, s->tp, s->ts, s->to, actions, write_obs, st),
+                 "task step kernel");
 }
 
 template <class R> int env_reset_done(arc_sim* s, cudaStream_t st)
@@ -1807,9 +1804,8 @@ template <class R> int env_step_chunk(arc_sim* s, int first, int count, int c, c
     Actuation A{nullptr, s->actions};
     if (int rc = step_any(s, A, st, ids, count, part))
         return rc;
-    if (check(s, launch_task_step<R>(dev_model<R>(s), view<R>(s), s->tp, s->ts, O, s->actions, 2, st, first, count),
-              "task step kernel") ||
-        check(s, launch_task_heights<R>(dev_model<R>(s), view<R>(s), s->tp, O, st, first, count), "task heights kernel"))
+    if (check(s, launch_task_step<R>(dev_model<R>(s), view<R>(s), s->tp, s->ts, O, s->actions, true, st, first, count),
+              "task step kernel"))
         return ARC_ERR_CUDA;
     return check(s,
                  launch_task_reset<R>(dev_model<R>(s), s->rm, view<R>(s), (TerrainGeom<R>*)s->tg, s->tgd, s->grid_of,
@@ -2136,15 +2132,11 @@ int arc_env_step_ids(arc_sim* s, const int* d_ids, int n_ids, void* stream)
         return rc;
     if (check(s, cudaMemsetAsync(s->to.done_count, 0, sizeof(int), st), "memset done_count"))
         return ARC_ERR_CUDA;
-    cudaError_t e = s->fp64 ? launch_task_step<double>(s->md, view<double>(s), s->tp, s->ts, s->to, s->actions, 2, st,
+    cudaError_t e = s->fp64 ? launch_task_step<double>(s->md, view<double>(s), s->tp, s->ts, s->to, s->actions, true, st,
                                                        0, n_ids, d_ids)
-                            : launch_task_step<float>(s->mf, view<float>(s), s->tp, s->ts, s->to, s->actions, 2, st,
+                            : launch_task_step<float>(s->mf, view<float>(s), s->tp, s->ts, s->to, s->actions, true, st,
                                                       0, n_ids, d_ids);
     if (check(s, e, "task step kernel"))
-        return ARC_ERR_CUDA;
-    e = s->fp64 ? launch_task_heights<double>(s->md, view<double>(s), s->tp, s->to, st, 0, n_ids, d_ids)
-                : launch_task_heights<float>(s->mf, view<float>(s), s->tp, s->to, st, 0, n_ids, d_ids);
-    if (check(s, e, "task heights kernel"))
         return ARC_ERR_CUDA;
     return s->fp64 ? env_reset_done<double>(s, st) : env_reset_done<float>(s, st);
 }

@@ -130,42 +130,20 @@ __device__ __forceinline__ double unit(uint64_t x) { return (double)(x >> 11) * 
 __device__ __forceinline__ int key_of(const TaskState& S, int i) { return S.key ? (int)S.key[i] : i; }
 
 // ---------------------------------------------------------------------------
-// world read-out in FP64 (what arc_sim_observe returns, csrc/arc_sim.c:140-183)
+// world read-outs in FP64 (what arc_sim_observe returns, csrc/arc_sim.c:140-183)
 
-struct Obs64 {
-    V3<double> x, v, w;
-    Q4<double> q;
-    M3<double> rot;
-    double angle[kNumJoints], rate[kNumJoints], torque[kNumJoints];
-    double contact[kNumLegs + 2];
-    int unstable;
-};
-
+// The largest touch share of the spheres of one contact channel.
 template <class R>
-__device__ void read_world(const DevModel<R>& M, const Worlds<R>& W, int i, Obs64& o)
+__device__ __forceinline__ double contact_of(const DevModel<R>& M, const uint32_t* sph, int channel)
 {
-    const R* rec = W.rec + (size_t)i * W.stride;
-    o.x = V3<double>{(double)rec[0], (double)rec[1], (double)rec[2]};
-    o.q = Q4<double>{(double)rec[3], (double)rec[4], (double)rec[5], (double)rec[6]};
-    o.v = V3<double>{(double)rec[7], (double)rec[8], (double)rec[9]};
-    o.w = V3<double>{(double)rec[10], (double)rec[11], (double)rec[12]};
-    o.rot = m3_from_quat(o.q);
-    const R* jr = rec + W.off_joint;
-    for (int j = 0; j < kNumJoints; ++j) {
-        o.angle[j] = (double)jr[j * kJointRec + 1];
-        o.rate[j] = (double)jr[j * kJointRec + 2];
-        o.torque[j] = (double)jr[j * kJointRec + 3];
-    }
-    const uint32_t* sph = W.sph + (size_t)i * M.ns;
     const double inv = 1.0 / M.substeps;
-    for (int c = 0; c < kNumLegs + 2; ++c)
-        o.contact[c] = 0.0;
+    double c = 0.0;
     for (int s = 0; s < M.ns; ++s) {
-        double v = (int)(sph[s] & 0xffffu) * inv;
-        double& c = o.contact[M.channel[s]];
-        c = c > v ? c : v;
+        const double v = (int)(sph[s] & 0xffffu) * inv;
+        if (M.channel[s] == channel)
+            c = c > v ? c : v;
     }
-    o.unstable = W.unstable[i];
+    return c;
 }
 
 template <class R> __device__ __forceinline__ double height_at(const Worlds<R>& W, int i, double x, double y)
@@ -212,57 +190,72 @@ __device__ __forceinline__ void heading_of(Q4<double> q, double& cy, double& sy)
     sy = sin(yaw);
 }
 
-// Sample m of the 143 terrain heights around x in the heading frame; th, g:
-// world i's columns.
-template <class R>
-__device__ __forceinline__ double sample_height(const TaskParams& P, const Worlds<R>& W, int i, const TerrainGeomD& g,
-                                                const R* th, V3<double> x, double cy, double sy, int m)
+// a / b correctly rounded, y = 1 / b correctly rounded: the quotient from
+// the reciprocal, corrected twice by its exact remainder (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990). a / b infinite gives NaN.
+__device__ __forceinline__ double divide(double a, double b, double y)
 {
-    const double fo = P.offsets[m][0], lo = P.offsets[m][1];
-    const double px = x.x + cy * fo - sy * lo, py = x.y + sy * fo + cy * lo;
-    // csrc/arc_terrain.h:42-50
-    const double fx = floor((px - g.ox) / g.cell), fy = floor((py - g.oy) / g.cell);
-    const bool in = fx >= 0.0 && fy >= 0.0 && fx < g.nx && fy < g.ny &&
-                    terrain_column_ok(W, i, (int)fx + (long long)(int)fy * g.nx, kCheckHeightsRead);
-    const int idx = in ? (int)fx + (int)fy * g.nx : 0;
-    const double top = (double)th[idx];
-    return in ? top : g.outside;
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// Where a world's terrain heights are sampled (csrc/arc_sim.c:185-203): its
+// heading, position and columns.
+template <class R> struct HeightFrame {
+    double cy, sy, x, y;
+    double z;  // height of the standing torso's ground: x.z - stand_height
+    double cell, inv_cell, ox, oy, outside, nx, ny;
+    const R* th;
+    int pitch, world;
+};
+
+template <class R>
+__device__ __forceinline__ HeightFrame<R> height_frame(const TaskParams& P, const Worlds<R>& W, int i, V3<double> x,
+                                                       Q4<double> q)
+{
+    const TerrainGeomD g = W.tgd[i];
+    HeightFrame<R> f;
+    heading_of(q, f.cy, f.sy);
+    f.x = x.x;
+    f.y = x.y;
+    f.z = x.z - P.stand_height;
+    f.cell = g.cell;
+    f.inv_cell = 1.0 / g.cell;
+    f.ox = g.ox;
+    f.oy = g.oy;
+    f.outside = g.outside;
+    f.nx = g.nx;
+    f.ny = g.ny;
+    f.th = W.th + W.toff[i];
+    f.pitch = g.nx;
+    f.world = i;
+    return f;
+}
+
+// The height at (fo, lo) in the frame.
+template <class R>
+__device__ __forceinline__ double sample_height(const Worlds<R>& W, const HeightFrame<R>& f, double fo, double lo)
+{
+    const double px = f.x + f.cy * fo - f.sy * lo, py = f.y + f.sy * fo + f.cy * lo;
+    // csrc/arc_terrain.h:42-50: floor((p - o) / cell) in 0 .. n - 1, which
+    // the quotient itself decides
+    const double qx = divide(px - f.ox, f.cell, f.inv_cell), qy = divide(py - f.oy, f.cell, f.inv_cell);
+    const bool in = qx >= 0.0 && qy >= 0.0 && qx < f.nx && qy < f.ny &&
+                    terrain_column_ok(W, f.world, (int)qx + (long long)(int)qy * f.pitch, kCheckHeightsRead);
+    const int idx = in ? (int)qx + (int)qy * f.pitch : 0;
+    const double top = (double)f.th[idx];
+    return in ? top : f.outside;
 }
 
 // The observation's entry of a terrain height.
-__device__ __forceinline__ float height_value(const TaskParams& P, V3<double> x, double h)
+template <class R> __device__ __forceinline__ float height_value(const HeightFrame<R>& f, double h)
 {
-    const double rel = x.z - P.stand_height - h;
+    const double rel = f.z - h;
     return obs_value(rel < -1.0 ? -1.0 : (rel > 1.0 ? 1.0 : rel));
 }
 
-// Observation entries m_begin .. m_end - 1 of the 143 terrain heights,
-// written to dst[m - m_begin], kChunk samples at a time: their terrain loads
-// are all issued before any is used.
-template <int kChunk, class R>
-__device__ void write_heights(const TaskParams& P, const Worlds<R>& W, int i, V3<double> x, Q4<double> q, float* dst,
-                              int m_begin, int m_end)
-{
-    double cy, sy;
-    heading_of(q, cy, sy);
-    const TerrainGeomD g = W.tgd[i];
-    const R* th = W.th + W.toff[i];
-    int k = 0;
-    for (int m0 = m_begin; m0 < m_end; m0 += kChunk) {
-        double h[kChunk];
-#pragma unroll
-        for (int u = 0; u < kChunk; ++u)
-            h[u] = sample_height(P, W, i, g, th, x, cy, sy, m0 + u < m_end ? m0 + u : m_end - 1);
-#pragma unroll
-        for (int u = 0; u < kChunk; ++u) {
-            if (m0 + u >= m_end)
-                break;
-            dst[k++] = height_value(P, x, h[u]);
-        }
-    }
-}
-
-// arc/task.py:231-259: writes the 195 observation values of world i
 // The parts of an observation row (arc/task.py:231-259): entries 0..8 the
 // torso's, 9..44 the joints', 45..47 the checkpoint's, then the heights and
 // the feet's contacts.
@@ -299,23 +292,6 @@ __device__ __forceinline__ void obs_target(double c, double s, double dx, double
     row[kHeightsAt - 1] = obs_value((dist < 6.0 ? dist : 6.0) / 6.0);
 }
 
-template <class R>
-__device__ void write_obs(const TaskParams& P, const Worlds<R>& W, const TaskState& S, int i, const Obs64& o,
-                          float* dst, bool heights = true)
-{
-    const M3<double>& r = o.rot;
-    obs_torso(r, o.v, o.w, dst);
-    for (int j = 0; j < kNumJoints; ++j)
-        obs_joint(P, j, o.angle[j], o.rate[j], (double)S.prev_action[(size_t)i * kNumJoints + j], dst);
-    const double heading = atan2(r.m[1][0], r.m[0][0]);
-    const double dx = S.target[2 * i] - o.x.x, dy = S.target[2 * i + 1] - o.x.y;
-    obs_target(cos(heading), sin(heading), dx, dy, dst);
-    if (heights)
-        write_heights<8>(P, W, i, o.x, o.q, dst + kHeightsAt, 0, kNumOffsets);
-    for (int l = 0; l < kNumLegs; ++l)
-        dst[kHeightsAt + kNumOffsets + l] = obs_value(o.contact[l]);
-}
-
 // Checkpoint 3-6 m away inside the terrain (arc/task.py:127-151), drawn
 // from the device stream; also refreshes target_z, prev_dist, prev_gaze.
 template <class R>
@@ -347,22 +323,28 @@ __device__ void place_target(const TaskParams& P, const Worlds<R>& W, const Task
 }
 
 // ---------------------------------------------------------------------------
-// arc/task.py:155-220 (+ 231-259 for the observation): one thread per world
+// arc/task.py:155-220, and 231-259 for the observation: 32 worlds per CTA
 
-// One world's step of the task layer; returns whether its episode ended.
-// Compiled once (not inlined): the separate task kernel and the fused
-// control step run the same code.
-template <class R>
-__device__ __noinline__ bool task_step_world(const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P, const TaskState& S,
-                                const TaskOut& O, const float* __restrict__ actions, int write_obs_rows, int i)
+__device__ __forceinline__ double clip_action(float action)
 {
-    Obs64 o;
-    read_world(M, W, i, o);
+    const double a = (double)action;
+    return a < -1.0 ? -1.0 : (a > 1.0 ? 1.0 : a);
+}
+
+// One world's step of the task layer but its observation and stored action;
+// returns whether its episode ended. jr, sph: its joints' and spheres' records.
+template <class R>
+__device__ __forceinline__ bool task_step_world(const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P,
+                                                const TaskState& S, const TaskOut& O, const R* jr,
+                                                const uint32_t* sph, const float* action, const float* prev_action,
+                                                V3<double> x, Q4<double> q, V3<double> v, V3<double> w,
+                                                const M3<double>& rot, int i)
+{
     const int steps = S.steps[i] + 1;
     S.steps[i] = steps;
     const double* tgt = S.target + 2 * i;
-    const double dist = hypot(tgt[0] - o.x.x, tgt[1] - o.x.y);
-    const double gaze = gaze_error(o.rot, o.x, tgt);
+    const double dist = hypot(tgt[0] - x.x, tgt[1] - x.y);
+    const double gaze = gaze_error(rot, x, tgt);
     double view = (cos(gaze) - P.cos_fov) / (1.0 - P.cos_fov);
     view = view < 0.0 ? 0.0 : (view > 1.0 ? 1.0 : view);
     const bool in_view = gaze < P.fov_rad;
@@ -372,35 +354,31 @@ __device__ __noinline__ bool task_step_world(const DevModel<R>& M, const Worlds<
         progress = progress * view;
     const double turn = S.prev_gaze[i] - gaze;
     const bool reached = dist < P.checkpoint_radius && in_view;
-    const V3<double> br = rt_mul(o.rot, o.w);
-    const bool torso = o.contact[kNumLegs] > 0;
+    const V3<double> br = rt_mul(rot, w);
+    const bool torso = contact_of(M, sph, kNumLegs) > 0;
     const int torso_steps = torso ? S.torso_steps[i] + 1 : 0;
     S.torso_steps[i] = torso_steps;
     double power = 0.0, rate = 0.0;
-    float* pa = S.prev_action + (size_t)i * kNumJoints;
     for (int j = 0; j < kNumJoints; ++j) {
-        power += fabs(o.rate[j] * o.torque[j]);
-        double a = (double)actions[(size_t)i * kNumJoints + j];
-        a = a < -1.0 ? -1.0 : (a > 1.0 ? 1.0 : a);
-        const double d = a - (double)pa[j];
+        power += fabs((double)jr[j * kJointRec + 2] * (double)jr[j * kJointRec + 3]);
+        const double d = clip_action(action[j]) - (double)prev_action[j];
         rate += d * d;
-        pa[j] = (float)a;
     }
     double reward = P.w_progress * progress + P.w_turn * turn + P.w_checkpoint * (reached ? 1.0 : 0.0) - P.w_time -
                     P.w_energy * power * P.dt - P.w_action_rate * rate -
-                    P.w_body_contact * (o.contact[kNumLegs + 1] > 0 ? 1.0 : 0.0) -
+                    P.w_body_contact * (contact_of(M, sph, kNumLegs + 1) > 0 ? 1.0 : 0.0) -
                     P.w_torso_contact * (torso ? 1.0 : 0.0) - P.w_body_rate * (br.x * br.x + br.y * br.y) -
-                    P.w_bounce * (o.v.z * o.v.z);
+                    P.w_bounce * (v.z * v.z);
     bool finite = true;
     {
-        const double r13[13] = {o.x.x, o.x.y, o.x.z, o.q.w, o.q.x, o.q.y, o.q.z,
-                                o.v.x, o.v.y, o.v.z, o.w.x, o.w.y, o.w.z};
+        const double r13[13] = {x.x, x.y, x.z, q.w, q.x, q.y, q.z,
+                                v.x, v.y, v.z, w.x, w.y, w.z};
         for (int c = 0; c < 13; ++c)
             finite = finite && isfinite(r13[c]);
     }
-    const bool bad = o.unstable != 0 || !finite;
-    const bool vd = fabs(o.x.x) > P.half_extent || fabs(o.x.y) > P.half_extent || o.x.z < P.void_z;
-    const bool flip = o.rot.m[2][2] < P.flip_up_z;
+    const bool bad = W.unstable[i] != 0 || !finite;
+    const bool vd = fabs(x.x) > P.half_extent || fabs(x.y) > P.half_extent || x.z < P.void_z;
+    const bool flip = rot.m[2][2] < P.flip_up_z;
     const bool beached = torso_steps > P.beached_steps;
     const bool fell = flip || beached || vd || bad;
     const int cause = bad ? 1 : (vd ? 2 : (flip ? 3 : (beached ? 4 : 0)));
@@ -414,7 +392,7 @@ __device__ __noinline__ bool task_step_world(const DevModel<R>& M, const Worlds<
     const int checkpoints = S.checkpoints[i] + (reached ? 1 : 0);
     S.checkpoints[i] = checkpoints;
     if (reached && !fell)
-        place_target(P, W, S, i, o.x, o.rot);
+        place_target(P, W, S, i, x, rot);
     const bool truncated = steps >= P.max_steps && !fell;
     O.reward[i] = (float)reward;
     O.terminated[i] = fell;
@@ -436,85 +414,203 @@ __device__ __noinline__ bool task_step_world(const DevModel<R>& M, const Worlds<
         if (O.done_list)
             O.done_list[atomicAdd(O.done_count, 1)] = i;
     }
-    if (write_obs_rows && O.obs) {
-        float* row = O.obs + (size_t)i * kObsSize;
-        write_obs(P, W, S, i, o, row, write_obs_rows == 1);
-        if (done && O.terminal_obs) {
-            float* t = O.terminal_obs + (size_t)i * kObsSize;
-            for (int k = 0; k < kObsSize; ++k)
-                t[k] = row[k];
-        }
-    }
     return done;
 }
 
-// Worlds first + k (or ids[k]) for k < count, one thread each.
-template <class R>
-__global__ void k_task_step(const __grid_constant__ DevModel<R> M, Worlds<R> W, const __grid_constant__ TaskParams P,
-                            TaskState S, TaskOut O, const float* __restrict__ actions, int write_obs_rows, int first,
-                            int count, const int* __restrict__ ids)
+// What the task layer does with a group of worlds.
+enum : int {
+    kTaskStep = 0,     // the step, no observation
+    kTaskStepObs = 1,  // the step and the observation
+    kTaskObserve = 2,  // the observation alone
+};
+
+constexpr int kTaskWorlds = 32;
+constexpr int kTaskThreads = 128;
+
+constexpr int kTaskSpheres = 21;  // the quadruped's
+
+template <class R> struct TaskSmem {
+    HeightFrame<R> frame[kTaskWorlds];
+    double head_c[kTaskWorlds], head_s[kTaskWorlds];
+    double off[kNumOffsets][2];
+    int world[kTaskWorlds];
+    int done[kTaskWorlds];  // the world's episode ended in this step
+    // the worlds' records, copied in (odd row lengths: no bank conflicts)
+    R rec[kTaskWorlds][kBodyRec + kNumJoints * kJointRec];
+    uint32_t sph[kTaskWorlds][kTaskSpheres];
+    float action[kTaskWorlds][kNumJoints + 1], prev[kTaskWorlds][kNumJoints + 1];
+    // their observation rows but the heights: entries 0..47, the feet's contacts
+    float row[kTaskWorlds][kHeightsAt + kNumLegs + 1];
+};
+
+// The task layer on up to 32 worlds by the four warps of a CTA: lane j of
+// every warp has the same world (< 0: none). Warp 0 does the step (rewards,
+// terminations, the next checkpoint), warp 1 the torso's and the
+// checkpoint's entries, warp 2 the feet's and the frame the heights are
+// sampled in, warp 3 the joints'; then all threads sample the heights, on
+// consecutive entries of a row. Compiled once per mode (not inlined): the
+// task kernels and the fused control step run the same code. On return every
+// thread has passed a barrier after the last read of ts but done.
+//
+// Latency bound: a chain of FP64 functions per world, then scattered terrain
+// loads. One thread per world did all but the heights in 35 us whatever the
+// batch, each lane reading its own record and writing its own row 32 sectors
+// at a time; here the records come in and the rows go out through shared
+// memory, a lane per word, and the chain's parts run side by side. The
+// heights took another 79-102 us per 65,536 worlds in a kernel whose nine
+// threads per world each took the heading's arctangent, sine and cosine anew,
+// read the sample offsets from the constant bank at another address in every
+// lane, and divided twice; a warp per world keeps its offsets in registers
+// and has five samples in flight per lane (a thread per sample, with the
+// frame read from shared memory for each, took 70k cycles against 25k). Both
+// together: 65,536 worlds 205 -> 99 us, 4,096 48 -> 19 us, FP64 16,384 78 ->
+// 34 us; the observation alone of one world 42 -> 9 us.
+template <class R, int kMode>
+__device__ __noinline__ void task_group(TaskSmem<R>& ts, const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P,
+                                        const TaskState& S, const TaskOut& O, const float* __restrict__ actions,
+                                        int i)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count)
+    const int tid = threadIdx.x, role = tid / 32, lane = tid & 31;
+    if (role == 0)
+        ts.world[lane] = i;
+    if (kMode != kTaskStep)
+        for (int c = tid; c < 2 * kNumOffsets; c += kTaskThreads)
+            ts.off[c / 2][c % 2] = P.offsets[c / 2][c % 2];
+    __syncthreads();
+    // each warp copies eight worlds, four at a time: a lane per word
+    constexpr int kRec = kBodyRec + kNumJoints * kJointRec, kEach = kTaskWorlds / (kTaskThreads / 32);
+    static_assert(kRec > 32 && kRec <= 64 && kTaskSpheres <= 32 && kNumJoints <= 16, "words of a world per lane");
+#pragma unroll 1
+    for (int k0 = role * kEach; k0 < (role + 1) * kEach; k0 += 4) {
+        R lo[4], hi[4];
+        uint32_t sph[4];
+        float act[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int w = ts.world[k0 + u] < 0 ? 0 : ts.world[k0 + u];
+            const R* rec = W.rec + (size_t)w * W.stride;
+            const int c = lane + 32;
+            lo[u] = rec[lane < kBodyRec ? lane : W.off_joint + lane - kBodyRec];
+            hi[u] = c < kRec ? rec[W.off_joint + c - kBodyRec] : R(0);
+            sph[u] = lane < kTaskSpheres ? W.sph[(size_t)w * kTaskSpheres + lane] : 0u;
+            // lanes 0 .. 11: the stored action; 16 .. 27: the new one
+            act[u] = 0.0f;
+            if ((lane & 15) < kNumJoints && (lane < 16 || kMode != kTaskObserve))
+                act[u] = (lane < 16 ? S.prev_action : actions)[(size_t)w * kNumJoints + (lane & 15)];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            ts.rec[k0 + u][lane] = lo[u];
+            if (lane + 32 < kRec)
+                ts.rec[k0 + u][lane + 32] = hi[u];
+            if (lane < kTaskSpheres)
+                ts.sph[k0 + u][lane] = sph[u];
+            if ((lane & 15) < kNumJoints)
+                (lane < 16 ? ts.prev : ts.action)[k0 + u][lane & 15] = act[u];
+        }
+    }
+    __syncthreads();
+    V3<double> x{0.0, 0.0, 0.0};
+    if (i >= 0) {
+        const R* rec = ts.rec[lane];
+        const R* jr = rec + kBodyRec;
+        float* row = ts.row[lane];
+        x = V3<double>{(double)rec[0], (double)rec[1], (double)rec[2]};
+        const Q4<double> q{(double)rec[3], (double)rec[4], (double)rec[5], (double)rec[6]};
+        if (role <= 1) {
+            const V3<double> v{(double)rec[7], (double)rec[8], (double)rec[9]};
+            const V3<double> w{(double)rec[10], (double)rec[11], (double)rec[12]};
+            const M3<double> rot = m3_from_quat(q);
+            if (role == 0) {
+                if (kMode != kTaskObserve)
+                    ts.done[lane] = task_step_world(M, W, P, S, O, jr, ts.sph[lane], ts.action[lane], ts.prev[lane],
+                                                    x, q, v, w, rot, i);
+            } else if (kMode != kTaskStep) {
+                obs_torso(rot, v, w, row);
+                const double heading = atan2(rot.m[1][0], rot.m[0][0]);
+                ts.head_c[lane] = cos(heading);
+                ts.head_s[lane] = sin(heading);
+            }
+        } else if (kMode != kTaskStep) {
+            if (role == 2) {
+                ts.frame[lane] = height_frame(P, W, i, x, q);
+                for (int l = 0; l < kNumLegs; ++l)
+                    row[kHeightsAt + l] = obs_value(contact_of(M, ts.sph[lane], l));
+            } else {
+                for (int j = 0; j < kNumJoints; ++j)  // the action as the step stores it
+                    obs_joint(P, j, (double)jr[j * kJointRec + 1], (double)jr[j * kJointRec + 2],
+                              kMode == kTaskObserve ? (double)ts.prev[lane][j]
+                                                    : (double)(float)clip_action(ts.action[lane][j]),
+                              row);
+            }
+        }
+    } else if (role == 0) {
+        ts.done[lane] = 0;
+    }
+    __syncthreads();
+    if (kMode != kTaskObserve)
+        for (int t = tid; t < kTaskWorlds * kNumJoints; t += kTaskThreads) {
+            const int k = t / kNumJoints, c = t % kNumJoints, w = ts.world[k];
+            if (w >= 0)
+                S.prev_action[(size_t)w * kNumJoints + c] = (float)clip_action(ts.action[k][c]);
+        }
+    if (kMode == kTaskStep)
         return;
-    task_step_world(M, W, P, S, O, actions, write_obs_rows, ids ? ids[k] : first + k);
-}
-
-// The observations' terrain heights of worlds first .. first + count - 1,
-// kHeightsPer samples per thread (k_task_step, with write_obs_rows == 2,
-// writes the rest of each row): the 143 samples of a world spread over nine
-// threads instead of one, four loads in flight per thread and registers sized
-// for eight blocks per SM (the kernel waits on latency: occupancy pays more
-// than loads in flight). Rows of worlds that ended this step get them in
-// their terminal observation too.
-constexpr int kHeightsPer = 16;
-constexpr int kHeightParts = (kNumOffsets + kHeightsPer - 1) / kHeightsPer;
-
-constexpr int kHeightThreads = 128;
-constexpr int kHeightBlocks = 8;
-
-// Part `part` (kHeightsPer samples) of world i's observation heights
-// (compiled once, as task_step_world).
-template <class R>
-__device__ __noinline__ void task_heights_part(const Worlds<R>& W, const TaskParams& P, const TaskOut& O, int i,
-                                                  int part)
-{
-    const int m0 = part * kHeightsPer, m1 = m0 + kHeightsPer < kNumOffsets ? m0 + kHeightsPer : kNumOffsets;
-    const R* b0 = W.rec + (size_t)i * W.stride;  // the torso's pose, as read_world reads it
-    const V3<double> x{(double)b0[0], (double)b0[1], (double)b0[2]};
-    const Q4<double> q{(double)b0[3], (double)b0[4], (double)b0[5], (double)b0[6]};
-    float* row = O.obs + (size_t)i * kObsSize + kHeightsAt;
-    write_heights<4>(P, W, i, x, q, row + m0, m0, m1);
-    if (O.terminal_obs && (O.terminated[i] | O.truncated[i])) {
-        float* t_row = O.terminal_obs + (size_t)i * kObsSize + kHeightsAt;
-        for (int m = m0; m < m1; ++m)
-            t_row[m] = row[m];
+    if (role == 1 && i >= 0)
+        obs_target(ts.head_c[lane], ts.head_s[lane], S.target[2 * i] - x.x, S.target[2 * i + 1] - x.y, ts.row[lane]);
+    // the heights: a warp per world, a lane's five samples (the last of some
+    // lanes is none) side by side
+    constexpr int kEachLane = (kNumOffsets + 31) / 32;
+    double fo[kEachLane], lo[kEachLane];
+#pragma unroll
+    for (int u = 0; u < kEachLane; ++u) {
+        const int m = lane + 32 * u < kNumOffsets ? lane + 32 * u : kNumOffsets - 1;
+        fo[u] = ts.off[m][0];
+        lo[u] = ts.off[m][1];
+    }
+#pragma unroll 1
+    for (int k = role; k < kTaskWorlds; k += kTaskThreads / 32) {
+        if (ts.world[k] < 0)
+            continue;
+        const HeightFrame<R> f = ts.frame[k];
+        float* dst = O.obs + (size_t)ts.world[k] * kObsSize + kHeightsAt + lane;
+        double h[kEachLane];
+#pragma unroll
+        for (int u = 0; u < kEachLane; ++u)
+            h[u] = sample_height(W, f, fo[u], lo[u]);
+#pragma unroll
+        for (int u = 0; u < kEachLane; ++u)
+            if (lane + 32 * u < kNumOffsets)
+                dst[32 * u] = height_value(f, h[u]);
+    }
+    __syncthreads();
+    for (int t = tid; t < kTaskWorlds * (kHeightsAt + kNumLegs); t += kTaskThreads) {
+        const int k = t / (kHeightsAt + kNumLegs), c = t % (kHeightsAt + kNumLegs);
+        if (ts.world[k] >= 0)
+            O.obs[(size_t)ts.world[k] * kObsSize + (c < kHeightsAt ? c : c + kNumOffsets)] = ts.row[k][c];
+    }
+    __syncthreads();
+    if (kMode == kTaskStepObs && O.terminal_obs) {
+        // the ended worlds' rows, a warp each
+        for (int k = role; k < kTaskWorlds; k += kTaskThreads / 32)
+            if (ts.done[k]) {
+                const size_t at = (size_t)ts.world[k] * kObsSize;
+                for (int c = lane; c < kObsSize; c += 32)
+                    O.terminal_obs[at + c] = O.obs[at + c];
+            }
+        __syncthreads();
     }
 }
 
-template <class R>
-__global__ void __launch_bounds__(kHeightThreads, kHeightBlocks)
-    k_task_heights(const __grid_constant__ DevModel<R> M, Worlds<R> W, const __grid_constant__ TaskParams P, TaskOut O,
-                   int first, int count, const int* __restrict__ ids)
+// Worlds first + k (or ids[k]; neither: k) for k < count.
+template <class R, int kMode>
+__global__ void __launch_bounds__(kTaskThreads)
+k_task(const __grid_constant__ DevModel<R> M, Worlds<R> W, const __grid_constant__ TaskParams P, TaskState S,
+       TaskOut O, const float* __restrict__ actions, int first, int count, const int* __restrict__ ids)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)count * kHeightParts)
-        return;
-    const int k = (int)(t / kHeightParts);
-    task_heights_part(W, P, O, ids ? ids[k] : first + k, (int)(t % kHeightParts));
-}
-
-template <class R>
-__global__ void k_task_observe(const __grid_constant__ DevModel<R> M, Worlds<R> W, const __grid_constant__ TaskParams P,
-                               TaskState S, float* obs, const int* __restrict__ ids, int n)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n)
-        return;
-    const int i = ids ? ids[k] : k;
-    Obs64 o;
-    read_world(M, W, i, o);
-    write_obs(P, W, S, i, o, obs + (size_t)i * kObsSize);
+    __shared__ TaskSmem<R> ts;
+    const int k = blockIdx.x * kTaskWorlds + (threadIdx.x & 31);
+    task_group<R, kMode>(ts, M, W, P, S, O, actions, k < count ? (ids ? ids[k] : first + k) : -1);
 }
 
 // ---------------------------------------------------------------------------
@@ -623,17 +719,6 @@ __device__ __forceinline__ unsigned long long scan_cells(double reach, double st
             outside = true;
     }
     return mask;
-}
-
-// a / 0.03 correctly rounded: the quotient from the reciprocal, corrected
-// twice by its exact remainder (Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990).
-__device__ __forceinline__ double over_step(double a)
-{
-    constexpr double b = 0.03, y = 1.0 / 0.03;
-    double q = __dmul_rn(a, y);
-    q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
 // A lattice's interpolation along x at row gy, and between two rows: the
@@ -796,7 +881,7 @@ __device__ __forceinline__ void reset_world(ResetSmem& sm, const ResetModel& RM,
                                            __dmul_rn(amp2, noise_between(top2, bot2, sm.frac[1][iy0 + k])));
                 const double jitter = __fma_rn((double)*dr, 2.0 / 4294967296.0, -1.0);
                 const double hj = __dadd_rn(v, __dmul_rn(ampj, jitter));
-                const double top = __dmul_rn(0.03, floor(__dadd_rn(over_step(hj), 0.5)));
+                const double top = __dmul_rn(0.03, floor(__dadd_rn(divide(hj, 0.03, 1.0 / 0.03), 0.5)));
                 const double hf = __dsub_rn(top, base);
                 *col = (R)hf;
                 if ((below >> k) & 1)
@@ -918,12 +1003,9 @@ __device__ __noinline__ void task_reset_world(ResetSmem& sm, const DevModel<R>& 
                           V3<double>{(double)b0[10], (double)b0[11], (double)b0[12]}, row);
         }
     } else if (row) {
-        double cy, sy;
-        heading_of(q, cy, sy);
-        const TerrainGeomD g = W.tgd[i];
-        const R* th = W.th + W.toff[i];
+        const HeightFrame<R> f = height_frame(P, W, i, x, q);
         for (int m = tid - 64; m < kNumOffsets; m += kResetThreads - 64)
-            row[kHeightsAt + m] = height_value(P, x, sample_height(P, W, i, g, th, x, cy, sy, m));
+            row[kHeightsAt + m] = height_value(f, sample_height(W, f, P.offsets[m][0], P.offsets[m][1]));
     }
     __syncthreads();  // the next world's reset reuses sm
 }
@@ -971,9 +1053,7 @@ __global__ void k_task_set_targets(Worlds<R> W, const __grid_constant__ TaskPara
 //   kPhysics      the step alone (arc_sim_step, the separate env step, tiles
 //                 of substeps);
 //   kWithTask     each CTA steps a group of 32 worlds, then, before its next
-//                 group, runs the task step on them (warp 0, one lane per
-//                 world) and their observations' heights (all threads); the
-//                 ended worlds go to the ended-world list, which a separate
+//                 group, runs the task layer on them (task_group); the ended worlds go to the ended-world list, which a separate
 //                 reset launch then takes;
 //   kWithResets   the same, and the group's ended worlds are reset in the
 //                 kernel too, one after the other by the whole CTA.
@@ -992,7 +1072,8 @@ enum : int { kPhysics = 0, kWithTask = 1, kWithResets = 2 };
 struct ControlSmem {
     union {
         wl::Smem step;
-        ResetSmem reset;  // after the group's step
+        TaskSmem<float> task;  // after the group's step
+        ResetSmem reset;       // after the task layer
     };
     int ended[wl::kWorlds];  // worlds of the group whose episode ended
     int n_ended;
@@ -1031,23 +1112,15 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
         wl::step_group(cs.step, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, group, tid, leg, j, sub0, sub1,
                        tile_q, per_group, list);
         if constexpr (kMode != kPhysics) {
+            // arc/task.py:155-259
+            const int world = world_of(group * wl::kWorlds + j);
+            __syncthreads();  // warp 0 has read the step's shared memory for the last time
+            task_group<float, kTaskStepObs>(cs.task, M, W, P, S, O, A.actions32, world);
             if (tid == 0)
                 cs.n_ended = 0;
             __syncthreads();
-            // arc/task.py:155-259 but the heights; warp 0's lane j takes the
-            // world its own lane stepped as leg 0 (time and unstable written by it)
-            if (tid < wl::kWorlds) {
-                const int world = world_of(group * wl::kWorlds + j);
-                if (world >= 0 && task_step_world(M, W, P, S, O, A.actions32, 2, world))
-                    cs.ended[atomicAdd(&cs.n_ended, 1)] = world;
-            }
-            __syncthreads();
-#pragma unroll 1
-            for (int t = tid; t < wl::kWorlds * kHeightParts; t += wl::kThreads) {
-                const int world = world_of(group * wl::kWorlds + t / kHeightParts);
-                if (world >= 0)
-                    task_heights_part(W, P, O, world, t % kHeightParts);
-            }
+            if (tid < wl::kWorlds && cs.task.done[j])
+                cs.ended[atomicAdd(&cs.n_ended, 1)] = world;
             if constexpr (kMode == kWithResets) {
                 __syncthreads();
 #pragma unroll 1
@@ -1165,28 +1238,18 @@ int reset_grid(int n)
 
 template <class R>
 cudaError_t launch_task_step(const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P, const TaskState& S,
-                             const TaskOut& O, const float* actions, int write_obs_rows, cudaStream_t stream, int first,
+                             const TaskOut& O, const float* actions, bool write_obs, cudaStream_t stream, int first,
                              int count, const int* ids)
 {
     if (count < 0)
         count = W.n - first;
     if (count <= 0 || (!ids && (first < 0 || first + count > W.n)))
         return count == 0 ? cudaSuccess : cudaErrorInvalidValue;
-    k_task_step<R><<<(count + 127) / 128, 128, 0, stream>>>(M, W, P, S, O, actions, write_obs_rows, first, count, ids);
-    return cudaGetLastError();
-}
-
-template <class R>
-cudaError_t launch_task_heights(const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P, const TaskOut& O,
-                                cudaStream_t stream, int first, int count, const int* ids)
-{
-    if (count < 0)
-        count = W.n - first;
-    if (count <= 0 || (!ids && (first < 0 || first + count > W.n)))
-        return count == 0 ? cudaSuccess : cudaErrorInvalidValue;
-    const long long threads = (long long)count * kHeightParts;
-    k_task_heights<R><<<(unsigned)((threads + kHeightThreads - 1) / kHeightThreads), kHeightThreads, 0, stream>>>(
-        M, W, P, O, first, count, ids);
+    const int grid = (count + kTaskWorlds - 1) / kTaskWorlds;
+    if (write_obs && O.obs)
+        k_task<R, kTaskStepObs><<<grid, kTaskThreads, 0, stream>>>(M, W, P, S, O, actions, first, count, ids);
+    else
+        k_task<R, kTaskStep><<<grid, kTaskThreads, 0, stream>>>(M, W, P, S, O, actions, first, count, ids);
     return cudaGetLastError();
 }
 
@@ -1196,7 +1259,10 @@ cudaError_t launch_task_observe(const DevModel<R>& M, const Worlds<R>& W, const 
 {
     if (n_ids <= 0)
         return cudaSuccess;
-    k_task_observe<R><<<(n_ids + 127) / 128, 128, 0, stream>>>(M, W, P, S, obs, ids, n_ids);
+    TaskOut O{};
+    O.obs = obs;
+    k_task<R, kTaskObserve><<<(n_ids + kTaskWorlds - 1) / kTaskWorlds, kTaskThreads, 0, stream>>>(
+        M, W, P, S, O, nullptr, 0, n_ids, ids);
     return cudaGetLastError();
 }
 
@@ -1312,10 +1378,8 @@ cudaError_t launch_step_warps(const DevModel<float>& M, const Worlds<float>& W, 
 
 #define ARC_INSTANTIATE_TASK(R)                                                                                    \
     template cudaError_t launch_task_step<R>(const DevModel<R>&, const Worlds<R>&, const TaskParams&,            \
-                                             const TaskState&, const TaskOut&, const float*, int, cudaStream_t,  \
+                                             const TaskState&, const TaskOut&, const float*, bool, cudaStream_t, \
                                              int, int, const int*);                                              \
-    template cudaError_t launch_task_heights<R>(const DevModel<R>&, const Worlds<R>&, const TaskParams&,         \
-                                                const TaskOut&, cudaStream_t, int, int, const int*);             \
     template cudaError_t launch_task_observe<R>(const DevModel<R>&, const Worlds<R>&, const TaskParams&,         \
                                                 const TaskState&, float*, const int*, int, cudaStream_t);        \
     template cudaError_t launch_task_reset<R>(const DevModel<R>&, const ResetModel&, const Worlds<R>&,           \

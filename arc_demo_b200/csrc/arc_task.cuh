@@ -67,15 +67,10 @@ struct TaskOut {
 template <class R>
 // Worlds first .. first + count - 1 (count < 0: to the last world), or with
 // ids the count worlds ids[0 .. count) (device array).
-// write_obs: 0 no observation rows, 1 whole rows, 2 rows without the terrain
-// heights, which launch_task_heights then writes with more threads.
+// write_obs: their observation rows too.
 cudaError_t launch_task_step(const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P, const TaskState& S,
-                             const TaskOut& O, const float* actions, int write_obs, cudaStream_t stream, int first = 0,
+                             const TaskOut& O, const float* actions, bool write_obs, cudaStream_t stream, int first = 0,
                              int count = -1, const int* ids = nullptr);
-
-template <class R>
-cudaError_t launch_task_heights(const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P, const TaskOut& O,
-                                cudaStream_t stream, int first = 0, int count = -1, const int* ids = nullptr);
 
 template <class R>
 cudaError_t launch_task_observe(const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P, const TaskState& S,
@@ -98,8 +93,7 @@ cudaError_t launch_task_reset(const DevModel<R>& M, const ResetModel& RM, const 
 // launches) one wave of resident CTAs takes the groups. O.done_count must be
 // zero before the launch. Without resets the ended worlds are only listed
 // (O.done_list), for launch_task_reset. The results equal launch_step_warps,
-// launch_task_step (write_obs 2), launch_task_heights and launch_task_reset
-// over O.done_list in turn to FP32 rounding: the task functions are compiled
+// launch_task_step with observations and launch_task_reset over O.done_list in turn to FP32 rounding: the task functions are compiled
 // once, and the physics is the same source compiled into this form's kernel.
 cudaError_t launch_control_step(const DevModel<float>& M, const ResetModel& RM, const Worlds<float>& W,
                                 TerrainGeom<float>* tg, TerrainGeomD* tgd, const int* grid_of, double cell,

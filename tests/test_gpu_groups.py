@@ -37,3 +37,38 @@ def test_small_batches_equal_large(fp64):
         for queue in (False, True):
             got = _states(n, fp64, queue)
             assert np.array_equal(got, whole[: len(got)]), (n, queue)
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+def test_task_rows_do_not_depend_on_the_batch(fp64):
+    # the task kernel takes 32 worlds per CTA, four at a time: one world, a
+    # partly filled CTA, one world in the last CTA; and the row that a step
+    # writes is the row that an observation of the same state gives. Bitwise
+    import torch
+    from arc_demo_b200.task import TaskConfig
+    from arc_demo_b200.torch_env import DeviceVecEnv
+
+    acts = torch.rand((2, 97, 12), generator=torch.Generator().manual_seed(3)).mul_(2).sub_(1).cuda()
+
+    def rows(n):
+        env = DeviceVecEnv(n, TaskConfig(curriculum=False, max_steps=2), seed=11, fp64=fp64)
+        env.set_levels(np.linspace(0.0, 1.0, 97)[:n])
+        env.reset()
+        out = []
+        for k in range(2):  # every episode ends at the second step
+            obs, reward, _, truncated = env.step(acts[k, :n])
+            out += [obs.clone(), reward.clone(), truncated.clone()]
+            if k == 0:
+                env.sim._check(env.gpu.lib.arc_env_observe(env.sim.ptr, None))
+                env.sim.synchronize()
+                assert torch.equal(env.obs, out[0])
+        out.append(env.terminal_obs.clone())
+        assert int(env.done_count[0]) == n
+        torch.cuda.synchronize()
+        env.close()
+        return out
+
+    whole = rows(97)
+    for n in (1, 31, 32, 33, 65):
+        for a, b in zip(rows(n), whole):
+            assert torch.equal(a, b[:n])
