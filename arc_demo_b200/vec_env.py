@@ -21,7 +21,39 @@ tensors):
 
 from __future__ import annotations
 
+import ctypes
+import functools
+
 import torch
+
+_vp, _dbl, _int = ctypes.c_void_p, ctypes.c_double, ctypes.c_int
+
+
+class _NormArgs(ctypes.Structure):
+    """arc_norm_step_args of include/arc_sim.h."""
+    _fields_ = ([("rows", ctypes.c_longlong)] + [(k, _int) for k in ("cols", "training", "norm_obs", "norm_reward")]
+                + [(k, _vp) for k in ("obs", "terminal_obs", "rewards", "dones", "returns", "obs_mean", "obs_var",
+                                      "ret_mean", "ret_var")]
+                + [(k, _dbl) for k in ("obs_count", "ret_count", "gamma", "epsilon", "clip_obs", "clip_reward")]
+                + [(k, _vp) for k in ("obs_out", "terminal_out", "rewards_out", "returns_out", "obs_mean_out",
+                                      "obs_var_out", "ret_mean_out", "ret_var_out", "work")])
+
+
+@functools.cache
+def _norm_lib():
+    from .native import sim_lib
+    lib = sim_lib()
+    lib.arc_norm_work_size.restype, lib.arc_norm_work_size.argtypes = ctypes.c_longlong, [ctypes.c_longlong, _int]
+    lib.arc_norm_step.restype, lib.arc_norm_step.argtypes = _int, [ctypes.POINTER(_NormArgs), _vp]
+    return lib
+
+
+def _plain(x, dtype, shape, device) -> bool:
+    """Whether the kernels can read x: a contiguous CUDA tensor of that type,
+    shape and device, with nothing recorded or transformed about it."""
+    return (type(x) is torch.Tensor and x.dtype == dtype and tuple(x.shape) == shape and x.device == device
+            and x.is_contiguous() and not x.requires_grad and not x.is_neg() and not x.is_inference()
+            and torch._C._functorch.maybe_get_level(x) == -1 and not torch.compiler.is_compiling())
 
 
 class DeviceRunningMeanStd:
@@ -73,9 +105,9 @@ class DeviceVecEnvAdapter:
 
     def step_wait(self):
         obs, reward, terminated, truncated = self.env.step(self._actions)
-        dones = terminated.bool() | truncated.bool()
-        infos = {"terminal_observation": self.env.terminal_obs, "truncated": truncated.bool() & ~terminated.bool()}
-        return obs, reward, dones, infos
+        term, trunc = terminated.bool(), truncated.bool()
+        infos = {"terminal_observation": self.env.terminal_obs, "truncated": trunc & ~term}
+        return obs, reward, term | trunc, infos
 
     def step(self, actions: torch.Tensor):
         self.step_async(actions)
@@ -131,6 +163,9 @@ class DeviceVecNormalize:
         obs, rewards, dones, infos = self.venv.step_wait()
         self._init_stats(obs)
         self.old_obs, self.old_reward = obs, rewards
+        done = self._step_kernels(obs, rewards, dones, infos)
+        if done is not None:
+            return done
         if self.training and self.norm_obs:
             self.obs_rms.update(obs)
         norm_obs = self.normalize_obs(obs)
@@ -142,6 +177,55 @@ class DeviceVecNormalize:
         if "terminal_observation" in infos:
             infos["terminal_observation"] = self.normalize_obs(infos["terminal_observation"])
         self.returns = torch.where(dones.bool(), torch.zeros_like(self.returns), self.returns)
+        return norm_obs, norm_rewards, dones, infos
+
+    def _step_kernels(self, obs, rewards, dones, infos):
+        """step_wait's statistics and normalisation by the library's kernels
+        (arc_norm_step): what it returns, or None where the tensors are not
+        ones they take (not on a CUDA device, other types, empty, recorded by
+        autograd, ...), which the tensor operations below handle. Like them it
+        leaves every tensor it was given or handed out before as it was."""
+        if type(obs) is not torch.Tensor or obs.device.type != "cuda" or obs.dim() != 2 or not obs.numel():
+            return None
+        n, cols = obs.shape
+        dev, f32, f64 = obs.device, torch.float32, torch.float64
+        term = infos.get("terminal_observation") if type(infos) is dict else None
+        rms, ret = self.obs_rms, self.ret_rms
+        if (cols > 2048 or n != self.num_envs or type(infos) is not dict
+                or not _plain(obs, f32, (n, cols), dev) or not _plain(rewards, f32, (n,), dev)
+                or not _plain(dones, torch.bool, (n,), dev) or not _plain(self.returns, f64, (n,), dev)
+                or not all(_plain(t, f64, (cols,), dev) for t in (rms.mean, rms.var))
+                or not all(_plain(t, f64, (), dev) for t in (ret.mean, ret.var))
+                or ("terminal_observation" in infos and not _plain(term, f32, (n, cols), dev))):
+            return None
+        lib = _norm_lib()
+        with torch.cuda.device(dev):
+            work = torch.empty(lib.arc_norm_work_size(n, cols) if self.training else 1, dtype=f64, device=dev)
+            returns, mean, var, ret_stats = torch.empty(n + 2 * cols + 2, dtype=f64, device=dev).split(
+                [n, cols, cols, 2])
+            norm_obs = torch.empty_like(obs) if self.norm_obs else obs
+            norm_term = torch.empty_like(term) if self.norm_obs and term is not None else term
+            norm_rewards = torch.empty_like(rewards) if self.norm_reward else rewards
+            args = _NormArgs(
+                n, cols, bool(self.training), bool(self.norm_obs), bool(self.norm_reward), obs.data_ptr(),
+                None if term is None else term.data_ptr(), rewards.data_ptr(), dones.data_ptr(),
+                self.returns.data_ptr(), rms.mean.data_ptr(), rms.var.data_ptr(), ret.mean.data_ptr(),
+                ret.var.data_ptr(), rms.count, ret.count, self.gamma, self.epsilon, self.clip_obs, self.clip_reward,
+                norm_obs.data_ptr() if self.norm_obs else None,
+                norm_term.data_ptr() if self.norm_obs and term is not None else None, norm_rewards.data_ptr(),
+                returns.data_ptr(), mean.data_ptr(), var.data_ptr(), ret_stats.data_ptr(), ret_stats[1:].data_ptr(),
+                work.data_ptr())
+            stream = torch.cuda.current_stream(dev).cuda_stream
+            if lib.arc_norm_step(ctypes.byref(args), stream or 1):  # 1: the legacy default stream
+                raise RuntimeError("arc_norm_step failed")
+        if self.training:
+            if self.norm_obs:
+                rms.mean, rms.var, rms.count = mean, var, rms.count + n
+            ret.mean, ret.var, ret.count = ret_stats[0], ret_stats[1], ret.count + n
+        self.returns = returns
+        infos = dict(infos)
+        if term is not None:
+            infos["terminal_observation"] = norm_term
         return norm_obs, norm_rewards, dones, infos
 
     def step(self, actions: torch.Tensor):

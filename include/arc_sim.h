@@ -415,6 +415,32 @@ int arc_env_set_task_state(arc_sim *s, const int *ids, int n_ids, const double *
 /* Places checkpoints at given points (target_z, prev_dist, prev_gaze follow). */
 int arc_env_set_targets(arc_sim *s, const int *ids, int n_ids, const double *xy);
 
+/* ---- running normalisation of a training loop's batch (Stable-Baselines3's
+ * VecNormalize, scripts/train.py:116-142): one step on the device. rows x
+ * cols float32 observations, rows rewards and done flags (bytes), rows FP64
+ * discounted returns. With training, the returns become returns * gamma +
+ * rewards, and the batch's moments are merged into the running mean and
+ * variance of the observations (norm_obs) and of the returns, from the *_in
+ * statistics over obs_count and ret_count samples to the *_out ones (which
+ * then hold rows more). Written: the observations and terminal observations
+ * ((x - mean) / sqrt(var + epsilon), clipped to +-clip_obs; NULL outputs: not
+ * written), with norm_reward the rewards (r / sqrt(ret_var + epsilon),
+ * clipped), and the returns, zero where done. No output may alias an input.
+ * work: arc_norm_work_size(rows, cols) doubles. cols <= 2048. Device
+ * pointers; asynchronous on `stream`. Returns a status code. */
+typedef struct arc_norm_step_args {
+    long long rows;
+    int cols, training, norm_obs, norm_reward;
+    const float *obs, *terminal_obs, *rewards;
+    const unsigned char *dones;
+    const double *returns, *obs_mean, *obs_var, *ret_mean, *ret_var;
+    double obs_count, ret_count, gamma, epsilon, clip_obs, clip_reward;
+    float *obs_out, *terminal_out, *rewards_out;
+    double *returns_out, *obs_mean_out, *obs_var_out, *ret_mean_out, *ret_var_out, *work;
+} arc_norm_step_args;
+long long arc_norm_work_size(long long rows, int cols);
+int arc_norm_step(const arc_norm_step_args *a, void *stream);
+
 /* ---- serving engine. No counterpart in the reference, which steps one
  * synchronous batch per call. A fixed pool of `capacity` world slots (the
  * device-memory budget) with the task layer, and one engine thread doing

@@ -1,0 +1,98 @@
+"""DeviceVecNormalize's kernels (arc_norm_step) against its tensor operations
+on the same batches: one column, ragged tiles of 256 columns and blocks of 32
+rows, every combination of its switches, values that are not finite."""
+
+import itertools
+
+import pytest
+import torch
+
+from arc_demo_b200.vec_env import DeviceVecNormalize
+
+pytestmark = pytest.mark.gpu
+
+
+class Env:
+    """Random batches (column 0 constant), the same for the same seed."""
+
+    def __init__(self, n, cols, bad=False):
+        self.num_envs, self.cols, self.bad = n, cols, bad
+        self.g = torch.Generator(device="cuda").manual_seed(1000 * n + cols)
+
+    def _obs(self):
+        x = torch.randn((self.num_envs, self.cols), device="cuda", generator=self.g)
+        x = x * torch.logspace(-3, 3, self.cols, device="cuda") + torch.linspace(-50, 50, self.cols, device="cuda")
+        x[:, 0] = 7.25
+        if self.bad:
+            x[0, 1], x[1, 2], x[2, 3] = float("inf"), float("nan"), float("-inf")
+        return x
+
+    def reset(self):
+        return self._obs()
+
+    def step_async(self, actions):
+        pass
+
+    def step_wait(self):
+        r = torch.randn(self.num_envs, device="cuda", generator=self.g) * 3 + 1
+        d = torch.rand(self.num_envs, device="cuda", generator=self.g) < 0.2
+        return self._obs(), r, d, {"terminal_observation": self._obs(), "truncated": d}
+
+
+class Tensors(DeviceVecNormalize):
+    def _step_kernels(self, *a):
+        return None
+
+
+def _close(a, b, rel):
+    assert a.dtype == b.dtype and a.shape == b.shape
+    assert torch.equal(torch.isnan(a), torch.isnan(b))
+    assert torch.allclose(a, b, rtol=rel, atol=rel, equal_nan=True), (a - b).abs().max()
+
+
+@pytest.mark.parametrize("n,cols", [(1, 1), (2, 195), (33, 5), (1000, 195), (8195, 256), (300, 300), (40, 2048)])
+@pytest.mark.parametrize("training,norm_obs,norm_reward", list(itertools.product([True, False], repeat=3)))
+def test_kernels_equal_tensor_operations(n, cols, training, norm_obs, norm_reward):
+    kw = dict(training=training, norm_obs=norm_obs, norm_reward=norm_reward)
+    a, b = DeviceVecNormalize(Env(n, cols), **kw), Tensors(Env(n, cols), **kw)
+    a.reset(), b.reset()
+    assert a._step_kernels(a.old_obs, torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda").bool(), {})
+    a = DeviceVecNormalize(Env(n, cols), **kw)  # that call was a step
+    a.reset()
+    kept = a.obs_rms.mean, a.obs_rms.mean.clone()
+    for _ in range(4):
+        x, y = a.step(None), b.step(None)
+        # FP32 results of FP64 arithmetic: within an ulp (6e-8) and what the
+        # 1e-11 of the statistics makes of values of up to 1e3 deviations
+        for u, v in zip((x[0], x[1], x[3]["terminal_observation"]), (y[0], y[1], y[3]["terminal_observation"])):
+            _close(u, v, 2e-7)
+        assert torch.equal(x[2], y[2])
+    # sums of up to 8,195 FP64 terms, 4 times: 8,195 x 1.1e-16 x a mean of up
+    # to 50 deviations squared at most
+    for u, v in ((a.obs_rms.mean, b.obs_rms.mean), (a.obs_rms.var, b.obs_rms.var), (a.ret_rms.mean, b.ret_rms.mean),
+                 (a.ret_rms.var, b.ret_rms.var), (a.returns, b.returns)):
+        _close(u, v, 1e-9)
+    assert a.obs_rms.count == b.obs_rms.count and a.ret_rms.count == b.ret_rms.count
+    assert torch.equal(*kept)  # statistics handed out before stay as they were
+
+
+def test_values_that_are_not_finite():
+    a, b = DeviceVecNormalize(Env(64, 8, bad=True)), Tensors(Env(64, 8, bad=True))
+    a.reset(), b.reset()
+    for _ in range(2):
+        x, y = a.step(None), b.step(None)
+        _close(x[0], y[0], 2e-7)
+    _close(a.obs_rms.mean, b.obs_rms.mean, 1e-9)
+    _close(a.obs_rms.var, b.obs_rms.var, 1e-9)
+
+
+def test_other_tensors_take_the_tensor_operations():
+    a = DeviceVecNormalize(Env(16, 6))
+    a.reset()
+    r, d = torch.zeros(16, device="cuda"), torch.zeros(16, device="cuda").bool()
+    x = a.old_obs
+    assert a._step_kernels(x, r, d, {}) is not None
+    for obs, rew, done in ((x.t().contiguous().t(), r, d), (x.double(), r, d), (x, r.double(), d),
+                           (x, r, d.to(torch.uint8)), (x.clone().requires_grad_(), r, d), (x[:8], r[:8], d[:8]),
+                           (x.cpu(), r, d)):
+        assert a._step_kernels(obs, rew, done, {}) is None
