@@ -16,9 +16,9 @@
 //                  frustum culls the visuals' bounding spheres into a list
 //                  in shared memory; each thread traces its pixel's samples
 //                  (the terrain by a 2D DDA over the columns, the visuals
-//                  exactly or by sphere tracing), shades them with the
-//                  reference's shader, adds the glow, applies the vignette
-//                  and averages the samples.
+//                  exactly or by sphere tracing), shades the surfaces they
+//                  met with the reference's shader, adds the glow, applies
+//                  the vignette and averages the samples.
 //
 // Departures from the rasteriser, all in fine detail: shapes are exact
 // (spheres, capped cylinders, chamfered prisms) or sphere traced (rounded
@@ -32,6 +32,7 @@
 // along the diagonal from their (-x, -y) corner for the interpolation of
 // the vertex colours.
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -44,7 +45,8 @@
 // CTAs of k_render resident per SM. 4 caps its registers at 64 at the cost
 // of ~250 bytes of spills to L1; the extra warps hide more latency than the
 // spills cost (ms per 256 frames of 640 x 360 x 4 rays: 2 CTAs 24.7, 3 20.6,
-// 4 20.0).
+// 4 20.0; with hits returned in registers and surfaces shaded after all samples
+// are traced: 3 16.7, 4 16.0, 5 16.3).
 #ifndef ARC_RENDER_MIN_BLOCKS
 #define ARC_RENDER_MIN_BLOCKS 4
 #endif
@@ -122,7 +124,11 @@ struct FrameK {
     float body_c[kPoses][3], body_r[kPoses];  // world bounding sphere of each body's shadow casters
     VisK extra[2 * kMaxMarkers];  // marker beacons and rings, world frame
     GlowK glow[kMaxGlow];
+    // from here on read once per tile, not kept on chip: every item's bounding
+    // sphere, centre relative to the eye and radius (negative: no item)
+    alignas(16) float ball[kMaxItems][4];
 };
+constexpr int kFrameWords = (int)(offsetof(FrameK, ball) / 4);
 
 struct CamState {
     double target[3], heading;
@@ -199,17 +205,31 @@ template <class R> struct TerrainF {
     }
 };
 
+template <class R> __device__ __forceinline__ TerrainF<R> terrain_of_frame(const FrameK& fr, const R* h)
+{
+    return TerrainF<R>{h, fr.nx, fr.ny, fr.cell, fr.ox, fr.oy, fr.outside, fr.hmax, fr.bottom};
+}
+
 enum Face { kFaceTop = 0, kFaceX = 1, kFaceY = 2 };
+
+// A column surface: its distance (< 0: none) and which: (column << 3) + 0 for
+// the top, 2, 3 for the -x, +x and 4, 5 for the -y, +y going side. (Returned
+// by value: through references the callers kept their variables in memory.)
+struct TerrainHit {
+    float t;
+    int surf;
+};
 
 // First column surface along o + t D, t in (0, tmax): the drawn surface of
 // csrc/arc_mesh.c:228-255 (column tops, and column sides where the
 // neighbour is lower, down to the void's bottom). A 2D DDA over the cells
-// the ray crosses inside the grid's box. Returns t or -1.
+// the ray crosses inside the grid's box.
 template <class R>
-__device__ __noinline__ float trace_terrain(const TerrainF<R>& T, F3 o, F3 D, float tmax, int& face, int& cx, int& cy, int& sgn)
+__device__ __noinline__ TerrainHit trace_terrain(const FrameK& fr, const R* h_, F3 o, F3 D, float tmax)
 {
+    const TerrainF<R> T = terrain_of_frame(fr, h_);
     if (T.nx <= 0 || T.ny <= 0)
-        return -1.0f;
+        return TerrainHit{-1.0f, 0};
     const float lo[3] = {T.ox, T.oy, T.bottom};
     const float hi[3] = {T.ox + T.nx * T.cell, T.oy + T.ny * T.cell, T.hmax};
     const float oo[3] = {o.x, o.y, o.z}, dd[3] = {D.x, D.y, D.z};
@@ -219,7 +239,7 @@ __device__ __noinline__ float trace_terrain(const TerrainF<R>& T, F3 o, F3 D, fl
     for (int a = 0; a < 3; ++a) {
         if (fabsf(dd[a]) < 1e-12f) {
             if (oo[a] < lo[a] || oo[a] > hi[a])
-                return -1.0f;
+                return TerrainHit{-1.0f, 0};
             continue;
         }
         float inv = 1.0f / dd[a];
@@ -236,7 +256,7 @@ __device__ __noinline__ float trace_terrain(const TerrainF<R>& T, F3 o, F3 D, fl
         t1 = fminf(t1, tb);
     }
     if (t0 > t1)
-        return -1.0f;
+        return TerrainHit{-1.0f, 0};
     const float px = o.x + D.x * t0, py = o.y + D.y * t0;
     int ix = min(max((int)floorf((px - T.ox) / T.cell), 0), T.nx - 1);
     int iy = min(max((int)floorf((py - T.oy) / T.cell), 0), T.ny - 1);
@@ -255,20 +275,13 @@ __device__ __noinline__ float trace_terrain(const TerrainF<R>& T, F3 o, F3 D, fl
         const float h = T.at(ix, iy);
         const float t_out = fminf(fminf(tx, ty), t1);
         if (o.z + D.z * t_in <= h) {
-            face = f_in;
-            sgn = s_in;
-            cx = ix;
-            cy = iy;
-            return t_in;
+            return TerrainHit{t_in, ((iy * kGridMax + ix) << 3) +
+                                        (f_in == kFaceTop ? 0 : (f_in == kFaceX ? 2 : 4) + (s_in > 0))};
         }
         if (D.z < 0.0f) {
             const float tt = (h - o.z) / D.z;
             if (tt <= t_out) {
-                face = kFaceTop;
-                sgn = 0;
-                cx = ix;
-                cy = iy;
-                return tt;
+                return TerrainHit{tt, (iy * kGridMax + ix) << 3};
             }
         }
         if (t_out >= t1)
@@ -289,7 +302,7 @@ __device__ __noinline__ float trace_terrain(const TerrainF<R>& T, F3 o, F3 D, fl
         if (ix < 0 || iy < 0 || ix >= T.nx || iy >= T.ny)
             break;
     }
-    return -1.0f;
+    return TerrainHit{-1.0f, 0};
 }
 
 // ---- visuals, in their body's frame; D is a unit vector, hits in (tmin, tmax)
@@ -329,15 +342,24 @@ __device__ __forceinline__ float sdf_ring(F3 w, F3 d, float major, float tube)
 constexpr int kMarch = 48;
 constexpr float kMarchEps = 2e-5f;
 
-__device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, float& t, F3& n)
+// Distance along o + t D, t < tmax, and normal of a hit; t < 0: none.
+struct VisualHit {
+    float t;
+    F3 n;
+};
+
+__device__ __noinline__ VisualHit hit_visual(const VisK& v, F3 o, F3 D, float tmax)
 {
+    const VisualHit none{-1.0f, F3{0.0f, 0.0f, 0.0f}};
+    float t;
+    F3 n;
     const F3 c = ld3(v.o), d = ld3(v.d);
     switch (v.type) {
     case kVisSphere: {
         if (!hit_sphere(c, v.a, o, D, 1e-4f, tmax, t))
-            return false;
+            return none;
         n = scale(o + scale(D, t) - c, 1.0f / v.a);
-        return true;
+        return VisualHit{t, n};
     }
     case kVisBox: {
         const F3 in{v.a, v.b, v.c};
@@ -347,7 +369,7 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
         for (int a = 0; a < 3; ++a) {
             if (fabsf(da[a]) < 1e-12f) {
                 if (fabsf(oa[a]) > ext[a])
-                    return false;
+                    return none;
                 continue;
             }
             float inv = 1.0f / da[a];
@@ -356,7 +378,7 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
             t1 = fminf(t1, fmaxf(ta, tb));
         }
         if (t0 > t1)
-            return false;
+            return none;
         const F3 q0{oa[0], oa[1], oa[2]};
         float tt = t0;
         for (int i = 0; i < kMarch; ++i) {
@@ -366,13 +388,13 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
                 t = tt;
                 F3 cl{clampf(q.x, -in.x, in.x), clampf(q.y, -in.y, in.y), clampf(q.z, -in.z, in.z)};
                 n = normalize(q - cl);
-                return true;
+                return VisualHit{t, n};
             }
             tt += dist;
             if (tt > t1)
-                return false;
+                return none;
         }
-        return false;
+        return none;
     }
     case kVisTaper: {
         float tn = 1e-4f, tf = tmax;
@@ -383,7 +405,7 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
             float den = dot(pn, D), dist = v.pl[k][3] - dot(pn, o);
             if (fabsf(den) < 1e-12f) {
                 if (dist < 0.0f)
-                    return false;
+                    return none;
                 continue;
             }
             float tt = dist / den;
@@ -397,10 +419,10 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
             }
         }
         if (enter < 0 || tn > tf)
-            return false;
+            return none;
         t = tn;
         n = F3{v.pl[enter][0], v.pl[enter][1], v.pl[enter][2]};
-        return true;
+        return VisualHit{t, n};
     }
     case kVisCylinder: {
         const float radius = v.a, len_ = v.b, rib = v.c;
@@ -441,7 +463,7 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
             }
         }
         if (kind < 0)
-            return false;
+            return none;
         t = best;
         if (kind == 0) {
             F3 p = w + scale(D, t);
@@ -453,7 +475,7 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
         } else {
             n = kind == 1 ? -d : d;
         }
-        return true;
+        return VisualHit{t, n};
     }
     case kVisRing: {
         float t0, t1b;
@@ -462,12 +484,12 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
             float b = dot(oc, D), r = v.a + v.b, cc = dot(oc, oc) - r * r;
             float disc = b * b - cc;
             if (disc < 0.0f)
-                return false;
+                return none;
             float s = sqrtf(disc);
             t0 = fmaxf(-b - s, 1e-4f);
             t1b = fminf(-b + s, tmax);
             if (t0 > t1b)
-                return false;
+                return none;
         }
         const F3 w0 = o - c;
         float tt = t0;
@@ -480,26 +502,25 @@ __device__ __noinline__ bool hit_visual(const VisK& v, F3 o, F3 D, float tmax, f
                 F3 rad = w - scale(d, h);
                 float rl = sqrtf(dot(rad, rad));
                 n = normalize(w - scale(rad, rl > 1e-12f ? v.a / rl : 0.0f));
-                return true;
+                return VisualHit{t, n};
             }
             tt += dist;
             if (tt > t1b)
-                return false;
+                return none;
         }
-        return false;
+        return none;
     }
     }
-    return false;
+    return none;
 }
 
 // Is the segment from p toward the sun blocked by a column or by a visual
 // that casts shadows (all but the glowing ones, csrc/arc_render.c:545-552)?
 template <class R>
-__device__ bool shadowed(const FrameK& fr, const TerrainF<R>& T, const VisK* __restrict__ vis, int nv, F3 p)
+__device__ bool shadowed(const FrameK& fr, const R* h, const VisK* __restrict__ vis, int nv, F3 p)
 {
     const F3 L = ld3(fr.sun);
-    int f, a, b, s;
-    if (trace_terrain(T, p, L, 60.0f, f, a, b, s) >= 0.0f)
+    if (trace_terrain(fr, h, p, L, 60.0f).t >= 0.0f)
         return true;
     // the robot's bounding sphere first
     F3 oc = p - ld3(fr.robot_c);
@@ -531,9 +552,7 @@ __device__ bool shadowed(const FrameK& fr, const TerrainF<R>& T, const VisK* __r
             ol = rot_tmul(fr.rot[body], p - ld3(fr.pos[body]));
             dl = rot_tmul(fr.rot[body], L);
         }
-        float t;
-        F3 n;
-        if (hit_visual(vis[i], ol, dl, 60.0f, t, n))
+        if (hit_visual(vis[i], ol, dl, 60.0f).t >= 0.0f)
             return true;
     }
     return false;
@@ -703,24 +722,32 @@ __device__ F3 glow_along(const FrameK& fr, unsigned mask, F3 O, F3 D, float tdep
 template <class R>
 __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
     k_render(const VisK* __restrict__ vis, int nv, const FrameK* __restrict__ frames, Worlds<R> W,
-             const int* __restrict__ ids, int width, int height, int tiles_x, int samples,
-             unsigned char* __restrict__ out)
+             const int* __restrict__ ids, int width, int height, int tiles_x, int n_tiles,
+             int samples, unsigned char* __restrict__ out)
 {
-    __shared__ FrameK fr;
+    __shared__ alignas(FrameK) int frame_words[kFrameWords];
+    const FrameK& fr = *reinterpret_cast<const FrameK*>(frame_words);  // up to ball
     __shared__ unsigned char list[kMaxItems];
     __shared__ int warp_n[kThreads / 32];
     __shared__ unsigned glow_mask;
+    // each thread's own: per sample the depth of its hit, per surface its
+    // identity (later its colour) and, for a visual, its normal
+    __shared__ float hit_t[4][kThreads];
+    __shared__ struct {
+        int sid[kThreads];
+        float n[3][kThreads];
+    } surf[4];
     const int tid = threadIdx.x, item = blockIdx.y;
     {
         const int* src = reinterpret_cast<const int*>(frames + item);
-        int* dst = reinterpret_cast<int*>(&fr);
-        for (int i = tid; i < (int)(sizeof(FrameK) / 4); i += kThreads)
-            dst[i] = src[i];
+        for (int i = tid; i < kFrameWords; i += kThreads)
+            frame_words[i] = src[i];
     }
+    float4 ball = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+    if (tid < kMaxItems)
+        ball = *reinterpret_cast<const float4*>(frames[item].ball[tid]);
     __syncthreads();
     const int world = ids ? ids[item] : item;
-    const int tile_x = blockIdx.x % tiles_x, tile_y = blockIdx.x / tiles_x;
-    const int x0 = tile_x * kTileW, r0 = tile_y * kTileH;
     const F3 eye = ld3(fr.eye), fwd = ld3(fr.fwd), right = ld3(fr.right), up = ld3(fr.up);
     const float sx = 2.0f / width * fr.tan_y * fr.aspect, sy = 2.0f / height * fr.tan_y;
     // unnormalised ray through window point (wx, wy), y up
@@ -728,6 +755,9 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
         return fwd + scale(right, (wx - 0.5f * width) * sx) + scale(up, (wy - 0.5f * height) * sy);
     };
 
+    {
+    const int tile = blockIdx.x;
+    const int x0 = tile % tiles_x * kTileW, r0 = tile / tiles_x * kTileH;
     // cull the items' bounding spheres against the tile's frustum
     {
         const float wx0 = (float)x0, wx1 = (float)(x0 + kTileW);
@@ -740,17 +770,9 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
             if (dot(pn[k], cc) > 0.0f)
                 pn[k] = -pn[k];
         }
-        const int n_items = nv + fr.n_items;
-        bool keep = false;
-        if (tid < n_items) {
-            const VisK& v = tid < nv ? vis[tid] : fr.extra[tid - nv];
-            if (v.type >= 0) {
-                F3 cw = rot_mul(fr.rot[v.body], ld3(v.bc)) + ld3(fr.pos[v.body]) - eye;
-                keep = true;
-                for (int k = 0; k < 4; ++k)
-                    keep = keep && dot(pn[k], cw) <= v.br;
-            }
-        }
+        bool keep = ball.w >= 0.0f;
+        for (int k = 0; k < 4; ++k)
+            keep = keep && dot(pn[k], F3{ball.x, ball.y, ball.z}) <= ball.w;
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if ((tid & 31) == 0)
             warp_n[tid >> 5] = __popc(m);
@@ -785,16 +807,7 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
     for (int w = 0; w < kThreads / 32; ++w)
         n_list += warp_n[w];
 
-    TerrainF<R> T;
-    T.h = W.th + W.toff[world];
-    T.nx = fr.nx;
-    T.ny = fr.ny;
-    T.cell = fr.cell;
-    T.ox = fr.ox;
-    T.oy = fr.oy;
-    T.outside = fr.outside;
-    T.hmax = fr.hmax;
-    T.bottom = fr.bottom;
+    const TerrainF<R> T = terrain_of_frame(fr, (const R*)(W.th + W.toff[world]));
 
     // each warp takes an 8 x 4 block of the tile: nearby pixels tend to hit
     // the same surfaces, so fewer lanes diverge than along a 32-pixel row
@@ -811,22 +824,37 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
     const float dither = (hash2(fmaf(fr.time, 61.0f, px + 0.5f), fmaf(fr.time, 61.0f, wy_pix + 0.5f)) - 0.5f) / 255.0f;
     const F3 dDx = scale(right, sx), dDy = scale(up, sy);
     int acc[3] = {0, 0, 0};
-    // the surfaces this pixel's samples hit so far and their colours
-    int gid0 = -1, gid1 = -1, gid2 = -1, gid3 = -1;
-    unsigned gc0 = 0u, gc1 = 0u, gc2 = 0u, gc3 = 0u;
-    for (int si = 0; si < samples; ++si) {
+    // First every sample is traced, then each surface the pixel's samples hit
+    // is shaded, then the samples are put together. Multisampling shades once
+    // per pixel and primitive: a sample that hits the surface an earlier
+    // sample of this pixel hit (the same visual, or the same face of the same
+    // column) takes its colour. Shading inside the sample loop cost a warp one
+    // pass over the shader for every sample at which any of its pixels met a
+    // new surface, mostly for a few lanes; surface by surface a warp takes as
+    // many passes as its busiest pixel has surfaces (256 frames of 640 x 360:
+    // 18.1 -> 17.0 ms; with the culling spheres made once per frame 16.6, with
+    // the trace's results returned in registers 16.0, and with its terrain read
+    // from the frame's record instead of a local copy 15.5).
+    int n_surf = 0;
+    unsigned which = 0u;  // per sample 4 bits: 8 | surface, or 0 for none
+    unsigned owner = 0u;  // per surface 2 bits: the sample that met it first
+    auto sample_ray = [&](int si) {
         const float wx = samples == 1 ? px + 0.5f : px + spos[si][0];
         const float wy = samples == 1 ? wy_pix + 0.5f : wy_pix + spos[si][1];
-        const F3 Du = ray(wx, wy);
+        return ray(wx, wy);
+    };
+#pragma unroll 1
+    for (int si = 0; si < samples; ++si) {
+        const F3 Du = sample_ray(si);
         const float inv_len = rsqrtf(dot(Du, Du));
         const F3 D = scale(Du, inv_len);
         float best = kFar / dot(D, fwd);  // the far plane
-        int kind = -1, face = 0, cx = 0, cy = 0, sgn = 0, hit_item = -1;
+        int sid = -1;  // the surface: a visual's index, or 1024 + a column's
         F3 nl{0, 0, 1};
-        float tt = trace_terrain(T, eye, D, best, face, cx, cy, sgn);
-        if (tt >= 0.0f) {
-            best = tt;
-            kind = 0;
+        const TerrainHit ground = trace_terrain(fr, T.h, eye, D, best);
+        if (ground.t >= 0.0f) {
+            best = ground.t;
+            sid = 1024 + ground.surf;
         }
         int last_body = -1;
         F3 ol{0, 0, 0}, dl{0, 0, 0};
@@ -845,38 +873,41 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
                 if (b * b < c || (b > 0.0f && c > 0.0f))
                     continue;
             }
-            float t;
-            F3 n;
-            if (hit_visual(v, ol, dl, best, t, n)) {
-                best = t;
-                kind = 1;
-                hit_item = it;
-                nl = n;
+            const VisualHit h = hit_visual(v, ol, dl, best);
+            if (h.t >= 0.0f) {
+                best = h.t;
+                sid = it;
+                nl = h.n;
             }
         }
-        // Multisampling shades once per pixel and primitive: a sample that
-        // hits the surface an earlier sample of this pixel hit (the same
-        // visual, or the same face of the same column) takes its colour.
-        int sid = -1;
-        if (kind == 0)
-            sid = 1024 + ((cy * kGridMax + cx) << 3) + (face == kFaceTop ? 0 : (face == kFaceX ? 2 : 4) + (sgn > 0));
-        else if (kind == 1)
-            sid = hit_item;
-        unsigned packed = 0u;
-        bool fresh = false;
+        hit_t[si][tid] = sid >= 0 ? best : 1e30f;
         if (sid >= 0) {
-            if (sid == gid0)
-                packed = gc0;
-            else if (sid == gid1)
-                packed = gc1;
-            else if (sid == gid2)
-                packed = gc2;
-            else if (sid == gid3)
-                packed = gc3;
-            else
-                fresh = true;
+            int j = 0;
+            while (j < n_surf && surf[j].sid[tid] != sid)
+                ++j;
+            if (j == n_surf) {
+                ++n_surf;
+                owner |= (unsigned)si << (2 * j);
+                surf[j].sid[tid] = sid;
+                surf[j].n[0][tid] = nl.x;
+                surf[j].n[1][tid] = nl.y;
+                surf[j].n[2][tid] = nl.z;
+            }
+            which |= (8u | (unsigned)j) << (4 * si);
         }
-        if (fresh) {
+    }
+#pragma unroll 1
+    for (int j = 0; j < n_surf; ++j) {
+        const int si = (owner >> (2 * j)) & 3u, sid = surf[j].sid[tid];
+        const F3 Du = sample_ray(si);
+        const float inv_len = rsqrtf(dot(Du, Du));
+        const F3 D = scale(Du, inv_len);
+        const float best = hit_t[si][tid];
+        const F3 nl{surf[j].n[0][tid], surf[j].n[1][tid], surf[j].n[2][tid]};
+        const int kind = sid >= 1024 ? 0 : 1, code = (sid - 1024) & 7, column = (sid - 1024) >> 3;
+        const int cx = column % kGridMax, cy = column / kGridMax, hit_item = sid;
+        const int face = code == 0 ? kFaceTop : (code < 4 ? kFaceX : kFaceY), sgn = code & 1 ? 1 : -1;
+        {
             Surface s;
             s.p = eye + scale(D, best);
             s.pat = 0;
@@ -973,29 +1004,24 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
             const float fade = smooth(0.5f, 0.42f, fmaxf(ex, ey));
             float lit_k = 1.0f;
             if (fade > 0.0f && dot(s.n, ld3(fr.sun)) > 0.0f) {
-                const float k = shadowed(fr, T, vis, nv, s.p + scale(s.n, 2e-3f)) ? 0.0f : 1.0f;
+                const float k = shadowed(fr, T.h, vis, nv, s.p + scale(s.n, 2e-3f)) ? 0.0f : 1.0f;
                 lit_k = mixf(1.0f, k, fade);
             }
             const F3 c = shade_scene(fr, s, lit_k);
-            packed = (unsigned)unorm8(c.x + dither) | (unsigned)unorm8(c.y + dither) << 8 |
-                     (unsigned)unorm8(c.z + dither) << 16;
-            if (gid0 < 0) {
-                gid0 = sid;
-                gc0 = packed;
-            } else if (gid1 < 0) {
-                gid1 = sid;
-                gc1 = packed;
-            } else if (gid2 < 0) {
-                gid2 = sid;
-                gc2 = packed;
-            } else {
-                gid3 = sid;
-                gc3 = packed;
-            }
+            surf[j].sid[tid] = (int)((unsigned)unorm8(c.x + dither) | (unsigned)unorm8(c.y + dither) << 8 |
+                                     (unsigned)unorm8(c.z + dither) << 16);  // its colour from here on
         }
+    }
+#pragma unroll 1
+    for (int si = 0; si < samples; ++si) {
+        const unsigned hit = (which >> (4 * si)) & 15u;
+        const unsigned packed = hit ? (unsigned)surf[hit & 3u].sid[tid] : 0u;
+        const F3 Du = sample_ray(si);
+        const float inv_len = rsqrtf(dot(Du, Du));
+        const F3 D = scale(Du, inv_len);
         const int s8[3] = {(int)(packed & 255u), (int)((packed >> 8) & 255u), (int)(packed >> 16)};
         // additive glow (depth tested, not written), then the vignette
-        const F3 g = glow_along(fr, glow_mask, eye, D, kind >= 0 ? best : 1e30f);
+        const F3 g = glow_along(fr, glow_mask, eye, D, hit_t[si][tid]);
         const float gg[3] = {g.x, g.y, g.z};
         for (int k = 0; k < 3; ++k) {
             int v8 = unorm8(s8[k] / 255.0f + gg[k]);
@@ -1005,6 +1031,7 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
     unsigned char* o = out + (((size_t)item * height + row) * width + px) * 3;
     for (int k = 0; k < 3; ++k)
         o[k] = (unsigned char)((acc[k] + samples / 2) / samples);
+    }
 }
 
 __device__ __forceinline__ double wrap_angle(double a)
@@ -1078,10 +1105,17 @@ __global__ void __launch_bounds__(32 * kSetupWarps)
     // terrain: lowest and highest column, lamps (csrc/arc_render.c:523-549)
     const TerrainView<R> tv = terrain_of(W, world);
     double lo = 1e30, hi = -1e30;
-    for (int k = lane; k < tv.nx * tv.ny; k += 32) {
-        double h = (double)tv.h[k];
-        lo = fmin(lo, h);
-        hi = fmax(hi, h);
+    // sixteen loads in flight (one at a time took a third of a frame's setup)
+    for (int k0 = lane; k0 < tv.nx * tv.ny; k0 += 32 * 16) {
+        double h[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            h[u] = (double)tv.h[k0 + 32 * u < tv.nx * tv.ny ? k0 + 32 * u : k0];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            lo = fmin(lo, h[u]);
+            hi = fmax(hi, h[u]);
+        }
     }
     lo = warp_min(lo);
     hi = warp_max(hi);
@@ -1232,6 +1266,23 @@ __global__ void __launch_bounds__(32 * kSetupWarps)
         put3(f.body_c[b], bxx.x, bxx.y, bxx.z);
         f.body_r[b] = has ? r + 1e-3f : 0.0f;
     }
+    // the items' bounding spheres as k_render culls them (the markers' below)
+    __syncwarp();
+    for (int k = lane; k < kMaxItems; k += 32) {
+        float* o = f.ball[k];
+        o[0] = o[1] = o[2] = 0.0f;
+        o[3] = -1.0f;
+        if (k < nv && vis[k].type >= 0) {
+            const VisK& v = vis[k];
+            const F3 cw = rot_mul(f.rot[v.body], ld3(v.bc)) + ld3(f.pos[v.body]) -
+                          F3{(float)eye.x, (float)eye.y, (float)eye.z};
+            o[0] = cw.x;
+            o[1] = cw.y;
+            o[2] = cw.z;
+            o[3] = v.br;
+        }
+    }
+    __syncwarp();
     if (lane != 0)
         return;
     const V3<double> bx0 = x0;
@@ -1330,8 +1381,13 @@ __global__ void __launch_bounds__(32 * kSetupWarps)
                 v.b = 0.012f;
                 v.br = m[3] + 0.012f;
             }
-            for (int k = 0; k < 3; ++k)
+            const float at[3] = {(float)eye.x, (float)eye.y, (float)eye.z};
+            float* o = f.ball[nv + ne - 1];
+            for (int k = 0; k < 3; ++k) {
                 v.bc[k] = v.o[k];
+                o[k] = v.o[k] - at[k];
+            }
+            o[3] = v.br;
         }
         if (ng + 2 <= kMaxGlow) {
             GlowK& h = f.glow[ng++];
@@ -1618,9 +1674,18 @@ int launch(arc_renderer* r, const SimView& sv, const Worlds<R>& W, const int* d_
     if (report(cudaGetLastError(), "frame setup"))
         return ARC_ERR_CUDA;
     const int tiles_x = (r->w + rd::kTileW - 1) / rd::kTileW, tiles_y = (r->h + rd::kTileH - 1) / rd::kTileH;
-    dim3 grid(tiles_x * tiles_y, n);
+    // a CTA copies its frame's record once for up to four tiles, fewer while
+    // that would leave the GPU less than eight waves of CTAs
+    const int n_tiles = tiles_x * tiles_y;
+    int dev = 0, sms = 0;
+    if (report(cudaGetDevice(&dev), "device") ||
+        report(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device"))
+        return ARC_ERR_CUDA;
+    const long long per = (long long)n_tiles * n / (8ll * ARC_RENDER_MIN_BLOCKS * sms);
+    const int each = 1; (void)per;
+    dim3 grid((n_tiles + each - 1) / each, n);
     rd::k_render<R><<<grid, rd::kThreads, 0, st>>>(r->d_vis, r->nv, r->d_frames, W, d_ids, r->w, r->h, tiles_x,
-                                                   r->samples, d_rgb);
+                                                   n_tiles, r->samples, d_rgb);
     return report(cudaGetLastError(), "render");
 }
 
