@@ -367,8 +367,9 @@ __device__ __forceinline__ int collide(P& b, const BodyK<F>& k, Ref body, const 
 }
 
 // per-warp operation lists: kind | a << 4 | b << 8 | wait << 12 | arrive << 16
-// | flags. An op with a wait first syncs on that named barrier; one with an
-// arrive arrives on it when done.
+// | align << 20. An op with a wait first syncs on that named barrier; one with
+// an arrive arrives on it when done; one with align starts with its sibling
+// warps (AlignedSync).
 enum : uint32_t { OP_END = 0, OP_INT, OP_JNT, OP_COL, OP_UPD, OP_DMP, OP_CVL, OP_CNT };
 // INT/UPD a..b: body ordinals (0 torso, 1..3 coxa, femur, tibia)
 // JNT/DMP a..b: the leg's joints (0 torso->coxa, 1 coxa->femur, 2 femur->tibia)
@@ -408,7 +409,7 @@ enum : uint32_t { OP_END = 0, OP_INT, OP_JNT, OP_COL, OP_UPD, OP_DMP, OP_CVL, OP
     ARC_OP(OP_INT, 0, 4, 0, 0), ARC_OP(OP_JNT, 0, 1, 0, 1), ARC_OP(OP_JNT, 1, 2, 0, 0), ARC_OP(OP_UPD, 1, 2, 0, 0)
 #define ARC_TORSO_DAMP ARC_OP(OP_COL, 0, 1, 4, 0), ARC_OP(OP_UPD, 0, 1, 0, 0), ARC_OP(OP_DMP, 0, 1, 0, 5)
 #define ARC_LEG_DAMP(k) ARC_OP(OP_DMP, 0, 1, 4 + (k), 5 + (k))
-#define ARC_JOINT3 ARC_OP(OP_JNT, 2, 3, 0, 0)
+#define ARC_JOINT3 (ARC_OP(OP_JNT, 2, 3, 0, 0) | 1 << 20)
 #define ARC_FEMUR ARC_OP(OP_COL, 1, 2, 0, 0)
 #define ARC_LEG_TAIL                                                                                           \
     ARC_OP(OP_COL, 2, 6, 0, 0), ARC_OP(OP_UPD, 2, 4, 0, 0), ARC_OP(OP_DMP, 1, 3, 0, 0), ARC_OP(OP_CVL, 0, 0, 0, 0)
@@ -451,6 +452,83 @@ __constant__ uint32_t kOps[3][kWarps][kMaxOps] = {
 // ---------------------------------------------------------------------------
 
 
+// How the warps of a group wait for one another, by the kernel that runs it.
+// CtaSync: the CTA is the group.
+struct CtaSync {
+    __device__ __forceinline__ void group() const { __syncthreads(); }
+    __device__ __forceinline__ void wait(int id) const { bar_sync(id); }
+    __device__ __forceinline__ void arrive(int id) const { bar_arrive(id); }
+    __device__ __forceinline__ void align(int, int) const {}
+};
+
+// AlignedSync: the CTA holds several groups that start their third joints
+// together. The step is bound by instruction fetch: its loop is larger than
+// the SM's instruction cache, and with four CTAs of one group each the 16
+// warps stream through it at 16 places (12 % of the fetches miss, and waiting
+// for instructions is the largest stall but the barriers: 1.4 of 7.8 cycles
+// per instruction at 16,384 worlds). Warps of the same leg, which share a
+// scheduler, run the same code in the same order; where they run it at the
+// same time they fetch it once. Once a substep is enough, and the third
+// joint is the best place for it (65,536 worlds 3.41 ms in CTAs of their
+// own, 3.64 four to a CTA without aligning, 3.24 aligned at leg 0's substep
+// start, 3.20 before the tibia's spheres, 3.16 before joint 3, 3.30 at both).
+//
+// Each group has four of the sixteen named barriers, one per neighbouring
+// pair of warps around the ring (0-1, 1-2, 2-3, 3-0). A pair's joint and
+// damping hand-offs take turns on it: the second cannot be signalled before
+// the first was received, as each follows from the last around the ring. The
+// whole group's barrier is the first pair's, used only where every warp has
+// passed the substeps' last hand-off.
+//
+// The aligned start is a schedule, not an exchange: no result depends on it,
+// and a wait for it ends by itself after a while.
+struct AlignedSync {
+    int base;        // the group's first barrier
+    unsigned* word;  // per leg: groups running | arrived << 8 | starts so far << 16
+    __device__ __forceinline__ void group() const
+    {
+        asm volatile("bar.sync %0, %1;" ::"r"(base), "n"(kThreads) : "memory");
+    }
+    __device__ __forceinline__ void wait(int id) const { bar_sync(((id - 1) & 3) + base); }
+    __device__ __forceinline__ void arrive(int id) const { bar_arrive(((id - 1) & 3) + base); }
+    // one lane: arrives (+1) or leaves (-1); the last one starts the others
+    __device__ __forceinline__ unsigned change(unsigned* w, bool leaving) const
+    {
+        unsigned old = *(volatile unsigned*)w;
+        for (;;) {
+            const unsigned running = (old & 255u) - (leaving ? 1u : 0u), here = ((old >> 8) & 255u) + (leaving ? 0u : 1u);
+            const unsigned go = here > 0 && here >= running ? 1u : 0u;
+            const unsigned next = running | (go ? 0u : here << 8) | (((old >> 16) + go) & 0xffffu) << 16;
+            const unsigned seen = atomicCAS(w, old, next);
+            if (seen == old)
+                return go ? ~0u : old >> 16;  // ~0: started
+            old = seen;
+        }
+    }
+    __device__ __forceinline__ void align(int leg, int lane) const
+    {
+        if (lane == 0) {
+            const unsigned starts = change(word + leg, false);
+            if (starts != ~0u)
+                for (int spin = 0; spin < (1 << 16) && *(volatile unsigned*)(word + leg) >> 16 == starts; ++spin)
+                    ;
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ void join(int leg) const { atomicAdd(word + leg, 1u); }
+    __device__ __forceinline__ void leave(int leg) const { change(word + leg, true); }
+};
+
+// Groups that share an SM's memory and registers, and so an aligned CTA.
+constexpr int kAligned = sizeof(F) == 4 ? 4 : 2;
+constexpr int kAlignedFrom = sizeof(F) == 4 ? 3 : 2;  // groups per SM
+
+struct AlignedSmem {
+    Smem step[kAligned];
+    int next[kAligned];    // each slot's next group
+    unsigned word[kWarps];
+};
+
 // How a launch over n_items worlds is split: worlds per group (one CTA's
 // lanes) and the operation list.
 //   Worlds per group. A group's time is that of the longest path over its
@@ -463,10 +541,16 @@ __constant__ uint32_t kOps[3][kWarps][kMaxOps] = {
 //   Operation list: kListLatency up to two groups per SM in FP32, up to one
 // in FP64, whose SMs hold two (4,096 worlds: 758 us against 848; 7,000:
 // 1,119 against 1,069).
+//   Aligned CTAs (AlignedSync) take a work queue and a whole SM each, so not
+// beside others, and from three groups per SM on in FP32 (12,000 worlds, 2.5
+// per SM: as fast without; 14,300: 862 us without, 787 aligned; 65,536: 3,461
+// and 3,107), from two in FP64 (9,500 worlds: 1,579 us without, 1,411
+// aligned; 32,768: 4,142 and 3,600).
 struct GroupPlan {
     int per_group, groups, list;
+    bool aligned;
 };
-inline GroupPlan group_plan(int n_items, int sms, bool alone)
+inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue)
 {
     const int spread = sms / 2 > 0 ? sms / 2 : 1;
     GroupPlan p;
@@ -475,13 +559,14 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone)
         p.per_group = (n_items + spread - 1) / spread;
     p.groups = (n_items + p.per_group - 1) / p.per_group;
     p.list = alone && p.groups <= (sizeof(F) == 4 ? 2 : 1) * sms ? kListLatency : kListThroughput;
+    p.aligned = alone && queue && p.groups >= kAlignedFrom * sms;
     return p;
 }
 
-// One control step of the worlds of group `group` (items group * per_group
-// .. + per_group - 1, at most 32: worlds ids[item], or item itself without
-// ids) by a CTA of kThreads threads, thread tid = lane j of warp `leg`, in
-// the order of the operation list `list`. On return the
+// One control step of a group's worlds (items first .. first + per_group - 1,
+// at most 32: worlds ids[item], or item itself without ids) by kThreads
+// threads, thread tid = lane j of warp `leg`, in the order of the operation
+// list `list`. On return the
 // worlds' records, flags, time and unstable marks are written and every
 // thread of the CTA has passed the group's last barrier.
 //
@@ -492,14 +577,15 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone)
 // torques, and tile_q (13 x 4 floats per world) the position-pass q whose
 // rotation the next substep's gyroscopic term uses; the joint outputs, time
 // and stability come at the end of the last tile.
-__device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const Worlds<F>& W, const Actuation& A,
+template <class Sync>
+__device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const DevModel<F>& M, const Worlds<F>& W, const Actuation& A,
                                            F* __restrict__ spill, int spill_per_lane, int lane_cap,
-                                           const int* __restrict__ ids, int n_items, int group, int tid, int leg,
+                                           const int* __restrict__ ids, int n_items, int first, int tid, int leg,
                                            int j, int sub0, int sub1, F* __restrict__ tile_q, int per_group, int list)
 {
     (void)tid;
     const bool first_tile = sub0 == 0, last_tile = sub1 >= M.substeps;
-    const int item = group * per_group + j;
+    const int item = first + j;
     const int world = j < per_group && item < n_items ? (ids ? ids[item] : item) : -1;
     const bool valid = world >= 0 && world < W.n;
     const int wi = valid ? world : 0;
@@ -582,7 +668,7 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
     }
     const uint32_t* ops = &kOps[capped ? (int)kListCapped : list][leg][0];
     int last_nc = 0;  // this lane's contact records in the last substep
-    __syncthreads();
+    sync.group();
 
     for (int sub = sub0; sub < sub1; ++sub) {
         int nc = 0;
@@ -607,13 +693,15 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
             if (kind == OP_END)
                 break;
             const int a = (op >> 4) & 15, b = (op >> 8) & 15, wait = (op >> 12) & 15, arrive = (op >> 16) & 15;
+            if (op >> 20)
+                sync.align(leg, j);
             if (wait)
-                bar_sync(wait);
+                sync.wait(wait);
             if (kind == OP_CNT) {
                 // double-buffered: a warp may record substep s+1 while
                 // another still reads the counts of substep s
                 sm.nc[sub & 1][leg][j] = nc;
-                __syncthreads();
+                sync.group();
             } else if (active) {
                 switch (kind) {
                 case OP_INT:
@@ -773,11 +861,11 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
                 }
             }
             if (arrive)
-                bar_arrive(arrive);
+                sync.arrive(arrive);
         }
         last_nc = nc;
     }
-    __syncthreads();
+    sync.group();
 
     if (last_tile && W.lastc) {
         // the last substep's contact list in the reference's order
@@ -785,7 +873,7 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
         // which is the four warps' lists in warp order (the torso's records
         // lead warp 0's). Counts go through the (now free) count array.
         sm.nc[0][leg][j] = last_nc < lane_cap ? last_nc : lane_cap;
-        __syncthreads();
+        sync.group();
         if (active) {
             int before = 0, total = 0;  // records of the warps listed ahead of this one; of all
             for (int l = 0; l < kWarps; ++l) {
@@ -861,7 +949,7 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
                 sphw[0] = (uint32_t)((touches >> 50) & 1023u) | (((anch >> 5) & 1u) << 16);
             }
         }
-        __syncthreads();
+        sync.group();
         return;
     }
 
@@ -914,11 +1002,62 @@ __device__ __forceinline__ void step_group(Smem& sm, const DevModel<F>& M, const
         }
     }
     sm.bad[leg][j] = bad;
-    __syncthreads();
+    sync.group();
     if (active && leg == 0) {
         W.time[world] += M.step_dt;
         if (sm.bad[0][j] | sm.bad[1][j] | sm.bad[2][j] | sm.bad[3][j])
             W.unstable[world] = 1;
+    }
+}
+
+// The groups of a launch in CTAs of kAligned groups, one CTA per SM: slot g of
+// CTA b takes group b + g * gridDim.x first (so that few groups spread over
+// the SMs) and then what the queue hands out. All threads of the CTA call it.
+//
+// What is left over from whole waves of slots runs on SMs that are emptying:
+// up to kAligned / 2 groups per SM it takes the latency list, and fewer worlds
+// than one group per SM are split into as many groups as SMs (20,000 worlds,
+// 33 groups more than one wave: 1,524 us without either, 1,458 with the list).
+__device__ __forceinline__ void step_aligned(AlignedSmem& as, const DevModel<F>& M, const Worlds<F>& W,
+                                             const Actuation& A, F* __restrict__ spill, int spill_per_lane,
+                                             int lane_cap, const int* __restrict__ ids, int n_items, int* queue,
+                                             int sub0, int sub1, F* __restrict__ tile_q, int list)
+{
+    const int tid = threadIdx.x % kThreads, slot = threadIdx.x / kThreads, leg = tid / kWorlds, j = tid % kWorlds;
+    const int grid = gridDim.x, whole = n_items / (kAligned * grid * kWorlds) * kAligned * grid;  // groups
+    const int rest = n_items - whole * kWorlds;
+    const bool tail = whole > 0 && rest <= kAligned / 2 * grid * kWorlds;
+    const int rest_per = tail && rest < grid * kWorlds ? (rest + grid - 1) / grid : kWorlds;
+    const int n_groups = whole + (rest > 0 ? (rest + rest_per - 1) / rest_per : 0);
+    if (threadIdx.x < kWarps)
+        as.word[threadIdx.x] = 0u;
+    __syncthreads();  // the only barrier of the whole CTA: its barrier 0 is slot 0's from here on
+    const AlignedSync sync{kWarps * slot, as.word};
+    int group = blockIdx.x + slot * grid;
+#pragma unroll 1
+    while (group < n_groups) {
+        if (j == 0)
+            sync.join(leg);
+        const bool over = group >= whole;
+        step_group(sync, as.step[slot], M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
+                   over ? whole * kWorlds + (group - whole) * rest_per : group * kWorlds, tid, leg, j, sub0, sub1,
+                   tile_q, over ? rest_per : kWorlds, over && tail ? (int)kListLatency : list);
+        if (j == 0)
+            sync.leave(leg);
+        if (tid == 0)
+            as.next[slot] = kAligned * grid + atomicAdd(queue, 1);
+        sync.group();
+        group = as.next[slot];
+        sync.group();
+    }
+    // the last slot to leave zeroes the queue for the next launch
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(queue + 1, 1) == kAligned * grid - 1) {
+            queue[0] = 0;
+            queue[1] = 0;
+            __threadfence();
+        }
     }
 }
 

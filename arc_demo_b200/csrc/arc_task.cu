@@ -1109,8 +1109,8 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
     }
 #pragma unroll 1
     for (int group = first; group < n_groups;) {
-        wl::step_group(cs.step, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, group, tid, leg, j, sub0, sub1,
-                       tile_q, per_group, list);
+        wl::step_group(wl::CtaSync{}, cs.step, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
+                       group * per_group, tid, leg, j, sub0, sub1, tile_q, per_group, list);
         if constexpr (kMode != kPhysics) {
             // arc/task.py:155-259
             const int world = world_of(group * wl::kWorlds + j);
@@ -1149,6 +1149,17 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
     }
 }
 
+// The physics of many groups, in CTAs of four that run aligned.
+__global__ void __launch_bounds__(wl::kThreads * wl::kAligned, 1)
+k_step_aligned(const __grid_constant__ DevModel<float> M, Worlds<float> W, Actuation A, float* __restrict__ spill,
+               int spill_per_lane, int lane_cap, const int* __restrict__ ids, int n_items, int* queue, int sub0,
+               int sub1, float* __restrict__ tile_q, int list)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    wl::step_aligned(*reinterpret_cast<wl::AlignedSmem*>(smem_raw), M, W, A, spill, spill_per_lane, lane_cap, ids,
+                     n_items, queue, sub0, sub1, tile_q, list);
+}
+
 // One launch of k_control_step<kMode> over the n_items worlds ids[0 .. n_items).
 template <int kMode>
 cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Worlds<float>& W,
@@ -1164,6 +1175,9 @@ cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Wo
     static int resident[64] = {}, sm_count[64] = {};
     cudaError_t e = once_per_device(configured, [&](int dev) {
         cudaError_t r = cudaFuncSetAttribute(k_control_step<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (r == cudaSuccess && kMode == kPhysics)
+            r = cudaFuncSetAttribute(k_step_aligned, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(wl::AlignedSmem));
         int sms = 0, per_sm = 0;
         if (r == cudaSuccess)
             r = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1178,9 +1192,14 @@ cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Wo
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess)
         return e;
-    wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone);
+    wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone, queue != nullptr);
     if (kMode != kPhysics)  // the fused forms' task work takes whole groups of 32
-        plan = wl::GroupPlan{wl::kWorlds, (n_items + wl::kWorlds - 1) / wl::kWorlds, plan.list};
+        plan = wl::GroupPlan{wl::kWorlds, (n_items + wl::kWorlds - 1) / wl::kWorlds, plan.list, false};
+    if (plan.aligned) {
+        k_step_aligned<<<sm_count[dev], wl::kThreads * wl::kAligned, sizeof(wl::AlignedSmem), stream>>>(
+            M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, queue, sub0, sub1, tile_q, plan.list);
+        return cudaGetLastError();
+    }
     // with a queue, one wave of resident CTAs
     const int grid = queue && plan.groups > resident[dev] ? resident[dev] : plan.groups;
     k_control_step<kMode><<<grid, wl::kThreads, smem, stream>>>(M, RM, W, tg, tgd, grid_of, cell, P, S, O, A, spill,

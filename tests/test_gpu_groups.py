@@ -39,6 +39,30 @@ def test_small_batches_equal_large(fp64):
             assert np.array_equal(got, whole[: len(got)]), (n, queue)
 
 
+@pytest.mark.parametrize("fp64,n,cell", [
+    # three groups per SM; whole waves of four per SM; one world over, split
+    # over the SMs; a tail of groups of 32 in the latency list, and one in the
+    # other; contact lists at the reference's cap (their own list)
+    (False, 14208, 0.4), (False, 18944, 0.4), (False, 18945, 0.4), (False, 26000, 0.4), (False, 33000, 0.4),
+    (False, 14300, 0.05), (True, 9472, 0.4), (True, 9473, 0.4), (True, 12001, 0.4), (True, 16384, 0.4)])
+def test_aligned_groups_equal_groups_of_their_own(fp64, n, cell):
+    # bitwise; without the work queue every group has a CTA of its own
+    rng = np.random.default_rng(n)
+    seeds, diffs = rng.integers(0, 2**32, n, dtype=np.uint64).astype(np.uint32), rng.uniform(0.0, 1.0, n)
+    acts = rng.uniform(-1.0, 1.0, (2, n, 12))
+    states = []
+    for queue in (True, False):
+        s = Sim(n, fp64=fp64, cell=cell, grid=32)
+        s.set_kernel(KERNEL_WARPS)
+        s.set_work_queue(queue)
+        s.reset(np.arange(n), seeds, diffs)
+        for k in range(2):
+            s.step(s.default_angles + 0.6 * acts[k])
+        states.append(s.get_state())
+        s.close()
+    assert np.array_equal(*states)
+
+
 @pytest.mark.parametrize("fp64", [False, True])
 def test_task_rows_do_not_depend_on_the_batch(fp64):
     # the task kernel takes 32 worlds per CTA, four at a time: one world, a
