@@ -51,6 +51,9 @@ def _norm_lib():
 def _plain(x, dtype, shape, device) -> bool:
     """Whether the kernels can read x: a contiguous CUDA tensor of that type,
     shape and device, with nothing recorded or transformed about it."""
+    # forward-mode derivatives ride on plain tensors, but only inside a level
+    if torch.autograd.forward_ad._current_level >= 0:
+        return False
     return (type(x) is torch.Tensor and x.dtype == dtype and tuple(x.shape) == shape and x.device == device
             and x.is_contiguous() and not x.requires_grad and not x.is_neg() and not x.is_inference()
             and torch._C._functorch.maybe_get_level(x) == -1 and not torch.compiler.is_compiling())
@@ -191,6 +194,13 @@ class DeviceVecNormalize:
         dev, f32, f64 = obs.device, torch.float32, torch.float64
         term = infos.get("terminal_observation") if type(infos) is dict else None
         rms, ret = self.obs_rms, self.ret_rms
+        cls, base = type(self), DeviceVecNormalize
+        if (cls.normalize_obs is not base.normalize_obs or cls.normalize_reward is not base.normalize_reward
+                or type(rms) is not DeviceRunningMeanStd or type(ret) is not DeviceRunningMeanStd
+                or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+                or not all(isinstance(v, (int, float)) for v in (rms.count, ret.count, self.gamma, self.epsilon,
+                                                                 self.clip_obs, self.clip_reward))):
+            return None  # a subclass's own normalisation, something that traces the operations, tensor settings
         if (cols > 2048 or n != self.num_envs or type(infos) is not dict
                 or not _plain(obs, f32, (n, cols), dev) or not _plain(rewards, f32, (n,), dev)
                 or not _plain(dones, torch.bool, (n,), dev) or not _plain(self.returns, f64, (n,), dev)
@@ -201,8 +211,8 @@ class DeviceVecNormalize:
         lib = _norm_lib()
         with torch.cuda.device(dev):
             work = torch.empty(lib.arc_norm_work_size(n, cols) if self.training else 1, dtype=f64, device=dev)
-            returns, mean, var, ret_stats = torch.empty(n + 2 * cols + 2, dtype=f64, device=dev).split(
-                [n, cols, cols, 2])
+            returns, mean, var, ret_mean, ret_var = (torch.empty(s, dtype=f64, device=dev)
+                                                     for s in (n, cols, cols, (), ()))
             norm_obs = torch.empty_like(obs) if self.norm_obs else obs
             norm_term = torch.empty_like(term) if self.norm_obs and term is not None else term
             norm_rewards = torch.empty_like(rewards) if self.norm_reward else rewards
@@ -213,7 +223,7 @@ class DeviceVecNormalize:
                 ret.var.data_ptr(), rms.count, ret.count, self.gamma, self.epsilon, self.clip_obs, self.clip_reward,
                 norm_obs.data_ptr() if self.norm_obs else None,
                 norm_term.data_ptr() if self.norm_obs and term is not None else None, norm_rewards.data_ptr(),
-                returns.data_ptr(), mean.data_ptr(), var.data_ptr(), ret_stats.data_ptr(), ret_stats[1:].data_ptr(),
+                returns.data_ptr(), mean.data_ptr(), var.data_ptr(), ret_mean.data_ptr(), ret_var.data_ptr(),
                 work.data_ptr())
             stream = torch.cuda.current_stream(dev).cuda_stream
             if lib.arc_norm_step(ctypes.byref(args), stream or 1):  # 1: the legacy default stream
@@ -221,7 +231,7 @@ class DeviceVecNormalize:
         if self.training:
             if self.norm_obs:
                 rms.mean, rms.var, rms.count = mean, var, rms.count + n
-            ret.mean, ret.var, ret.count = ret_stats[0], ret_stats[1], ret.count + n
+            ret.mean, ret.var, ret.count = ret_mean, ret_var, ret.count + n
         self.returns = returns
         infos = dict(infos)
         if term is not None:

@@ -7,7 +7,7 @@ import itertools
 import pytest
 import torch
 
-from arc_demo_b200.vec_env import DeviceVecNormalize
+from arc_demo_b200.vec_env import DeviceRunningMeanStd, DeviceVecNormalize
 
 pytestmark = pytest.mark.gpu
 
@@ -96,3 +96,30 @@ def test_other_tensors_take_the_tensor_operations():
                            (x, r, d.to(torch.uint8)), (x.clone().requires_grad_(), r, d), (x[:8], r[:8], d[:8]),
                            (x.cpu(), r, d)):
         assert a._step_kernels(obs, rew, done, {}) is None
+
+
+def test_overridden_normalisation_is_used():
+    """A subclass's normalize_obs (or statistics of another class) decides, as
+    in the tensor operations; statistics keep storages of their own."""
+    class Half(DeviceVecNormalize):
+        def normalize_obs(self, obs):
+            return 0.5 * obs
+
+    class Rms(DeviceRunningMeanStd):
+        pass
+
+    a = Half(Env(16, 6))
+    a.reset()
+    obs = a.step(None)[0]
+    assert torch.equal(obs, 0.5 * a.old_obs)
+    b = DeviceVecNormalize(Env(16, 6))
+    b.reset()
+    b.step(None)
+    assert b.obs_rms.mean.untyped_storage().nbytes() == 6 * 8
+    r, d = torch.zeros(16, device="cuda"), torch.zeros(16, device="cuda").bool()
+    b.obs_rms = Rms(shape=(6,), device="cuda")
+    assert b._step_kernels(b.old_obs, r, d, {}) is None
+    b.obs_rms = DeviceRunningMeanStd(shape=(6,), device="cuda")
+    with torch.autograd.forward_ad.dual_level():
+        assert b._step_kernels(b.old_obs, r, d, {}) is None
+    assert b._step_kernels(b.old_obs, r, d, {}) is not None
