@@ -68,14 +68,18 @@ constexpr int kTorso = 3;  // body slot of the torso; 0..2: the lane's coxa, fem
 // The model constants stay in the kernel's parameter space: all lanes of a
 // warp read the same body, joint or sphere, a broadcast from the constant
 // cache.
-struct Smem {
+template <int OnChip, int Warps> struct SmemOf {
+    static constexpr int kOnChipRecords = OnChip;
     F leg[kWarps][3 * kBodyF][kWorlds];   // the lane's three bodies
     F anch[kWarps][5 * 6][kWorlds];       // anchor, anchor normal of the lane's five spheres
-    F con[kWarps][kOnChip * 7][kWorlds];  // on-chip contact records: local3 n3 body
+    F con[Warps][OnChip * 7][kWorlds];    // on-chip contact records: local3 n3 body
     F torso[kBodyF + 6][kWorlds];     // each world's torso, then its sphere's anchor
     int nc[2][kWarps][kWorlds];       // contact counts (capped lists), by substep parity
-    int bad[kWarps][kWorlds];
+    int bad[Warps][kWorlds];
 };
+using Smem = SmemOf<kOnChip, kWarps>;
+// of a split group (SplitSync): a foot's contacts, one or two, stay on chip
+using SplitSmem = SmemOf<2, 2 * kWarps>;
 
 // A field array in shared memory: element f at p[f * kWorlds]. Every
 // per-world array has the same row length, so fields are constant offsets
@@ -438,6 +442,36 @@ __constant__ uint32_t kOps[3][kWarps][kMaxOps] = {
       ARC_OP(OP_UPD, 1, 4, 0, 0), ARC_OP(OP_CNT, 0, 0, 0, 0), ARC_OP(OP_DMP, 0, 1, 0, 5), ARC_OP(OP_DMP, 1, 3, 0, 0),
       ARC_OP(OP_CVL, 0, 0, 0, 0), ARC_OP(OP_CVL, 1, 0, 8, 0), OP_END},
      ARC_CAPPED_OPS(1), ARC_CAPPED_OPS(2), ARC_CAPPED_OPS(3)}};
+// Split lists (SplitSync): two warps a leg. Warps 0..3 have the torso, the
+// coxas and the femurs' spheres, warps 4..7 joint 3k+2 and the tibias.
+// Barriers 1..4: the torso's hand-offs around the ring of the first four, for
+// joints and damping joints in turn (AlignedSync); 5+k: leg k's upper to its
+// lower warp (after joint 3k+1, after damping joint 3k+1); 9+k: back (the femur
+// integrated; joint 3k+2 solved). A leg's two barriers take turns: neither warp
+// signals again before it was signalled to. Leg 1's femur collides before its
+// damping joint, which comes late, leg 2's and 3's after theirs.
+#define ARC_UPPER_HEAD(k)                                                                                      \
+    ARC_OP(OP_INT, 1, 2, 0, 0), ARC_OP(OP_JNT, 0, 1, k, (k) + 1), ARC_OP(OP_JNT, 1, 2, 9 + (k), 5 + (k)),       \
+        ARC_OP(OP_UPD, 1, 2, 0, 0)
+#define ARC_UPPER_DAMP(k) ARC_OP(OP_DMP, 0, 1, k, (k) + 1)
+#define ARC_UPPER_FEMUR(k) ARC_OP(OP_COL, 1, 2, 9 + (k), 0), ARC_OP(OP_UPD, 2, 3, 0, 0)
+#define ARC_UPPER_TAIL(k) ARC_OP(OP_DMP, 1, 2, 0, 5 + (k)), OP_END
+#define ARC_LOWER(k)                                                                                           \
+    {ARC_OP(OP_INT, 2, 4, 0, 9 + (k)), ARC_OP(OP_JNT, 2, 3, 5 + (k), 9 + (k)), ARC_OP(OP_COL, 2, 6, 0, 0),      \
+     ARC_OP(OP_UPD, 3, 4, 0, 0), ARC_OP(OP_DMP, 2, 3, 5 + (k), 0), ARC_OP(OP_CVL, 0, 0, 0, 0), OP_END}
+__constant__ uint32_t kSplitOps[2 * kWarps][kMaxOps] = {
+    {ARC_OP(OP_INT, 0, 2, 0, 0), ARC_OP(OP_JNT, 0, 1, 0, 1), ARC_OP(OP_JNT, 1, 2, 9, 5), ARC_OP(OP_UPD, 1, 2, 0, 0),
+     ARC_UPPER_FEMUR(0), ARC_OP(OP_COL, 0, 1, 4, 0), ARC_OP(OP_UPD, 0, 1, 0, 0), ARC_OP(OP_DMP, 0, 1, 0, 1),
+     ARC_OP(OP_DMP, 1, 2, 0, 5), ARC_OP(OP_CVL, 1, 0, 4, 0), OP_END},
+    {ARC_UPPER_HEAD(1), ARC_UPPER_FEMUR(1), ARC_UPPER_DAMP(1), ARC_UPPER_TAIL(1)},
+    {ARC_UPPER_HEAD(2), ARC_UPPER_DAMP(2), ARC_UPPER_FEMUR(2), ARC_UPPER_TAIL(2)},
+    {ARC_UPPER_HEAD(3), ARC_UPPER_DAMP(3), ARC_UPPER_FEMUR(3), ARC_UPPER_TAIL(3)},
+    ARC_LOWER(0), ARC_LOWER(1), ARC_LOWER(2), ARC_LOWER(3)};
+#undef ARC_UPPER_HEAD
+#undef ARC_UPPER_DAMP
+#undef ARC_UPPER_FEMUR
+#undef ARC_UPPER_TAIL
+#undef ARC_LOWER
 #undef ARC_LEG_HEAD
 #undef ARC_TORSO_HEAD
 #undef ARC_TORSO_DAMP
@@ -455,6 +489,8 @@ __constant__ uint32_t kOps[3][kWarps][kMaxOps] = {
 // How the warps of a group wait for one another, by the kernel that runs it.
 // CtaSync: the CTA is the group.
 struct CtaSync {
+    static constexpr bool kSplit = false;
+    static constexpr int half = 0;
     __device__ __forceinline__ void group() const { __syncthreads(); }
     __device__ __forceinline__ void wait(int id) const { bar_sync(id); }
     __device__ __forceinline__ void arrive(int id) const { bar_arrive(id); }
@@ -483,6 +519,8 @@ struct CtaSync {
 // The aligned start is a schedule, not an exchange: no result depends on it,
 // and a wait for it ends by itself after a while.
 struct AlignedSync {
+    static constexpr bool kSplit = false;
+    static constexpr int half = 0;
     int base;        // the group's first barrier
     unsigned* word;  // per leg: groups running | arrived << 8 | starts so far << 16
     __device__ __forceinline__ void group() const
@@ -519,9 +557,31 @@ struct AlignedSync {
     __device__ __forceinline__ void leave(int leg) const { change(word + leg, true); }
 };
 
+// SplitSync: the CTA is one group, with two warps a leg (the split lists). A
+// group alone on an SM waits: its four warps are busy for 33k of a substep's
+// 47k cycles, and the tail of a leg, its tibia's spheres above all (10k), holds
+// back the next substep's first joint. With the tibias on warps of their own the
+// next substep's torso joints, which need the coxas only, run beside that tail.
+// A substep is then 27k cycles: the ring of four torso joints (4.1k each), the
+// torso's sphere and the damping ring on one side, and on the other a leg's
+// joints, spheres, damping and contact velocities in turn (27k too), so a third
+// warp a leg would not help. Tried on top and slower or not the same bits: the
+// tibia's spheres looked at together before (+0..13 %), the joints' four stages
+// unrolled (-5..10 %, but rounded otherwise than the rolled loop of large
+// batches, and a world must not depend on its batch).
+struct SplitSync {
+    static constexpr bool kSplit = true;
+    int half;  // 0: the torso's and the coxas' warps, 1: the femurs' and tibias'
+    __device__ __forceinline__ void group() const { __syncthreads(); }
+    __device__ __forceinline__ void wait(int id) const { bar_sync(id); }
+    __device__ __forceinline__ void arrive(int id) const { bar_arrive(id); }
+    __device__ __forceinline__ void align(int, int) const {}
+};
+
 // Groups that share an SM's memory and registers, and so an aligned CTA.
 constexpr int kAligned = sizeof(F) == 4 ? 4 : 2;
 constexpr int kAlignedFrom = sizeof(F) == 4 ? 3 : 2;  // groups per SM
+constexpr int kSplitTo = sizeof(F) == 4 ? 2 : 1;      // groups per SM
 
 struct AlignedSmem {
     Smem step[kAligned];
@@ -541,6 +601,12 @@ struct AlignedSmem {
 //   Operation list: kListLatency up to two groups per SM in FP32, up to one
 // in FP64, whose SMs hold two (4,096 worlds: 758 us against 848; 7,000:
 // 1,119 against 1,069).
+//   Split groups (SplitSync) up to two groups per SM in FP32, one in FP64
+// (FP32, one group per CTA of four warps and split: 1 world 298 and 256 us, 64:
+// 320 and 272, 1,000: 367 and 293, 4,096: 405 and 350, 6,000: 456 and 441,
+// 9,400: 500 and 477; FP64, 1: 458 and 378, 4,096: 621 and 565), where a whole
+// control step runs in one launch, no list can reach the reference's cap and
+// nobody records contacts.
 //   Aligned CTAs (AlignedSync) take a work queue and a whole SM each, so not
 // beside others, and from three groups per SM on in FP32 (12,000 worlds, 2.5
 // per SM: as fast without; 14,300: 862 us without, 787 aligned; 65,536: 3,461
@@ -548,9 +614,10 @@ struct AlignedSmem {
 // aligned; 32,768: 4,142 and 3,600).
 struct GroupPlan {
     int per_group, groups, list;
-    bool aligned;
+    bool aligned, split;
 };
-inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue)
+// splittable: a whole control step with uncapped lists that nobody records
+inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue, bool splittable)
 {
     const int spread = sms / 2 > 0 ? sms / 2 : 1;
     GroupPlan p;
@@ -560,6 +627,7 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue)
     p.groups = (n_items + p.per_group - 1) / p.per_group;
     p.list = alone && p.groups <= (sizeof(F) == 4 ? 2 : 1) * sms ? kListLatency : kListThroughput;
     p.aligned = alone && queue && p.groups >= kAlignedFrom * sms;
+    p.split = alone && splittable && p.groups <= kSplitTo * sms;
     return p;
 }
 
@@ -577,14 +645,20 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue)
 // torques, and tile_q (13 x 4 floats per world) the position-pass q whose
 // rotation the next substep's gyroscopic term uses; the joint outputs, time
 // and stability come at the end of the last tile.
-template <class Sync>
-__device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const DevModel<F>& M, const Worlds<F>& W, const Actuation& A,
+template <class Sync, class Mem>
+__device__ __forceinline__ void step_group(const Sync& sync, Mem& sm, const DevModel<F>& M, const Worlds<F>& W, const Actuation& A,
                                            F* __restrict__ spill, int spill_per_lane, int lane_cap,
                                            const int* __restrict__ ids, int n_items, int first, int tid, int leg,
                                            int j, int sub0, int sub1, F* __restrict__ tile_q, int per_group, int list)
 {
     (void)tid;
-    const bool first_tile = sub0 == 0, last_tile = sub1 >= M.substeps;
+    // a split group steps whole control steps with uncapped lists only
+    const bool first_tile = Sync::kSplit || sub0 == 0, last_tile = Sync::kSplit || sub1 >= M.substeps;
+    // what this warp has of the leg: the coxa (leg 0: and the torso), the femur
+    // and tibia, or both; its contact list
+    const bool upper = !Sync::kSplit || sync.half == 0, lower = !Sync::kSplit || sync.half == 1;
+    const int body0 = upper ? 0 : 1, body1 = lower ? 3 : 1, warp = kWarps * sync.half + leg;
+    auto has_sphere = [&](int s) { return s == 0 ? upper : lower; };  // of the leg's: the femur's, the tibia's
     const int item = first + j;
     const int world = j < per_group && item < n_items ? (ids ? ids[item] : item) : -1;
     const bool valid = world >= 0 && world < W.n;
@@ -601,12 +675,14 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
     };
     // actuation (csrc/arc_sim.c:132-136)
     F target0 = F(0), target1 = F(0), target2 = F(0);
-    if (valid) {
+    if (valid && upper) {
         target0 = actuate(M, A, world, j0);
         target1 = actuate(M, A, world, j0 + 1);
-        target2 = actuate(M, A, world, j0 + 2);
         jr[j0 * kJointRec] = target0;
         jr[(j0 + 1) * kJointRec] = target1;
+    }
+    if (valid && lower) {
+        target2 = actuate(M, A, world, j0 + 2);
         jr[(j0 + 2) * kJointRec] = target2;
     }
     F tacc0 = F(0), tacc1 = F(0), tacc2 = F(0);
@@ -629,7 +705,7 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
         setq(r, kQ, Q{tq[0], tq[1], tq[2], tq[3]});
     };
 #pragma unroll 1
-    for (int i = 0; i < 3; ++i) {
+    for (int i = body0; i < body1; ++i) {
         stage_body(body_ref(i), rec + (b_c + i) * kBodyRec);
         if (!first_tile)
             stage_q(body_ref(i), b_c + i);
@@ -638,15 +714,17 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
     const uint32_t* sphr = W.sph + (size_t)wi * 21;
 #pragma unroll
     for (int s = 0; s < 5; ++s) {
-        const F* a = sr + (5 * leg + 1 + s) * kSphereRec;
+        if (has_sphere(s)) {
+            const F* a = sr + (5 * leg + 1 + s) * kSphereRec;
 #pragma unroll
-        for (int c = 0; c < 6; ++c)
-            sm.anch[leg][6 * s + c][j] = a[c];
-        anch |= ((sphr[5 * leg + 1 + s] >> 16) & 1u) << s;
+            for (int c = 0; c < 6; ++c)
+                sm.anch[leg][6 * s + c][j] = a[c];
+            anch |= ((sphr[5 * leg + 1 + s] >> 16) & 1u) << s;
+        }
     }
     // warp 0 collides the torso's sphere and keeps its flags
-    const bool capped = kWarps * lane_cap > kMaxContacts;
-    if (leg == 0) {
+    const bool capped = !Sync::kSplit && kWarps * lane_cap > kMaxContacts;
+    if (leg == 0 && upper) {
         stage_body(torso, rec);
         if (!first_tile)
             stage_q(torso, 0);
@@ -666,20 +744,27 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
         if (leg == 0)
             touches |= (unsigned long long)(sphr[0] & 1023u) << 50;
     }
-    const uint32_t* ops = &kOps[capped ? (int)kListCapped : list][leg][0];
+    const uint32_t* ops = Sync::kSplit ? &kSplitOps[warp][0] : &kOps[capped ? (int)kListCapped : list][leg][0];
+    // a warp's contact records of this lane beyond the on-chip ones; the upper
+    // list of a split group's leg fills the room, which holds both, from its end
+    constexpr int kOn = Mem::kOnChipRecords;
+    auto spill_at = [&](int list_warp, int c) {
+        const int slot = Sync::kSplit && list_warp < kWarps ? spill_per_lane - 1 - (c - kOn) : c - kOn;
+        return spill + (((size_t)wi * kWarps + leg) * (size_t)spill_per_lane + slot) * 8;
+    };
     int last_nc = 0;  // this lane's contact records in the last substep
     sync.group();
 
     for (int sub = sub0; sub < sub1; ++sub) {
         int nc = 0;
         auto record = [&](int body, V local, V n) {
-            if (nc < kOnChip) {
-                const Ref d{&sm.con[leg][nc * 7][j]};
+            if (nc < kOn) {
+                const Ref d{&sm.con[warp][nc * 7][j]};
                 setv(d, 0, local);
                 setv(d, 3, n);
                 d[6] = (F)body;
-            } else if (nc < lane_cap && ARC_IN_BOUNDS(nc - kOnChip, spill_per_lane, kCheckSpillWrite)) {
-                F* d = spill + (((size_t)wi * kWarps + leg) * (size_t)spill_per_lane + (nc - kOnChip)) * 8;
+            } else if (nc < lane_cap && ARC_IN_BOUNDS(nc - kOn, spill_per_lane, kCheckSpillWrite)) {
+                F* d = spill_at(warp, nc);
                 d[0] = local.x; d[1] = local.y; d[2] = local.z;
                 d[3] = n.x; d[4] = n.y; d[5] = n.z;
                 d[6] = (F)body;
@@ -768,6 +853,8 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
                         setv(ra, 3, ss.anchor_n);
                     }
                     store_pose(r, pose);
+                    if (Sync::kSplit && a == 1)
+                        sm.nc[0][leg][j] = nc;  // the femur's, for the lower warp
                     break;
                 }
                 case OP_UPD:
@@ -823,36 +910,44 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
                     if (capped)
                         for (int l = 0; l < leg; ++l)
                             base += sm.nc[sub & 1][l][j];
-                    const int ncl = nc < lane_cap ? nc : lane_cap;
+                    // a split leg's lower warp takes the femur's contacts too,
+                    // from its upper warp's list
+                    int list_warp = Sync::kSplit && lower ? leg : warp;
+                    int count = Sync::kSplit && lower ? sm.nc[0][leg][j] : nc;
 #pragma unroll 1
-                    for (int c = 0; c < ncl && base + c < kMaxContacts; ++c) {
-                        F rc[7];
-                        if (c < kOnChip) {
+                    for (;; list_warp = warp, count = nc) {
+                        const int ncl = count < lane_cap ? count : lane_cap;
+#pragma unroll 1
+                        for (int c = 0; c < ncl && base + c < kMaxContacts; ++c) {
+                            F rc[7];
+                            if (c < kOn) {
 #pragma unroll
-                            for (int f = 0; f < 7; ++f)
-                                rc[f] = sm.con[leg][c * 7 + f][j];
-                        } else {
-                            if (!ARC_IN_BOUNDS(c - kOnChip, spill_per_lane, kCheckSpillRead))
+                                for (int f = 0; f < 7; ++f)
+                                    rc[f] = sm.con[list_warp][c * 7 + f][j];
+                            } else {
+                                if (!ARC_IN_BOUNDS(c - kOn, spill_per_lane, kCheckSpillRead))
+                                    continue;
+                                const F* src = spill_at(list_warp, c);
+#pragma unroll
+                                for (int f = 0; f < 7; ++f)
+                                    rc[f] = src[f];
+                            }
+                            const int bid = (int)rc[6];
+                            if ((bid == 0) != (a == 1))
                                 continue;
-                            const F* src =
-                                spill + (((size_t)wi * kWarps + leg) * (size_t)spill_per_lane + (c - kOnChip)) * 8;
-#pragma unroll
-                            for (int f = 0; f < 7; ++f)
-                                rc[f] = src[f];
+                            const Ref r = body_ref(bid == 0 ? kTorso : (bid == b_f ? 1 : 2));
+                            const BodyK<F>& k = M.body[bid];
+                            P pose;
+                            pose.q = getq(r, kQ);
+                            body_sync(pose, k);
+                            V v = getv(r, kV), w = getv(r, kW);
+                            contact_velocity(pose.rot, pose.iiw, k.inv_mass, v, w,
+                                             ContactRec<F>{V{rc[0], rc[1], rc[2]}, V{rc[3], rc[4], rc[5]}});
+                            setv(r, kV, v);
+                            setv(r, kW, w);
                         }
-                        const int bid = (int)rc[6];
-                        if ((bid == 0) != (a == 1))
-                            continue;
-                        const Ref r = body_ref(bid == 0 ? kTorso : (bid == b_f ? 1 : 2));
-                        const BodyK<F>& k = M.body[bid];
-                        P pose;
-                        pose.q = getq(r, kQ);
-                        body_sync(pose, k);
-                        V v = getv(r, kV), w = getv(r, kW);
-                        contact_velocity(pose.rot, pose.iiw, k.inv_mass, v, w,
-                                         ContactRec<F>{V{rc[0], rc[1], rc[2]}, V{rc[3], rc[4], rc[5]}});
-                        setv(r, kV, v);
-                        setv(r, kW, w);
+                        if (!Sync::kSplit || list_warp == warp)
+                            break;
                     }
                     break;
                 }
@@ -867,7 +962,7 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
     }
     sync.group();
 
-    if (last_tile && W.lastc) {
+    if (!Sync::kSplit && last_tile && W.lastc) {
         // the last substep's contact list in the reference's order
         // (csrc/arc_phys.c:493-499): sphere by sphere, the torso's first,
         // which is the four warps' lists in warp order (the torso's records
@@ -889,14 +984,14 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
                 if (at >= kMaxContacts)
                     continue;
                 F rc[7];
-                if (c < kOnChip) {
+                if (c < kOn) {
 #pragma unroll
                     for (int f = 0; f < 7; ++f)
-                        rc[f] = sm.con[leg][c * 7 + f][j];
+                        rc[f] = sm.con[warp][c * 7 + f][j];
                 } else {
-                    if (!ARC_IN_BOUNDS(c - kOnChip, spill_per_lane, kCheckSpillRead))
+                    if (!ARC_IN_BOUNDS(c - kOn, spill_per_lane, kCheckSpillRead))
                         continue;
-                    const F* src = spill + (((size_t)wi * kWarps + leg) * (size_t)spill_per_lane + (c - kOnChip)) * 8;
+                    const F* src = spill_at(warp, c);
 #pragma unroll
                     for (int f = 0; f < 7; ++f)
                         rc[f] = src[f];
@@ -962,15 +1057,19 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
         const JointK<F>& J0 = M.joint[j0];
         const JointK<F>& J1 = M.joint[j0 + 1];
         const JointK<F>& J2 = M.joint[j0 + 2];
-        jr[(j0 + 0) * kJointRec + 1] = joint_angle(tq, q0, J0);
-        jr[(j0 + 0) * kJointRec + 2] = joint_rate(tq, tw, w0, J0);
-        jr[(j0 + 1) * kJointRec + 1] = joint_angle(q0, q1, J1);
-        jr[(j0 + 1) * kJointRec + 2] = joint_rate(q0, w0, w1, J1);
-        jr[(j0 + 2) * kJointRec + 1] = joint_angle(q1, q2, J2);
-        jr[(j0 + 2) * kJointRec + 2] = joint_rate(q1, w1, w2, J2);
-        jr[(j0 + 0) * kJointRec + 3] = tacc0 / F(M.substeps);
-        jr[(j0 + 1) * kJointRec + 3] = tacc1 / F(M.substeps);
-        jr[(j0 + 2) * kJointRec + 3] = tacc2 / F(M.substeps);
+        if (upper) {
+            jr[(j0 + 0) * kJointRec + 1] = joint_angle(tq, q0, J0);
+            jr[(j0 + 0) * kJointRec + 2] = joint_rate(tq, tw, w0, J0);
+            jr[(j0 + 1) * kJointRec + 1] = joint_angle(q0, q1, J1);
+            jr[(j0 + 1) * kJointRec + 2] = joint_rate(q0, w0, w1, J1);
+            jr[(j0 + 0) * kJointRec + 3] = tacc0 / F(M.substeps);
+            jr[(j0 + 1) * kJointRec + 3] = tacc1 / F(M.substeps);
+        }
+        if (lower) {
+            jr[(j0 + 2) * kJointRec + 1] = joint_angle(q1, q2, J2);
+            jr[(j0 + 2) * kJointRec + 2] = joint_rate(q1, w1, w2, J2);
+            jr[(j0 + 2) * kJointRec + 3] = tacc2 / F(M.substeps);
+        }
         auto put = [&](Ref r, F* d) {
             const V x = getv(r, kX), v = getv(r, kV), w = getv(r, kW);
             const Q q = getq(r, kQP);
@@ -981,33 +1080,54 @@ __device__ __forceinline__ void step_group(const Sync& sync, Smem& sm, const Dev
             d[10] = w.x; d[11] = w.y; d[12] = w.z;
         };
 #pragma unroll 1
-        for (int i = 0; i < 3; ++i)
+        for (int i = body0; i < body1; ++i)
             put(body_ref(i), rec + (b_c + i) * kBodyRec);
         uint32_t* sphw = W.sph + (size_t)world * 21;
 #pragma unroll
         for (int s = 0; s < 5; ++s) {
-            F* a = sr + (5 * leg + 1 + s) * kSphereRec;
+            if (has_sphere(s)) {
+                F* a = sr + (5 * leg + 1 + s) * kSphereRec;
 #pragma unroll
-            for (int c = 0; c < 6; ++c)
-                a[c] = sm.anch[leg][6 * s + c][j];
-            sphw[5 * leg + 1 + s] = (uint32_t)((touches >> (10 * s)) & 1023u) | (((anch >> s) & 1u) << 16);
+                for (int c = 0; c < 6; ++c)
+                    a[c] = sm.anch[leg][6 * s + c][j];
+                sphw[5 * leg + 1 + s] = (uint32_t)((touches >> (10 * s)) & 1023u) | (((anch >> s) & 1u) << 16);
+            }
         }
-        if (leg == 0)
+        if (leg == 0 && upper)
             put(torso, rec);
-        if (leg == 0) {
+        if (leg == 0 && upper) {
 #pragma unroll
             for (int c = 0; c < 6; ++c)
                 sr[c] = torso[kBodyF + c];
             sphw[0] = (uint32_t)((touches >> 50) & 1023u) | (((anch >> 5) & 1u) << 16);
         }
     }
-    sm.bad[leg][j] = bad;
+    sm.bad[warp][j] = bad;
     sync.group();
-    if (active && leg == 0) {
+    if (active && leg == 0 && upper) {
         W.time[world] += M.step_dt;
-        if (sm.bad[0][j] | sm.bad[1][j] | sm.bad[2][j] | sm.bad[3][j])
+        int any = 0;
+#pragma unroll
+        for (int w = 0; w < (Sync::kSplit ? 2 : 1) * kWarps; ++w)
+            any |= sm.bad[w][j];
+        if (any)
             W.unstable[world] = 1;
     }
+}
+
+template <class W> inline bool splittable(const W& w, int lane_cap, int sub0, int sub1, int substeps)
+{
+    return kWarps * lane_cap <= kMaxContacts && !w.lastc && sub0 == 0 && sub1 >= substeps;
+}
+
+// One group per CTA of 2 * kThreads threads, split (SplitSync).
+__device__ __forceinline__ void step_split(SplitSmem& sm, const DevModel<F>& M, const Worlds<F>& W,
+                                           const Actuation& A, F* __restrict__ spill, int spill_per_lane,
+                                           int lane_cap, const int* __restrict__ ids, int n_items, int per_group)
+{
+    const int tid = threadIdx.x % kThreads;
+    step_group(SplitSync{(int)threadIdx.x / kThreads}, sm, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
+               blockIdx.x * per_group, tid, tid / kWorlds, tid % kWorlds, 0, M.substeps, nullptr, per_group, 0);
 }
 
 // The groups of a launch in CTAs of kAligned groups, one CTA per SM: slot g of

@@ -74,6 +74,16 @@ k_step_warps64_aligned(const __grid_constant__ DevModel<double> M, Worlds<double
                      n_items, queue, 0, M.substeps, nullptr, list);
 }
 
+__global__ void __launch_bounds__(2 * wl::kThreads, 1)
+k_step_warps64_split(const __grid_constant__ DevModel<double> M, Worlds<double> W, Actuation A,
+                     double* __restrict__ spill, int spill_per_lane, int lane_cap, const int* __restrict__ ids,
+                     int n_items, int per_group)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    wl::step_split(*reinterpret_cast<wl::SplitSmem*>(smem_raw), M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
+                   per_group);
+}
+
 }  // namespace
 
 cudaError_t launch_step_warps64(const DevModel<double>& M, const Worlds<double>& W, const Actuation& A,
@@ -94,6 +104,9 @@ cudaError_t launch_step_warps64(const DevModel<double>& M, const Worlds<double>&
         if (r == cudaSuccess)
             r = cudaFuncSetAttribute(k_step_warps64_aligned, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(wl::AlignedSmem));
+        if (r == cudaSuccess)
+            r = cudaFuncSetAttribute(k_step_warps64_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(wl::SplitSmem));
         int sms = 0, per_sm = 0;
         if (r == cudaSuccess)
             r = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -108,7 +121,13 @@ cudaError_t launch_step_warps64(const DevModel<double>& M, const Worlds<double>&
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess)
         return e;
-    const wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone, queue != nullptr);
+    const wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone, queue != nullptr,
+                                              wl::splittable(W, lane_cap, 0, M.substeps, M.substeps));
+    if (plan.split) {
+        k_step_warps64_split<<<plan.groups, 2 * wl::kThreads, sizeof(wl::SplitSmem), stream>>>(
+            M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, plan.per_group);
+        return cudaGetLastError();
+    }
     if (plan.aligned) {
         k_step_warps64_aligned<<<sm_count[dev], wl::kThreads * wl::kAligned, sizeof(wl::AlignedSmem), stream>>>(
             M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, queue, plan.list);

@@ -1160,6 +1160,16 @@ k_step_aligned(const __grid_constant__ DevModel<float> M, Worlds<float> W, Actua
                      n_items, queue, sub0, sub1, tile_q, list);
 }
 
+// The physics of few groups, each split over eight warps.
+__global__ void __launch_bounds__(2 * wl::kThreads, 2)
+k_step_split(const __grid_constant__ DevModel<float> M, Worlds<float> W, Actuation A, float* __restrict__ spill,
+             int spill_per_lane, int lane_cap, const int* __restrict__ ids, int n_items, int per_group)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    wl::step_split(*reinterpret_cast<wl::SplitSmem*>(smem_raw), M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
+                   per_group);
+}
+
 // One launch of k_control_step<kMode> over the n_items worlds ids[0 .. n_items).
 template <int kMode>
 cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Worlds<float>& W,
@@ -1178,6 +1188,9 @@ cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Wo
         if (r == cudaSuccess && kMode == kPhysics)
             r = cudaFuncSetAttribute(k_step_aligned, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(wl::AlignedSmem));
+        if (r == cudaSuccess && kMode == kPhysics)
+            r = cudaFuncSetAttribute(k_step_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(wl::SplitSmem));
         int sms = 0, per_sm = 0;
         if (r == cudaSuccess)
             r = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1192,9 +1205,16 @@ cudaError_t launch_form(const DevModel<float>& M, const ResetModel& RM, const Wo
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess)
         return e;
-    wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone, queue != nullptr);
+    wl::GroupPlan plan = wl::group_plan(n_items, sm_count[dev], alone, queue != nullptr,
+                                        wl::splittable(W, lane_cap, sub0, sub1, M.substeps));
     if (kMode != kPhysics)  // the fused forms' task work takes whole groups of 32
-        plan = wl::GroupPlan{wl::kWorlds, (n_items + wl::kWorlds - 1) / wl::kWorlds, plan.list, false};
+        plan = wl::GroupPlan{wl::kWorlds, (n_items + wl::kWorlds - 1) / wl::kWorlds, plan.list, false,
+                             false};
+    if (plan.split) {
+        k_step_split<<<plan.groups, 2 * wl::kThreads, sizeof(wl::SplitSmem), stream>>>(
+            M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, plan.per_group);
+        return cudaGetLastError();
+    }
     if (plan.aligned) {
         k_step_aligned<<<sm_count[dev], wl::kThreads * wl::kAligned, sizeof(wl::AlignedSmem), stream>>>(
             M, W, A, spill, spill_per_lane, lane_cap, ids, n_items, queue, sub0, sub1, tile_q, plan.list);

@@ -1,6 +1,8 @@
 """The split of small launches (fewer worlds per group, the latency list of
 operations) gives the same worlds as groups of 32 in the throughput list."""
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -96,3 +98,41 @@ def test_task_rows_do_not_depend_on_the_batch(fp64):
     for n in (1, 31, 32, 33, 65):
         for a, b in zip(rows(n), whole):
             assert torch.equal(a, b[:n])
+
+
+def leg_contacts(s, i):
+    """The most contacts of one tibia in world i's last substep."""
+    w = s._lib.arc_sim_world(s.ptr, i).contents
+    bodies = [w.contacts[k].body for k in range(w.n_contacts)]
+    return max(bodies.count(3 * leg + 3) for leg in range(4))
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+def test_split_groups_equal_whole_groups(fp64):
+    # bitwise; recording contacts keeps a leg on one warp. Robots dropped into
+    # columns of random heights touch many: some leg's list must outgrow the
+    # split group's on-chip records (2), or the spill is not tested
+    from oracle.oracle import World
+
+    n, steps = 70, 8
+    rng = np.random.default_rng(9)
+    acts = rng.uniform(-1.0, 1.0, (steps, n, 12))
+    states, longest = [], 0
+    for record in (False, True):
+        s = Sim(n, fp64=fp64)
+        s.set_kernel(KERNEL_WARPS)
+        s.reset(np.arange(n), np.arange(n, dtype=np.uint32), np.full(n, 0.5))
+        terrain = np.random.default_rng(4)
+        for i in range(n):
+            s.set_terrain(i, terrain.uniform(-0.3, 0.9, (64, 64)), 0.4)
+        s._lib.arc_sim_world.restype = ctypes.POINTER(World)
+        s._lib.arc_sim_world.argtypes = [ctypes.c_void_p, ctypes.c_int]
+        s._check(s._lib.arc_sim_set_record_contacts(s.ptr, int(record)))
+        for k in range(steps):
+            s.step(s.default_angles + 0.6 * acts[k])
+            if record:
+                longest = max([longest] + [leg_contacts(s, i) for i in range(n)])
+        states.append(s.get_state())
+        s.close()
+    assert np.array_equal(*states)
+    assert longest > 2
