@@ -272,7 +272,7 @@ __device__ __noinline__ TerrainHit trace_terrain(const FrameK& fr, const R* h_, 
     int s_in = entry == 0 ? sx : sy;
     const int max_steps = T.nx + T.ny + 2;
     for (int step = 0; step < max_steps; ++step) {
-        const float h = T.at(ix, iy);
+        const float h = (float)T.h[ix + iy * T.nx];  // the walk stays inside the grid
         const float t_out = fminf(fminf(tx, ty), t1);
         if (o.z + D.z * t_in <= h) {
             return TerrainHit{t_in, ((iy * kGridMax + ix) << 3) +
@@ -637,7 +637,8 @@ __device__ F3 shade_scene(const FrameK& fr, const Surface& s, float lit_k)
         float d2 = dot(l, l);
         l = scale(l, rsqrtf(d2));
         float cone = smooth(0.35f, 0.85f, -dot(l, ld3(fr.eye_dir)));
-        c = c + scale(shade_light(a, spec, gloss, n, v, l, ld3(fr.eye_col)), cone / (1.0f + 2.0f * d2));
+        if (cone > 0.0f)  // few pixels are in it
+            c = c + scale(shade_light(a, spec, gloss, n, v, l, ld3(fr.eye_col)), cone / (1.0f + 2.0f * d2));
     }
     {
         F3 l = ld3(fr.beacon_pos) - s.p;
