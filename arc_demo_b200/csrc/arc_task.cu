@@ -1046,6 +1046,47 @@ __global__ void k_task_set_targets(Worlds<R> W, const __grid_constant__ TaskPara
     S.in_view[i] = S.prev_gaze[i] < P.fov_rad;
 }
 
+// A warp per world, a lane per column (arc_env_get_task_state).
+__global__ void __launch_bounds__(256)
+k_task_rows(TaskState S, TaskOut O, const int* __restrict__ ids, int n, double* __restrict__ rows,
+            float* __restrict__ reward, unsigned char* __restrict__ bytes)
+{
+    const int k = (blockIdx.x * 256 + threadIdx.x) / 32, lane = threadIdx.x & 31;
+    if (k >= n)
+        return;
+    const int i = ids ? ids[k] : k;
+    double v = 0.0;
+    switch (lane) {
+    case 0: case 1: v = S.target[2 * i + lane]; break;
+    case 2: v = S.target_z[i]; break;
+    case 3: v = S.prev_dist[i]; break;
+    case 4: v = S.prev_gaze[i]; break;
+    case 17: v = S.torso_steps[i]; break;
+    case 18: v = S.steps[i]; break;
+    case 19: v = S.checkpoints[i]; break;
+    case 20: v = S.level[i]; break;
+    case 21: v = S.difficulty[i]; break;
+    case 22: v = S.in_view[i]; break;
+    case 23: v = S.episode[i]; break;
+    case 24: v = S.draws[i]; break;
+    default:
+        if (lane < 17)
+            v = S.prev_action[(size_t)i * 12 + lane - 5];
+    }
+    if (lane < 25)
+        rows[(size_t)k * 25 + lane] = v;
+    if (!reward)
+        return;
+    if (lane == 25)
+        reward[k] = O.reward[i];
+    else if (lane == 26)
+        bytes[k] = O.terminated[i];
+    else if (lane == 27)
+        bytes[(size_t)n + k] = O.truncated[i];
+    else if (lane == 28)
+        bytes[2 * (size_t)n + k] = (unsigned char)O.cause[i];
+}
+
 // ---------------------------------------------------------------------------
 // The warp-per-leg step (FP32, the quadruped) and, fused with it, the task
 // layer of ArcVecEnv.step_wait (arc/env.py:99-117). One kernel template
@@ -1374,6 +1415,15 @@ cudaError_t launch_env_admit(const DevModel<R>& M, const ResetModel& RM, const W
     if (e != cudaSuccess)
         return e;
     return launch_task_reset<R>(M, RM, W, tg, tgd, grid_of, cell, P, S, obs, ids, nullptr, n, stream);
+}
+
+cudaError_t launch_task_rows(const TaskState& S, const TaskOut& O, const int* ids, int n, double* rows, float* reward,
+                             unsigned char* bytes, cudaStream_t stream)
+{
+    if (n <= 0)
+        return cudaSuccess;
+    k_task_rows<<<(n + 7) / 8, 256, 0, stream>>>(S, O, ids, n, rows, reward, bytes);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_control_step(const DevModel<float>& M, const ResetModel& RM, const Worlds<float>& W,

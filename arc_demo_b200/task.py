@@ -123,6 +123,7 @@ def env_lib() -> ctypes.CDLL:
     d("arc_env_download", _int, _vp, _int, _vp)
     d("arc_env_upload", _int, _vp, _int, _vp)
     d("arc_env_get_task_state", _int, _vp, i32, _int, f64)
+    d("arc_env_task_results", _int, _vp, _vp, _vp, _vp, _vp, _vp)
     d("arc_env_set_task_state", _int, _vp, i32, _int, f64)
     d("arc_env_set_targets", _int, _vp, i32, _int, f64)
     lib._env_declared = True
@@ -163,6 +164,14 @@ class GpuTask:
         ids = np.ascontiguousarray(ids, dtype=np.int32)
         out = np.zeros((len(ids), TASK_STATE_SIZE))
         self.sim._check(self.lib.arc_env_get_task_state(self.sim.ptr, ids, len(ids), out))
+        return out
+
+    def results(self):
+        """The last step's (task state rows, reward, terminated, truncated, cause)."""
+        n = self.sim.num_worlds
+        out = (np.empty((n, TASK_STATE_SIZE)), np.empty(n, dtype=np.float32), np.empty(n, dtype=np.uint8),
+               np.empty(n, dtype=np.uint8), np.empty(n, dtype=np.int8))
+        self.sim._check(self.lib.arc_env_task_results(self.sim.ptr, *[a.ctypes.data for a in out]))
         return out
 
     def set_state(self, state, ids=None) -> None:
@@ -250,13 +259,11 @@ class ArcTask:
         self.gpu.upload(ACTIONS, a)
         self.sim._check(self.gpu.lib.arc_env_task_step(self.sim.ptr, None, None))
         self.sim.observe()
-        reward = self.gpu.download(REWARD)
-        terminated = self.gpu.download(TERMINATED).astype(bool)
-        truncated = self.gpu.download(TRUNCATED).astype(bool)
-        st = self.gpu.get_state()
+        st, reward, terminated, truncated, cause = self.gpu.results()
+        terminated, truncated = terminated.astype(bool), truncated.astype(bool)
         fell = terminated
         stats = {"checkpoints": st[:, 19].astype(np.int64), "difficulty": st[:, 21].copy(),
-                 "fell": fell.copy(), "cause": self.gpu.download(CAUSE).astype(np.int64),
+                 "fell": fell.copy(), "cause": cause.astype(np.int64),
                  "steps": st[:, 18].astype(np.int64)}
         ended = np.flatnonzero(terminated | truncated)
         if len(ended):

@@ -412,6 +412,10 @@ int arc_env_dlpack(const arc_sim *s, int which, void **managed);
 #define ARC_TASK_STATE_SIZE 25
 int arc_env_get_task_state(const arc_sim *s, const int *ids, int n_ids, double *out);
 int arc_env_set_task_state(arc_sim *s, const int *ids, int n_ids, const double *in);
+/* What the last step left, into host arrays of num_worlds rows: the task
+ * state as above, rewards, terminated and truncated flags, causes. */
+int arc_env_task_results(const arc_sim *s, double *state, float *reward, unsigned char *terminated,
+                         unsigned char *truncated, signed char *cause);
 /* Places checkpoints at given points (target_z, prev_dist, prev_gaze follow). */
 int arc_env_set_targets(arc_sim *s, const int *ids, int n_ids, const double *xy);
 
