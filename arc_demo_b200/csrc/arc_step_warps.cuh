@@ -502,12 +502,15 @@ struct CtaSync {
 // the SM's instruction cache, and with four CTAs of one group each the 16
 // warps stream through it at 16 places (12 % of the fetches miss, and waiting
 // for instructions is the largest stall but the barriers: 1.4 of 7.8 cycles
-// per instruction at 16,384 worlds). Warps of the same leg, which share a
-// scheduler, run the same code in the same order; where they run it at the
-// same time they fetch it once. Once a substep is enough, and the third
+// per instruction at 16,384 worlds). Warps of the same leg run the same code
+// in the same order; where they run it at the same time they fetch it once. Once a substep is enough, and the third
 // joint is the best place for it (65,536 worlds 3.41 ms in CTAs of their
 // own, 3.64 four to a CTA without aligning, 3.24 aligned at leg 0's substep
 // start, 3.20 before the tibia's spheres, 3.16 before joint 3, 3.30 at both).
+// But warps that share a scheduler then have it to themselves in turns, so
+// each group's legs start at another warp (step_aligned): what the alignment
+// still gives is 2 % (65,536 worlds of another state: 2,694 us with leg k of
+// every group on one scheduler, 2,475 turned, 2,532 turned and not aligned).
 //
 // Each group has four of the sixteen named barriers, one per neighbouring
 // pair of warps around the ring (0-1, 1-2, 2-3, 3-0). A pair's joint and
@@ -611,7 +614,9 @@ struct AlignedSmem {
 // beside others, and from three groups per SM on in FP32 (12,000 worlds, 2.5
 // per SM: as fast without; 14,300: 862 us without, 787 aligned; 65,536: 3,461
 // and 3,107), from two in FP64 (9,500 worlds: 1,579 us without, 1,411
-// aligned; 32,768: 4,142 and 3,600).
+// aligned; 32,768: 4,142 and 3,600). In FP32 they run kListLatency, since the
+// groups' legs take turns on the schedulers (65,536: 2,472 us in
+// kListThroughput, 2,425 in it), in FP64 not (16,384: 1,400 and 1,458).
 struct GroupPlan {
     int per_group, groups, list;
     bool aligned, split;
@@ -627,6 +632,8 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue, bool s
     p.groups = (n_items + p.per_group - 1) / p.per_group;
     p.list = alone && p.groups <= (sizeof(F) == 4 ? 2 : 1) * sms ? kListLatency : kListThroughput;
     p.aligned = alone && queue && p.groups >= kAlignedFrom * sms;
+    if (p.aligned && sizeof(F) == 4)
+        p.list = kListLatency;
     p.split = alone && splittable && p.groups <= kSplitTo * sms;
     return p;
 }
@@ -1143,7 +1150,12 @@ __device__ __forceinline__ void step_aligned(AlignedSmem& as, const DevModel<F>&
                                              int lane_cap, const int* __restrict__ ids, int n_items, int* queue,
                                              int sub0, int sub1, F* __restrict__ tile_q, int list)
 {
-    const int tid = threadIdx.x % kThreads, slot = threadIdx.x / kThreads, leg = tid / kWorlds, j = tid % kWorlds;
+    // each group's legs start at another warp: warps 4 apart share a scheduler,
+    // and with leg k of every group on the same one, that scheduler had the
+    // chain's four joints to issue at once while the others waited (16,384
+    // worlds 740 -> 674 us, 65,536 2,694 -> 2,475; FP64 16,384 1,505 -> 1,398)
+    const int tid = threadIdx.x % kThreads, slot = threadIdx.x / kThreads, j = tid % kWorlds;
+    const int leg = (tid / kWorlds + slot * (kWarps / kAligned)) % kWarps;
     const int grid = gridDim.x, whole = n_items / (kAligned * grid * kWorlds) * kAligned * grid;  // groups
     const int rest = n_items - whole * kWorlds;
     const bool tail = whole > 0 && rest <= kAligned / 2 * grid * kWorlds;
