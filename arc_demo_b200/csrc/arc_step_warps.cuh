@@ -583,7 +583,6 @@ struct SplitSync {
 
 // Groups that share an SM's memory and registers, and so an aligned CTA.
 constexpr int kAligned = sizeof(F) == 4 ? 4 : 2;
-constexpr int kAlignedFrom = sizeof(F) == 4 ? 3 : 2;  // groups per SM
 constexpr int kSplitTo = sizeof(F) == 4 ? 2 : 1;      // groups per SM
 
 struct AlignedSmem {
@@ -611,12 +610,11 @@ struct AlignedSmem {
 // control step runs in one launch, no list can reach the reference's cap and
 // nobody records contacts.
 //   Aligned CTAs (AlignedSync) take a work queue and a whole SM each, so not
-// beside others, and from three groups per SM on in FP32 (12,000 worlds, 2.5
-// per SM: as fast without; 14,300: 862 us without, 787 aligned; 65,536: 3,461
-// and 3,107), from two in FP64 (9,500 worlds: 1,579 us without, 1,411
-// aligned; 32,768: 4,142 and 3,600). In FP32 they run kListLatency, since the
-// groups' legs take turns on the schedulers (65,536: 2,472 us in
-// kListThroughput, 2,425 in it), in FP64 not (16,384: 1,400 and 1,458).
+// beside others, and all that is more than split groups take (10,007 worlds:
+// 555 us in CTAs of their own, 546 aligned; 12,000: 584 and 565; 16,384: 950
+// and 672; FP64 7,000: 777 and 732; 9,400: 831 and 761). They run
+// kListThroughput (a control step of 65,536 standing robots 2,835 us, in
+// kListLatency 2,905; thrown-about ones, 2,472 and 2,425, like it less).
 struct GroupPlan {
     int per_group, groups, list;
     bool aligned, split;
@@ -631,9 +629,7 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue, bool s
         p.per_group = (n_items + spread - 1) / spread;
     p.groups = (n_items + p.per_group - 1) / p.per_group;
     p.list = alone && p.groups <= (sizeof(F) == 4 ? 2 : 1) * sms ? kListLatency : kListThroughput;
-    p.aligned = alone && queue && p.groups >= kAlignedFrom * sms;
-    if (p.aligned && sizeof(F) == 4)
-        p.list = kListLatency;
+    p.aligned = alone && queue && p.groups > kSplitTo * sms;
     p.split = alone && splittable && p.groups <= kSplitTo * sms;
     return p;
 }
