@@ -76,7 +76,13 @@ struct arc_sim {
     // page-locked staging of large device-to-host copies (copy_out)
     void* pin[2] = {nullptr, nullptr};
     cudaEvent_t pin_ev[2] = {nullptr, nullptr};
-    void* pin_small = nullptr;  // and of small ones
+    // and of small ones, with the device staging of task rows (ids, then rows,
+    // of up to rows_cap worlds): read-outs of a const sim may run in several
+    // threads at once, and hold small_mu while they use either
+    mutable std::mutex small_mu;
+    mutable void* pin_small = nullptr;
+    char* rows = nullptr;
+    size_t rows_cap = 0;
     std::vector<char> skip;  // observe's outputs the caller did not ask for
     std::vector<double> host_tmp;
     arc_world* hworld = nullptr;
@@ -514,9 +520,13 @@ int ensure_staging(arc_sim* s)
 }
 
 constexpr size_t kPinSmall = size_t(256) << 10;
+// a world's task row, and its reward, flags and cause beside it
+constexpr size_t kTaskRowBytes = ARC_TASK_STATE_SIZE * sizeof(double), kTaskResultBytes = sizeof(float) + 3;
+constexpr size_t align8(size_t bytes) { return (bytes + 7) & ~size_t(7); }
 
 // The page-locked buffer of small copies; NULL where there is none to be had.
-char* small_staging(arc_sim* s)
+// The caller holds small_mu until it is done with the buffer.
+char* small_staging(const arc_sim* s)
 {
     if (!s->pin_small && cudaMallocHost(&s->pin_small, kPinSmall) != cudaSuccess) {
         cudaGetLastError();
@@ -528,7 +538,7 @@ char* small_staging(arc_sim* s)
 // Of at most kPinSmall bytes: one copy into page-locked memory and then into
 // the pieces. A copy into pageable memory costs the host about 9 us however
 // small it is, and this one 5 us for all pieces.
-int copy_out_small(arc_sim* s, char* pin, const void* src, size_t bytes, int n_seg, void* const* seg_dst,
+int copy_out_small(const arc_sim* s, char* pin, const void* src, size_t bytes, int n_seg, void* const* seg_dst,
                    const size_t* seg_bytes, cudaStream_t st, const char* where)
 {
     if (check(s, cudaMemcpyAsync(pin, src, bytes, cudaMemcpyDeviceToHost, st), where) ||
@@ -555,9 +565,11 @@ int copy_out_pieces(const arc_sim* sc, const void* src, int n_seg, void* const* 
     size_t bytes = 0;
     for (int k = 0; k < n_seg; ++k)
         bytes += seg_bytes[k];
-    if (bytes <= kPinSmall)
+    if (bytes <= kPinSmall) {
+        std::lock_guard<std::mutex> lock(s->small_mu);
         if (char* pin = small_staging(s))
             return copy_out_small(s, pin, src, bytes, n_seg, seg_dst, seg_bytes, s->stream, where);
+    }
     if (bytes < (size_t(2) << 20)) {
         size_t off = 0;
         for (int k = 0; k < n_seg; ++k) {
@@ -2061,6 +2073,9 @@ int arc_env_init(arc_sim* s, const arc_task_config* cfg, unsigned long long seed
     O.done_list = env_alloc<int>(s, n, ok);
     O.done_count = env_alloc<int>(s, 1, ok);
     s->actions = env_alloc<float>(s, n * kNumJoints, ok);
+    // a copy's worth of rows at most
+    s->rows_cap = std::min(n, kPinSmall / (kTaskRowBytes + kTaskResultBytes));
+    s->rows = env_alloc<char>(s, align8(s->rows_cap * sizeof(int)) + s->rows_cap * (kTaskRowBytes + kTaskResultBytes), ok);
     if (!ok)
         return fail(s, ARC_ERR_CUDA, "arc_env_init: device allocation failed");
     // initial level / difficulty (arc/task.py:107-108)
@@ -2360,10 +2375,11 @@ static int env_copy(const arc_sim* s, int which, void* host, bool down)
     if (sync(s, "env copy"))
         return ARC_ERR_CUDA;
     // as cudaMemcpy orders itself: on the legacy stream
-    if (down && bytes <= kPinSmall)
-        if (char* pin = small_staging(const_cast<arc_sim*>(s)))
-            return copy_out_small(const_cast<arc_sim*>(s), pin, p, bytes, 1, &host, &bytes, cudaStreamLegacy,
-                                  "env copy");
+    if (down && bytes <= kPinSmall) {
+        std::lock_guard<std::mutex> lock(s->small_mu);
+        if (char* pin = small_staging(s))
+            return copy_out_small(s, pin, p, bytes, 1, &host, &bytes, cudaStreamLegacy, "env copy");
+    }
     return check(s, cudaMemcpy(down ? host : p, down ? p : host, bytes,
                                down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice),
                  "env copy");
@@ -2373,38 +2389,48 @@ int arc_env_download(const arc_sim* s, int which, void* host) { return env_copy(
 int arc_env_upload(arc_sim* s, int which, const void* host) { return env_copy(s, which, (void*)host, false); }
 
 // The rows of the task state (and of the last step's results) gathered on the
-// device and copied out in one piece: 13 copies of whole arrays before (one
-// world: 130 us). On the legacy stream, as the copies were, after the sim's own.
-static int task_rows_out(const arc_sim* sc, const int* ids, int n_ids, double* out, float* reward,
+// device and copied out, rows_cap worlds at a time: 13 copies of whole arrays
+// before (one world: 130 us). On the legacy stream, as the copies were, after
+// the sim's own. ids NULL: worlds 0 .. n - 1.
+static int task_rows_out(const arc_sim* s, const int* ids, size_t n, double* out, float* reward,
                          unsigned char* terminated, unsigned char* truncated, signed char* cause, const char* where)
 {
-    arc_sim* s = const_cast<arc_sim*>(sc);
-    const size_t n = (size_t)n_ids, row = ARC_TASK_STATE_SIZE * sizeof(double);
-    const bool results = reward != nullptr;
-    const size_t bytes = n * (row + (results ? sizeof(float) + 3 : 0));
     if (sync(s, where))
         return ARC_ERR_CUDA;
-    if (n == 0)
-        return ARC_OK;
-    char* d = (char*)grow(s, s->st_out, bytes);
-    int* d_ids = ids ? (int*)grow(s, s->st_in3, sizeof(int) * n) : nullptr;
-    if (!d || (ids && !d_ids))
-        return ARC_ERR_CUDA;
-    if (ids && check(s, cudaMemcpyAsync(d_ids, ids, sizeof(int) * n, cudaMemcpyHostToDevice, cudaStreamLegacy), where))
-        return ARC_ERR_CUDA;
-    float* d_reward = results ? (float*)(d + n * row) : nullptr;
-    unsigned char* d_bytes = results ? (unsigned char*)(d_reward + n) : nullptr;
-    if (check(s, launch_task_rows(s->ts, s->to, d_ids, n_ids, (double*)d, d_reward, d_bytes, cudaStreamLegacy), where))
-        return ARC_ERR_CUDA;
-    void* dst[5] = {out, reward, terminated, truncated, cause};
-    const size_t len[5] = {n * row, n * sizeof(float), n, n, n};
-    const int n_seg = results ? 5 : 1;
-    if (bytes <= kPinSmall)
-        if (char* pin = small_staging(s))
-            return copy_out_small(s, pin, d, bytes, n_seg, dst, len, cudaStreamLegacy, where);
-    for (int k = 0; k < n_seg; d += len[k], ++k)
-        if (check(s, cudaMemcpy(dst[k], d, len[k], cudaMemcpyDeviceToHost), where))
+    std::lock_guard<std::mutex> lock(s->small_mu);
+    char* pin = small_staging(s);
+    for (size_t first = 0; first < n; first += s->rows_cap) {
+        const size_t m = std::min(n - first, s->rows_cap);
+        int* d_ids = ids ? (int*)s->rows : nullptr;
+        char* d = s->rows + align8(s->rows_cap * sizeof(int));
+        if (ids && check(s, cudaMemcpyAsync(d_ids, ids + first, sizeof(int) * m, cudaMemcpyHostToDevice, cudaStreamLegacy),
+                         where))
             return ARC_ERR_CUDA;
+        const size_t len[5] = {m * kTaskRowBytes, m * sizeof(float), m, m, m};
+        float* d_reward = reward ? (float*)(d + len[0]) : nullptr;
+        unsigned char* d_bytes = reward ? (unsigned char*)(d_reward + m) : nullptr;
+        if (check(s, launch_task_rows(s->ts, s->to, d_ids, (int)first, (int)m, (double*)d, d_reward, d_bytes,
+                                      cudaStreamLegacy),
+                  where))
+            return ARC_ERR_CUDA;
+        void* dst[5] = {out + first * ARC_TASK_STATE_SIZE, nullptr, nullptr, nullptr, nullptr};
+        if (reward) {
+            dst[1] = reward + first;
+            dst[2] = terminated + first;
+            dst[3] = truncated + first;
+            dst[4] = cause + first;
+        }
+        const int n_seg = reward ? 5 : 1;
+        if (pin) {
+            if (copy_out_small(s, pin, d, m * (kTaskRowBytes + (reward ? kTaskResultBytes : 0)), n_seg, dst, len,
+                               cudaStreamLegacy, where))
+                return ARC_ERR_CUDA;
+            continue;
+        }
+        for (int k = 0; k < n_seg; d += len[k], ++k)
+            if (check(s, cudaMemcpy(dst[k], d, len[k], cudaMemcpyDeviceToHost), where))
+                return ARC_ERR_CUDA;
+    }
     return ARC_OK;
 }
 
@@ -2414,7 +2440,7 @@ int arc_env_get_task_state(const arc_sim* s, const int* ids, int n_ids, double* 
         return rc;
     if (!ids_ok(s, ids, n_ids))
         return fail(s, ARC_ERR_ARG, "arc_env_get_task_state: world index out of range");
-    return task_rows_out(s, ids, n_ids > 0 ? n_ids : 0, out, nullptr, nullptr, nullptr, nullptr, "task state");
+    return task_rows_out(s, ids, n_ids > 0 ? (size_t)n_ids : 0, out, nullptr, nullptr, nullptr, nullptr, "task state");
 }
 
 int arc_env_task_results(const arc_sim* s, double* state, float* reward, unsigned char* terminated,
@@ -2424,7 +2450,7 @@ int arc_env_task_results(const arc_sim* s, double* state, float* reward, unsigne
         return rc;
     if (!state || !reward || !terminated || !truncated || !cause)
         return fail(s, ARC_ERR_ARG, "arc_env_task_results: NULL output");
-    return task_rows_out(s, nullptr, s->n > 0 ? s->n : 0, state, reward, terminated, truncated, cause, "task results");
+    return task_rows_out(s, nullptr, (size_t)s->n, state, reward, terminated, truncated, cause, "task results");
 }
 
 int arc_env_set_task_state(arc_sim* s, const int* ids, int n_ids, const double* in)

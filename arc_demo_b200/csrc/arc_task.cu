@@ -1048,13 +1048,13 @@ __global__ void k_task_set_targets(Worlds<R> W, const __grid_constant__ TaskPara
 
 // A warp per world, a lane per column (arc_env_get_task_state).
 __global__ void __launch_bounds__(256)
-k_task_rows(TaskState S, TaskOut O, const int* __restrict__ ids, int n, double* __restrict__ rows,
+k_task_rows(TaskState S, TaskOut O, const int* __restrict__ ids, int first, int n, double* __restrict__ rows,
             float* __restrict__ reward, unsigned char* __restrict__ bytes)
 {
     const int k = (blockIdx.x * 256 + threadIdx.x) / 32, lane = threadIdx.x & 31;
     if (k >= n)
         return;
-    const int i = ids ? ids[k] : k;
+    const int i = ids ? ids[k] : first + k;
     double v = 0.0;
     switch (lane) {
     case 0: case 1: v = S.target[2 * i + lane]; break;
@@ -1417,12 +1417,12 @@ cudaError_t launch_env_admit(const DevModel<R>& M, const ResetModel& RM, const W
     return launch_task_reset<R>(M, RM, W, tg, tgd, grid_of, cell, P, S, obs, ids, nullptr, n, stream);
 }
 
-cudaError_t launch_task_rows(const TaskState& S, const TaskOut& O, const int* ids, int n, double* rows, float* reward,
-                             unsigned char* bytes, cudaStream_t stream)
+cudaError_t launch_task_rows(const TaskState& S, const TaskOut& O, const int* ids, int first, int n, double* rows,
+                             float* reward, unsigned char* bytes, cudaStream_t stream)
 {
     if (n <= 0)
         return cudaSuccess;
-    k_task_rows<<<(n + 7) / 8, 256, 0, stream>>>(S, O, ids, n, rows, reward, bytes);
+    k_task_rows<<<(n + 7) / 8, 256, 0, stream>>>(S, O, ids, first, n, rows, reward, bytes);
     return cudaGetLastError();
 }
 

@@ -112,10 +112,10 @@ cudaError_t launch_env_admit(const DevModel<R>& M, const ResetModel& RM, const W
                              const unsigned* keys, int n, cudaStream_t stream);
 
 // Task state rows of ARC_TASK_STATE_SIZE doubles (include/arc_sim.h) of worlds
-// ids[0 .. n) (NULL: 0 .. n - 1); with `reward`, the last step's rewards, and in
+// ids[0 .. n) (NULL: first .. first + n - 1); with `reward`, the last step's rewards, and in
 // `bytes` its terminated, truncated and cause arrays one after the other.
-cudaError_t launch_task_rows(const TaskState& S, const TaskOut& O, const int* ids, int n, double* rows, float* reward,
-                             unsigned char* bytes, cudaStream_t stream);
+cudaError_t launch_task_rows(const TaskState& S, const TaskOut& O, const int* ids, int first, int n, double* rows,
+                             float* reward, unsigned char* bytes, cudaStream_t stream);
 
 // Checkpoints at given points (host-injected; parity tests and callers that
 // draw their own): target, target_z, prev_dist, prev_gaze, in_view.

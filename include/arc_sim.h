@@ -408,7 +408,9 @@ int arc_env_dlpack(const arc_sim *s, int which, void **managed);
 
 /* Per-world task state, host FP64, ARC_TASK_STATE_SIZE values per world:
  * target x y, target_z, prev_dist, prev_gaze, prev_action x12, torso_steps,
- * steps, checkpoints, level, difficulty, in_view, episode, draws. */
+ * steps, checkpoints, level, difficulty, in_view, episode, draws. Several
+ * threads may read one sim at once (arc_env_download, arc_env_get_task_state,
+ * arc_env_task_results) while none changes it. */
 #define ARC_TASK_STATE_SIZE 25
 int arc_env_get_task_state(const arc_sim *s, const int *ids, int n_ids, double *out);
 int arc_env_set_task_state(arc_sim *s, const int *ids, int n_ids, const double *in);
