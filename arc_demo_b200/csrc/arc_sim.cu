@@ -2073,8 +2073,8 @@ int arc_env_init(arc_sim* s, const arc_task_config* cfg, unsigned long long seed
     O.done_list = env_alloc<int>(s, n, ok);
     O.done_count = env_alloc<int>(s, 1, ok);
     s->actions = env_alloc<float>(s, n * kNumJoints, ok);
-    // a copy's worth of rows at most
-    s->rows_cap = std::min(n, kPinSmall / (kTaskRowBytes + kTaskResultBytes));
+    // 13.8 MB at most (in copies of 256 KB instead, 65,536 results took 2.5 ms, not 1.0)
+    s->rows_cap = std::min(n, size_t(65536));
     s->rows = env_alloc<char>(s, align8(s->rows_cap * sizeof(int)) + s->rows_cap * (kTaskRowBytes + kTaskResultBytes), ok);
     if (!ok)
         return fail(s, ARC_ERR_CUDA, "arc_env_init: device allocation failed");
@@ -2389,7 +2389,7 @@ int arc_env_download(const arc_sim* s, int which, void* host) { return env_copy(
 int arc_env_upload(arc_sim* s, int which, const void* host) { return env_copy(s, which, (void*)host, false); }
 
 // The rows of the task state (and of the last step's results) gathered on the
-// device and copied out, rows_cap worlds at a time: 13 copies of whole arrays
+// device, rows_cap worlds at a time, and copied out: 13 copies of whole arrays
 // before (one world: 130 us). On the legacy stream, as the copies were, after
 // the sim's own. ids NULL: worlds 0 .. n - 1.
 static int task_rows_out(const arc_sim* s, const int* ids, size_t n, double* out, float* reward,
@@ -2398,7 +2398,6 @@ static int task_rows_out(const arc_sim* s, const int* ids, size_t n, double* out
     if (sync(s, where))
         return ARC_ERR_CUDA;
     std::lock_guard<std::mutex> lock(s->small_mu);
-    char* pin = small_staging(s);
     for (size_t first = 0; first < n; first += s->rows_cap) {
         const size_t m = std::min(n - first, s->rows_cap);
         int* d_ids = ids ? (int*)s->rows : nullptr;
@@ -2421,9 +2420,10 @@ static int task_rows_out(const arc_sim* s, const int* ids, size_t n, double* out
             dst[4] = cause + first;
         }
         const int n_seg = reward ? 5 : 1;
+        const size_t bytes = m * (kTaskRowBytes + (reward ? kTaskResultBytes : 0));
+        char* pin = bytes <= kPinSmall ? small_staging(s) : nullptr;
         if (pin) {
-            if (copy_out_small(s, pin, d, m * (kTaskRowBytes + (reward ? kTaskResultBytes : 0)), n_seg, dst, len,
-                               cudaStreamLegacy, where))
+            if (copy_out_small(s, pin, d, bytes, n_seg, dst, len, cudaStreamLegacy, where))
                 return ARC_ERR_CUDA;
             continue;
         }

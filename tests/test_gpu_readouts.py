@@ -1,4 +1,5 @@
-"""Task rows of more worlds than one copy takes, and read by two threads."""
+"""Task rows at the edge of a page-locked copy, more of them than the sim has
+worlds, and read by several threads."""
 
 import threading
 
@@ -10,9 +11,9 @@ from arc_demo_b200.task import OBS, REWARD, TASK_STATE_SIZE, ArcTask, TaskConfig
 pytestmark = pytest.mark.gpu
 
 
-# 1,266 rows are a copy: one short of it, one over, and two copies and a rest
+# the results of 1,266 worlds are the most that one page-locked copy holds
 @pytest.mark.parametrize("n", [1266, 1267, 2600])
-def test_rows_beyond_one_copy(n):
+def test_rows_beyond_a_small_copy(n):
     t = ArcTask(n, TaskConfig(curriculum=False), seed=3)
     rows = np.random.default_rng(n).integers(0, 1000, (n, TASK_STATE_SIZE)).astype(np.float64)
     rows[:, 22] = np.arange(n) % 2
@@ -20,7 +21,7 @@ def test_rows_beyond_one_copy(n):
     reward = np.random.default_rng(1).normal(size=n).astype(np.float32)
     t.gpu.upload(REWARD, reward)
     assert np.array_equal(t.gpu.get_state(), rows)
-    ids = np.random.default_rng(2).integers(0, n, n + 5)  # some twice, more than there are worlds
+    ids = np.random.default_rng(2).integers(0, n, n + 5)  # some twice; more than the staging's rows
     assert np.array_equal(t.gpu.get_state(ids), rows[ids])
     got = t.gpu.results()
     assert np.array_equal(got[0], rows) and np.array_equal(got[1], reward)
