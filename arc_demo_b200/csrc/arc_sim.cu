@@ -39,6 +39,7 @@ struct DevBuffer {
 
 struct arc_sim {
     int n = 0, substeps = 0, grid = 0, threads = 1;
+    int device = 0;  // current when the sim was made; its memory and streams are there
     double dt = 0.0, cell = 0.0;
     bool fp64 = false;
     int kernel = ARC_KERNEL_LEGS, wpc = 16;
@@ -369,7 +370,8 @@ arc_sim* create_with_model(const ModelHost& model, int n, double dt, int substep
         while (s->stride % 8 != 4)
             s->stride += 4;
     const size_t nn = (size_t)std::max(n, 1);
-    bool ok = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) == cudaSuccess;
+    bool ok = cudaGetDevice(&s->device) == cudaSuccess;
+    ok = ok && cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMalloc(&s->rec, nn * s->stride * rs) == cudaSuccess;
     ok = ok && cudaMalloc((void**)&s->sph, nn * std::max(s->model.ns, 1) * sizeof(uint32_t)) == cudaSuccess;
     ok = ok && cudaMalloc((void**)&s->unstable, nn * sizeof(int)) == cudaSuccess;
@@ -404,6 +406,31 @@ bool ids_ok(const arc_sim* s, const int* ids, int n_ids)
 }
 
 int sync(const arc_sim* s, const char* where) { return check(s, cudaStreamSynchronize(s->stream), where); }
+
+// The sim's device current, and the caller's again at the end: for read-outs,
+// which may come from a thread on another device and, unlike calls with a
+// stream of the sim's, would run there without an error.
+class OnDeviceOf {
+public:
+    explicit OnDeviceOf(const arc_sim* s)
+    {
+        status = cudaGetDevice(&before_);
+        if (status == cudaSuccess && before_ != s->device)
+            moved_ = (status = cudaSetDevice(s->device)) == cudaSuccess;
+    }
+    ~OnDeviceOf()
+    {
+        if (moved_)
+            cudaSetDevice(before_);
+    }
+    OnDeviceOf(const OnDeviceOf&) = delete;
+    OnDeviceOf& operator=(const OnDeviceOf&) = delete;
+    cudaError_t status;
+
+private:
+    int before_ = 0;
+    bool moved_ = false;
+};
 
 // Host memcpy split over a few persistent threads and the caller: copying
 // from page-locked staging into the caller's (pageable) arrays is the slow
@@ -2376,6 +2403,9 @@ static int env_copy(const arc_sim* s, int which, void* host, bool down)
         return ARC_ERR_CUDA;
     // as cudaMemcpy orders itself: on the legacy stream
     if (down && bytes <= kPinSmall) {
+        const OnDeviceOf device(s);
+        if (check(s, device.status, "env copy"))
+            return ARC_ERR_CUDA;
         std::lock_guard<std::mutex> lock(s->small_mu);
         if (char* pin = small_staging(s))
             return copy_out_small(s, pin, p, bytes, 1, &host, &bytes, cudaStreamLegacy, "env copy");
@@ -2396,6 +2426,9 @@ static int task_rows_out(const arc_sim* s, const int* ids, size_t n, double* out
                          unsigned char* terminated, unsigned char* truncated, signed char* cause, const char* where)
 {
     if (sync(s, where))
+        return ARC_ERR_CUDA;
+    const OnDeviceOf device(s);
+    if (check(s, device.status, where))
         return ARC_ERR_CUDA;
     std::lock_guard<std::mutex> lock(s->small_mu);
     for (size_t first = 0; first < n; first += s->rows_cap) {

@@ -84,3 +84,19 @@ def test_two_threads_read_task_rows(lib, sim):
     lib.fake_delay_us(500)
     _at_once(lambda: [read(n) for n in range(1, 64, 2)], lambda: [read(n) for n in range(2, 65, 2)])
     assert lib.fake_launches() == before + 64 and lib.fake_with_freed_memory() == 0
+
+
+def test_rows_are_gathered_on_the_sims_device(lib, sim):
+    """A thread whose current device is another one reads what it did with
+    plain copies, and keeps its device."""
+    out, device = np.zeros((64, TASK_STATE_SIZE)), _int()
+    ids = np.arange(64, dtype=np.int32)
+    lib.cudaSetDevice(1)
+    try:
+        before = lib.fake_launches(), lib.fake_on_other_device()
+        assert lib.arc_env_get_task_state(sim, ids.ctypes.data, 64, out.ctypes.data) == 0
+        lib.cudaGetDevice(ctypes.byref(device))
+    finally:
+        lib.cudaSetDevice(0)
+    assert (lib.fake_launches(), lib.fake_on_other_device()) == (before[0] + 1, before[1])
+    assert device.value == 1
