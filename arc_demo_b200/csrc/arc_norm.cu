@@ -4,15 +4,22 @@
 // Bound by memory and launches: the batch is read for its moments, and read
 // and written once to normalise it. As tensor operations the same step took
 // 55 launches (six FP64 copies of the batch among them) and 207 us of GPU
-// time at 10,007 x 195; here three launches and 25 us (4.5, 4.8 and 16; the
-// 40 MB read and written take 6 us at the copy rate, the rest is the FP64
-// arithmetic per element and launch latency):
-//   k_norm_moments  per block of rows and 256 columns: sums of (x - x0) and
-//                   (x - x0)^2 in FP64, x0 the column's first row, so that a
-//                   constant column has no variance at all; the last column
-//                   of blocks does the same for the discounted returns.
-//   k_norm_merge    a warp per column adds the blocks' sums and merges them
-//                   into the running statistics (Chan, Golub, LeVeque 1979).
+// time at 10,007 x 195; here three launches and 23 us, with a batch in L2
+// (5.2, 6.8 and 11.2; the 40 MB read and written take 6 us at the copy rate, the
+// rest is the FP64 arithmetic per element and launch latency):
+//   k_norm_moments  per block of rows and 256 columns: the column's mean and
+//                   sum of squared deviations from it, in FP64 and two passes
+//                   (the second reads from L1 and L2) with the deviations'
+//                   own sum as the correction (Chan, Golub, LeVeque 1983); the
+//                   last column of blocks does the same for the discounted
+//                   returns.
+//   k_norm_merge    a warp per column merges the blocks' moments in the same
+//                   two passes, and the result into the running statistics
+//                   (Chan, Golub, LeVeque 1979). A constant column has no
+//                   variance at all, and no row is a reference for the others:
+//                   in one pass around the first row's values (3.8 and 4.4
+//                   us) a first row 1,000 deviations out cost the variance
+//                   three digits.
 //   k_norm_apply    observations, terminal observations, rewards; the ended
 //                   worlds' returns to zero.
 // Sums are added in one order, so a step gives the same bits every time.
@@ -39,70 +46,113 @@ __device__ __forceinline__ double next_return(const arc_norm_step_args& a, long 
     return a.training ? __dadd_rn(__dmul_rn(a.returns[i], a.gamma), (double)a.rewards[i]) : a.returns[i];
 }
 
-// The value a column's sums are taken around: its first row's, if finite.
-__device__ __forceinline__ double origin_of(double first) { return isfinite(first) ? first : 0.0; }
-
-// blockIdx.y: a tile of 256 columns, or (the last, when training) the
-// returns. work: [2][row blocks][cols + 1] sums.
-__global__ void __launch_bounds__(kNormThreads) k_norm_moments(const __grid_constant__ arc_norm_step_args a)
+// The rows of block b of `blocks`: first, and how many.
+__device__ __forceinline__ void rows_of(long long rows, int blocks, int b, long long& first, int& count)
 {
-    const int tid = threadIdx.x, col = blockIdx.y * kNormThreads + tid, blocks = gridDim.x;
-    const long long per = (a.rows + blocks - 1) / blocks, r0 = blockIdx.x * per;
-    const long long r1 = r0 + per < a.rows ? r0 + per : a.rows;
-    double* first = a.work + (size_t)blockIdx.x * (a.cols + 1);
-    double* second = first + (size_t)blocks * (a.cols + 1);
-    double s = 0.0, q = 0.0;
-    if (blockIdx.y + 1 < gridDim.y) {
-        if (col >= a.cols || !a.norm_obs)
-            return;
-        const double x0 = origin_of((double)a.obs[col]);
-        const float* x = a.obs + (size_t)r0 * a.cols + col;
-        long long r = r0;
-        for (; r + 8 <= r1; r += 8, x += (size_t)8 * a.cols) {
-            float v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                v[u] = x[(size_t)u * a.cols];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const double d = (double)v[u] - x0;
-                s += d;
-                q = __fma_rn(d, d, q);
-            }
-        }
-        for (; r < r1; ++r, x += a.cols) {
-            const double d = (double)*x - x0;
-            s += d;
-            q = __fma_rn(d, d, q);
-        }
-        first[col] = s;
-        second[col] = q;
-        return;
-    }
+    const long long per = (rows + blocks - 1) / blocks;
+    first = b * per;
+    const long long left = rows - first;
+    count = (int)(left < per ? (left > 0 ? left : 0) : per);
+}
+
+// Of n values whose deviations from the rounded mean `hi` sum to s and their
+// squares to q: the mean's rest, and the squared deviations' sum from hi + rest.
+struct Moments {
+    double rest, m2;
+};
+__device__ __forceinline__ Moments corrected(double hi, double s, double q, double n)
+{
+    const double m2 = q - s * (s / n);
+    return Moments{isfinite(hi) ? s / n : 0.0, m2 < 0.0 ? 0.0 : m2};  // NaN stays
+}
+
+// The sums of s and q over the block, to every thread.
+__device__ __forceinline__ void block_sums(double& s, double& q)
+{
     __shared__ double sum[2][kNormThreads / 32];
-    const double x0 = origin_of(next_return(a, 0));
-    for (long long r = r0 + tid; r < r1; r += kNormThreads) {
-        const double d = next_return(a, r) - x0;
-        s += d;
-        q = __fma_rn(d, d, q);
-    }
     for (int off = 16; off > 0; off >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, off);
         q += __shfl_xor_sync(0xffffffffu, q, off);
     }
-    if ((tid & 31) == 0) {
-        sum[0][tid / 32] = s;
-        sum[1][tid / 32] = q;
+    __syncthreads();  // an earlier call's sums are read
+    if ((threadIdx.x & 31) == 0) {
+        sum[0][threadIdx.x / 32] = s;
+        sum[1][threadIdx.x / 32] = q;
     }
     __syncthreads();
+    s = q = 0.0;
+    for (int w = 0; w < kNormThreads / 32; ++w) {
+        s += sum[0][w];
+        q += sum[1][w];
+    }
+}
+
+// f(x[0]), f(x[cols]), ..., `count` of them, eight loads in flight.
+template <class Fn> __device__ __forceinline__ void each_row(const float* x, int count, int cols, Fn&& f)
+{
+    int r = 0;
+    for (; r + 8 <= count; r += 8, x += (size_t)8 * cols) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            v[u] = x[(size_t)u * cols];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            f((double)v[u]);
+    }
+    for (; r < count; ++r, x += cols)
+        f((double)*x);
+}
+
+// blockIdx.y: a tile of 256 columns, or (the last, when training) the
+// returns. work: [3][row blocks][cols + 1] means, their rests (a block's mean
+// rounded to FP64 is too far off where the deviations are small beside it),
+// sums of squares.
+__global__ void __launch_bounds__(kNormThreads) k_norm_moments(const __grid_constant__ arc_norm_step_args a)
+{
+    const int tid = threadIdx.x, col = blockIdx.y * kNormThreads + tid, blocks = gridDim.x;
+    long long r0;
+    int count;
+    rows_of(a.rows, blocks, blockIdx.x, r0, count);
+    if (count == 0)
+        return;  // k_norm_merge does not read its moments
+    const size_t plane = (size_t)blocks * (a.cols + 1);
+    double* out = a.work + (size_t)blockIdx.x * (a.cols + 1);
+    double s = 0.0, q = 0.0;
+    if (blockIdx.y + 1 < gridDim.y) {
+        if (col >= a.cols || !a.norm_obs)
+            return;
+        const float* x = a.obs + (size_t)r0 * a.cols + col;
+        each_row(x, count, a.cols, [&](double v) { s += v; });
+        const double mean = s / count;
+        s = 0.0;
+        each_row(x, count, a.cols, [&](double v) {
+            const double d = v - mean;
+            s += d;
+            q = __fma_rn(d, d, q);
+        });
+        const Moments m = corrected(mean, s, q, count);
+        out[col] = mean;
+        out[plane + col] = m.rest;
+        out[2 * plane + col] = m.m2;
+        return;
+    }
+    for (int r = tid; r < count; r += kNormThreads)
+        s += next_return(a, r0 + r);
+    block_sums(s, q);
+    const double mean = s / count;
+    s = q = 0.0;
+    for (int r = tid; r < count; r += kNormThreads) {
+        const double d = next_return(a, r0 + r) - mean;
+        s += d;
+        q = __fma_rn(d, d, q);
+    }
+    block_sums(s, q);
     if (tid == 0) {
-        s = q = 0.0;
-        for (int w = 0; w < kNormThreads / 32; ++w) {
-            s += sum[0][w];
-            q += sum[1][w];
-        }
-        first[a.cols] = s;
-        second[a.cols] = q;
+        const Moments m = corrected(mean, s, q, count);
+        out[a.cols] = mean;
+        out[plane + a.cols] = m.rest;
+        out[2 * plane + a.cols] = m.m2;
     }
 }
 
@@ -112,24 +162,45 @@ __global__ void __launch_bounds__(kNormThreads) k_norm_merge(const __grid_consta
     const int col = blockIdx.x * (kNormThreads / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (col > a.cols || (col < a.cols && !a.norm_obs))
         return;
-    const double* first = a.work + col;
-    const double* second = first + (size_t)blocks * (a.cols + 1);
+    constexpr int kEach = kNormBlocks / 32;
+    const size_t plane = (size_t)blocks * (a.cols + 1);
+    double mean_of[kEach], rest_of[kEach], m2_of[kEach], n_of[kEach];
     double s = 0.0, q = 0.0;
-    for (int b = lane; b < blocks; b += 32) {
-        s += first[(size_t)b * (a.cols + 1)];
-        q += second[(size_t)b * (a.cols + 1)];
+#pragma unroll
+    for (int u = 0; u < kEach; ++u) {
+        const int b = lane + 32 * u;
+        long long first = 0;
+        int count = 0;
+        if (b < blocks)
+            rows_of(a.rows, blocks, b, first, count);
+        const double* at = a.work + (size_t)b * (a.cols + 1) + col;
+        n_of[u] = count;
+        mean_of[u] = count ? at[0] : 0.0;
+        rest_of[u] = count ? at[plane] : 0.0;
+        m2_of[u] = count ? at[2 * plane] : 0.0;
+        s += n_of[u] * (mean_of[u] + rest_of[u]);
     }
+    for (int off = 16; off > 0; off >>= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, off);
+    const double n = (double)a.rows, hi = s / n;
+    s = 0.0;
+#pragma unroll
+    for (int u = 0; u < kEach; ++u)
+        if (n_of[u] != 0.0) {
+            const double d = mean_of[u] - hi + rest_of[u];
+            s += n_of[u] * d;
+            q += m2_of[u] + n_of[u] * d * d;
+        }
     for (int off = 16; off > 0; off >>= 1) {
         s += __shfl_xor_sync(0xffffffffu, s, off);
         q += __shfl_xor_sync(0xffffffffu, q, off);
     }
     if (lane != 0)
         return;
+    const Moments m = corrected(hi, s, q, n);
+    const double batch_mean = hi + m.rest;
     const bool ret = col == a.cols;
-    const double n = (double)a.rows, shift = s / n;
-    const double batch_mean = origin_of(ret ? next_return(a, 0) : (double)a.obs[col]) + shift;
-    double batch_var = q / n - shift * shift;
-    batch_var = batch_var < 0.0 ? 0.0 : batch_var;  // NaN stays
+    const double batch_var = m.m2 / n;
     const double mean = ret ? *a.ret_mean : a.obs_mean[col], var = ret ? *a.ret_var : a.obs_var[col];
     const double count = ret ? a.ret_count : a.obs_count, total = count + n;
     const double delta = batch_mean - mean;
@@ -187,7 +258,7 @@ extern "C" {
 
 long long arc_norm_work_size(long long rows, int cols)
 {
-    return rows > 0 && cols > 0 ? 2ll * arc::norm_row_blocks(rows) * (cols + 1) : 0;
+    return rows > 0 && cols > 0 ? 3ll * arc::norm_row_blocks(rows) * (cols + 1) : 0;
 }
 
 int arc_norm_step(const arc_norm_step_args* a, void* stream)

@@ -123,3 +123,33 @@ def test_overridden_normalisation_is_used():
     with torch.autograd.forward_ad.dual_level():
         assert b._step_kernels(b.old_obs, r, d, {}) is None
     assert b._step_kernels(b.old_obs, r, d, {}) is not None
+
+
+@pytest.mark.parametrize("n", [7, 4000, 8195])
+def test_moments_do_not_lean_on_one_row(n):
+    """A first (or any) row far out costs the other rows' moments nothing:
+    the batch's mean and variance against 80-bit arithmetic. Per variance at
+    most 33 rows in turn, 13 sums of lanes and blocks and 8 roundings beside
+    them, each 2^-53 of the sum; per mean a quarter of that, of the largest
+    summand's share."""
+    import numpy as np
+
+    g = np.random.default_rng(n)
+    x = (g.normal(size=(n, 9)) * np.logspace(-3, 3, 9) + np.linspace(-50, 50, 9)).astype(np.float32)
+    x[0] += np.array([0, 1, 10, 1e2, 1e3, 1e4, 1e5, 0, 0]) * x.std(0)
+    x[n // 2, 7] += 1e5 * x[:, 7].std()
+    x[:, 8] = 0.1
+    a = DeviceVecNormalize(Env(n, 9))
+    a.reset()
+    a.obs_rms.count = a.ret_rms.count = 0.0  # the merged statistics are then the batch's
+    a.returns = torch.as_tensor(np.concatenate([[1e5], g.normal(size=n - 1)]), device="cuda")
+    r, d = torch.as_tensor(g.normal(size=n).astype(np.float32), device="cuda"), torch.zeros(n, device="cuda").bool()
+    returns = a.returns.cpu().numpy() * a.gamma + r.cpu().numpy().astype(np.float64)
+    assert a._step_kernels(torch.as_tensor(x, device="cuda"), r, d, {}) is not None
+    for got, data in ((a.obs_rms, x), (a.ret_rms, returns[:, None])):
+        data = data.astype(np.longdouble)
+        mean = data.mean(0)
+        var = ((data - mean) ** 2).mean(0)
+        assert (np.abs(got.var.cpu().numpy() - var) <= 54 * 2.0**-53 * var).all()
+        assert (np.abs(got.mean.cpu().numpy() - mean) <= 14 * 2.0**-53 * np.abs(data).mean(0)).all()
+    assert a.obs_rms.var[8] == 0.0
