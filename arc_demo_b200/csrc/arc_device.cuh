@@ -32,6 +32,17 @@ constexpr int kContactRec = 8;
 constexpr int kNumLegs = 4;      // csrc/arc_robot.h:19-20
 constexpr int kNumJoints = 12;
 
+// a / b correctly rounded, y = 1 / b correctly rounded: the quotient from
+// the reciprocal, corrected twice by its exact remainder (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990). a / b infinite gives NaN.
+__device__ __forceinline__ double divide(double a, double b, double y)
+{
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
 template <class R> struct DevModel {
     int nb, nj, ns, n_channels;
     int substeps;

@@ -4,8 +4,8 @@
 // Bound by memory and launches: the batch is read for its moments, and read
 // and written once to normalise it. As tensor operations the same step took
 // 55 launches (six FP64 copies of the batch among them) and 207 us of GPU
-// time at 10,007 x 195; here three launches and 23 us, with a batch in L2
-// (5.2, 6.8 and 11.2; the 40 MB read and written take 6 us at the copy rate, the
+// time at 10,007 x 195; here three launches and 25 us, with a batch in L2
+// (5.0, 6.9 and 13.3; the 40 MB read and written take 6 us at the copy rate, the
 // rest is the FP64 arithmetic per element and launch latency):
 //   k_norm_moments  per block of rows and 256 columns: the column's mean and
 //                   sum of squared deviations from it, in FP64 and two passes
@@ -21,7 +21,9 @@
 //                   us) a first row 1,000 deviations out cost the variance
 //                   three digits.
 //   k_norm_apply    observations, terminal observations, rewards; the ended
-//                   worlds' returns to zero.
+//                   worlds' returns to zero. Divides by the deviation: with a
+//                   product by its reciprocal it took 11.2 us, and rounded
+//                   once more than a division.
 // Sums are added in one order, so a step gives the same bits every time.
 #include "arc_kernels.cuh"
 #include "../../include/arc_sim.h"
@@ -31,7 +33,7 @@ namespace arc {
 namespace {
 
 constexpr int kNormThreads = 256;
-constexpr int kNormMaxCols = 2048;   // mean and scale of every column in shared memory
+constexpr int kNormMaxCols = 2048;   // mean, deviation and its reciprocal of every column in shared memory
 constexpr int kNormBlocks = 256;     // blocks of rows at most
 
 int norm_row_blocks(long long rows)
@@ -209,6 +211,13 @@ __global__ void __launch_bounds__(kNormThreads) k_norm_merge(const __grid_consta
     (ret ? a.ret_var_out : a.obs_var_out + col)[0] = m2 / total;
 }
 
+// a / b where y = 1 / b, infinities and NaN as a division gives them
+__device__ __forceinline__ double quotient(double a, double b, double y)
+{
+    const double q = divide(a, b, y);
+    return isfinite(q) ? q : a * y;
+}
+
 __device__ __forceinline__ double clip_to(double v, double c) { return v < -c ? -c : (v > c ? c : v); }
 
 // blockIdx.y: 0 the observations (and, in the first blocks, rewards and
@@ -222,10 +231,12 @@ __global__ void __launch_bounds__(kNormThreads) k_norm_apply(const __grid_consta
     const bool updated = a.training && a.norm_obs;
     if (src && dst) {
         double* mean = stats;
-        double* scale = stats + a.cols;
+        double* dev = stats + a.cols;
+        double* scale = dev + a.cols;
         for (int c = tid; c < a.cols; c += kNormThreads) {
             mean[c] = updated ? a.obs_mean_out[c] : a.obs_mean[c];
-            scale[c] = 1.0 / sqrt((updated ? a.obs_var_out[c] : a.obs_var[c]) + a.epsilon);
+            dev[c] = sqrt((updated ? a.obs_var_out[c] : a.obs_var[c]) + a.epsilon);
+            scale[c] = 1.0 / dev[c];
         }
         __syncthreads();
         const size_t total = (size_t)a.rows * a.cols;
@@ -234,7 +245,7 @@ __global__ void __launch_bounds__(kNormThreads) k_norm_apply(const __grid_consta
         int c = (int)(e % a.cols);
         const int dc = (int)(step % a.cols);
         for (; e < total; e += step) {
-            dst[e] = (float)clip_to(((double)src[e] - mean[c]) * scale[c], a.clip_obs);
+            dst[e] = (float)clip_to(quotient((double)src[e] - mean[c], dev[c], scale[c]), a.clip_obs);
             c += dc;
             c -= c >= a.cols ? a.cols : 0;
         }
@@ -277,7 +288,7 @@ int arc_norm_step(const arc_norm_step_args* a, void* stream)
     const size_t each = (size_t)a->rows * a->cols, per_block = (size_t)kNormThreads * 8;
     const size_t want = (each + per_block - 1) / per_block;
     k_norm_apply<<<dim3((unsigned)(want < 1024 ? want : 1024), a->terminal_obs && a->terminal_out ? 2 : 1), kNormThreads,
-                   2 * sizeof(double) * a->cols, st>>>(*a);
+                   3 * sizeof(double) * a->cols, st>>>(*a);
     return cudaGetLastError() == cudaSuccess ? ARC_OK : ARC_ERR_CUDA;
 }
 

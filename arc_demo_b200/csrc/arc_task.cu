@@ -190,17 +190,6 @@ __device__ __forceinline__ void heading_of(Q4<double> q, double& cy, double& sy)
     sy = sin(yaw);
 }
 
-// a / b correctly rounded, y = 1 / b correctly rounded: the quotient from
-// the reciprocal, corrected twice by its exact remainder (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990). a / b infinite gives NaN.
-__device__ __forceinline__ double divide(double a, double b, double y)
-{
-    double q = __dmul_rn(a, y);
-    q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-
 // Where a world's terrain heights are sampled (csrc/arc_sim.c:185-203): its
 // heading, position and columns.
 template <class R> struct HeightFrame {

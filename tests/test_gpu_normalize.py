@@ -153,3 +153,25 @@ def test_moments_do_not_lean_on_one_row(n):
         assert (np.abs(got.var.cpu().numpy() - var) <= 54 * 2.0**-53 * var).all()
         assert (np.abs(got.mean.cpu().numpy() - mean) <= 14 * 2.0**-53 * np.abs(data).mean(0)).all()
     assert a.obs_rms.var[8] == 0.0
+
+
+def test_quotients_are_divisions():
+    """(obs - mean) / deviation rounds once, as a division does: quotients
+    halfway between two FP32 values (exact in FP64) round to the even one,
+    which a product with the reciprocal misses by the last bit; infinities,
+    NaN and deviations of zero as a division gives them."""
+    bad = float("inf"), float("-inf"), float("nan"), 0.0, 1.0
+    a = DeviceVecNormalize(Env(5, 900), training=False, norm_reward=False, clip_obs=float("inf"), epsilon=0.0)
+    a.reset()
+    dev = torch.arange(3, 1803, 2, dtype=torch.float64, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    half = torch.randint(2**23, 2**24, (900,), device="cuda", generator=g).double() + 0.5
+    a.obs_rms.mean, a.obs_rms.var = -half * dev, dev.square()
+    a.obs_rms.mean[:10] = 0.0
+    a.obs_rms.var[5:10] = 0.0
+    x = torch.zeros((5, 900), device="cuda")
+    x[:, :10] = torch.tensor(bad, device="cuda")[:, None]
+    r, d = torch.zeros(5, device="cuda"), torch.zeros(5, device="cuda").bool()
+    got = a._step_kernels(x, r, d, {})[0]
+    assert torch.equal(got[:, 10:], half[10:].float().expand(5, -1))
+    assert torch.equal(got.nan_to_num(7.0), a.normalize_obs(x).nan_to_num(7.0))
