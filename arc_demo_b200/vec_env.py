@@ -194,13 +194,12 @@ class DeviceVecNormalize:
         dev, f32, f64 = obs.device, torch.float32, torch.float64
         term = infos.get("terminal_observation") if type(infos) is dict else None
         rms, ret = self.obs_rms, self.ret_rms
-        cls, base = type(self), DeviceVecNormalize
-        if (cls.normalize_obs is not base.normalize_obs or cls.normalize_reward is not base.normalize_reward
-                or type(rms) is not DeviceRunningMeanStd or type(ret) is not DeviceRunningMeanStd
+        if (_replaced(self, _NORMALIZE) or any(type(r) is not DeviceRunningMeanStd or _replaced(r, _UPDATE)
+                                               for r in (rms, ret))
                 or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
                 or not all(isinstance(v, (int, float)) for v in (rms.count, ret.count, self.gamma, self.epsilon,
                                                                  self.clip_obs, self.clip_reward))):
-            return None  # a subclass's own normalisation, something that traces the operations, tensor settings
+            return None  # normalisation of the caller's own, something that traces the operations, tensor settings
         if (cols > 2048 or n != self.num_envs or type(infos) is not dict
                 or not _plain(obs, f32, (n, cols), dev) or not _plain(rewards, f32, (n,), dev)
                 or not _plain(dones, torch.bool, (n,), dev) or not _plain(self.returns, f64, (n,), dev)
@@ -253,3 +252,13 @@ class DeviceVecNormalize:
             self.returns = torch.zeros(self.num_envs, dtype=torch.float64, device=dev)
         self.obs_rms.load_state_dict(d["obs_rms"])
         self.ret_rms.load_state_dict(d["ret_rms"])
+
+
+# the methods that the kernels stand in for, unless a subclass, an instance or
+# a patched class has others
+_UPDATE = {n: getattr(DeviceRunningMeanStd, n) for n in ("update", "update_from_moments")}
+_NORMALIZE = {n: getattr(DeviceVecNormalize, n) for n in ("normalize_obs", "normalize_reward")}
+
+
+def _replaced(obj, methods) -> bool:
+    return any(n in vars(obj) or getattr(type(obj), n) is not f for n, f in methods.items())

@@ -175,3 +175,30 @@ def test_quotients_are_divisions():
     got = a._step_kernels(x, r, d, {})[0]
     assert torch.equal(got[:, 10:], half[10:].float().expand(5, -1))
     assert torch.equal(got.nan_to_num(7.0), a.normalize_obs(x).nan_to_num(7.0))
+
+
+def test_replaced_methods_are_used(monkeypatch):
+    """Functions set on the normaliser or its statistics, or patched into
+    their classes, decide as they do for the tensor operations."""
+    def fresh():
+        a = DeviceVecNormalize(Env(16, 6))
+        a.reset()
+        return a
+
+    a = fresh()
+    a.normalize_obs = lambda obs: 0.5 * obs
+    obs = a.step(None)[0]
+    assert torch.equal(obs, 0.5 * a.old_obs)
+    a = fresh()
+    a.normalize_reward = lambda r: r + 1
+    assert torch.equal(a.step(None)[1], a.old_reward + 1)
+    for name in ("update", "update_from_moments"):
+        for rms in ("obs_rms", "ret_rms"):
+            a, calls = fresh(), []
+            setattr(getattr(a, rms), name, lambda *x: calls.append(x))
+            a.step(None)
+            assert len(calls) == 1
+    a, calls = fresh(), []
+    monkeypatch.setattr(DeviceRunningMeanStd, "update", lambda self, x: calls.append(x))
+    a.step(None)
+    assert len(calls) == 2
