@@ -198,8 +198,9 @@ class DeviceVecNormalize:
                                                for r in (rms, ret))
                 or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
                 or not all(isinstance(v, (int, float)) for v in (rms.count, ret.count, self.gamma, self.epsilon,
-                                                                 self.clip_obs, self.clip_reward))):
-            return None  # normalisation of the caller's own, something that traces the operations, tensor settings
+                                                                 self.clip_obs, self.clip_reward))
+                or not (self.clip_obs >= 0.0 and self.clip_reward >= 0.0)):
+            return None  # normalisation of the caller's own, something that traces the operations, odd settings
         if (cols > 2048 or n != self.num_envs or type(infos) is not dict
                 or not _plain(obs, f32, (n, cols), dev) or not _plain(rewards, f32, (n,), dev)
                 or not _plain(dones, torch.bool, (n,), dev) or not _plain(self.returns, f64, (n,), dev)

@@ -202,3 +202,14 @@ def test_replaced_methods_are_used(monkeypatch):
     monkeypatch.setattr(DeviceRunningMeanStd, "update", lambda self, x: calls.append(x))
     a.step(None)
     assert len(calls) == 2
+
+
+@pytest.mark.parametrize("limit", [-1.0, float("nan")])
+def test_limits_that_are_no_limits(limit):
+    """Limits below zero, or NaN: what clamp makes of them."""
+    kw = dict(clip_obs=limit, clip_reward=limit)
+    a, b = DeviceVecNormalize(Env(33, 6), **kw), Tensors(Env(33, 6), **kw)
+    a.reset(), b.reset()
+    x, y = a.step(None), b.step(None)
+    for u, v in zip(x[:3], y[:3]):
+        assert torch.equal(u.nan_to_num(7.0), v.nan_to_num(7.0))
