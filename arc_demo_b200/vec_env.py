@@ -197,6 +197,7 @@ class DeviceVecNormalize:
         if (_replaced(self, _NORMALIZE) or any(type(r) is not DeviceRunningMeanStd or _replaced(r, _UPDATE)
                                                for r in (rms, ret))
                 or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+                or torch.jit.is_tracing()
                 or not all(isinstance(v, (int, float)) for v in (rms.count, ret.count, self.gamma, self.epsilon,
                                                                  self.clip_obs, self.clip_reward))
                 or not (self.clip_obs >= 0.0 and self.clip_reward >= 0.0)):

@@ -213,3 +213,12 @@ def test_limits_that_are_no_limits(limit):
     x, y = a.step(None), b.step(None)
     for u, v in zip(x[:3], y[:3]):
         assert torch.equal(u.nan_to_num(7.0), v.nan_to_num(7.0))
+
+
+def test_traced_steps_take_the_tensor_operations():
+    a, seen = DeviceVecNormalize(Env(16, 6)), []
+    a.reset()
+    r, d = torch.zeros(16, device="cuda"), torch.zeros(16, device="cuda").bool()
+    torch.jit.trace(lambda x: x + 0 * len(seen.append(a._step_kernels(x, r, d, {})) or seen), a.old_obs,
+                    check_trace=False)
+    assert seen == [None]
