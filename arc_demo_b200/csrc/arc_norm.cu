@@ -278,6 +278,13 @@ int arc_norm_step(const arc_norm_step_args* a, void* stream)
     if (!a || a->rows <= 0 || a->cols <= 0 || a->cols > kNormMaxCols || !a->obs || !a->rewards || !a->dones ||
         !a->returns || !a->returns_out || !a->work || (a->norm_reward && !a->rewards_out))
         return ARC_ERR_ARG;
+    // the statistics that the step reads and writes
+    const bool reads_obs = (a->training && a->norm_obs) || a->obs_out || (a->terminal_obs && a->terminal_out);
+    if ((reads_obs && (!a->obs_mean || !a->obs_var)) ||
+        (a->training && a->norm_obs && (!a->obs_mean_out || !a->obs_var_out)) ||
+        (a->training && (!a->ret_mean || !a->ret_mean_out || !a->ret_var_out)) ||
+        ((a->training || a->norm_reward) && !a->ret_var))
+        return ARC_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     const int blocks = norm_row_blocks(a->rows);
     if (a->training) {

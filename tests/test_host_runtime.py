@@ -1,5 +1,6 @@
-"""Read-outs of one sim by several host threads, on a runtime without a GPU
-(fake_cudart.cpp, linked with the library's own objects)."""
+"""The library's host code on a runtime without a GPU (fake_cudart.cpp, linked
+with the library's own objects): read-outs of one sim by several threads, and
+arguments that must not reach a kernel."""
 
 import ctypes
 import subprocess
@@ -11,6 +12,7 @@ import pytest
 
 from arc_demo_b200.build import BUILD, build, nvcc, sources
 from arc_demo_b200.task import ENDED_DIFFICULTY, REWARD, TASK_STATE_SIZE
+from arc_demo_b200.vec_env import _NormArgs
 
 _vp, _int = ctypes.c_void_p, ctypes.c_int
 
@@ -100,3 +102,21 @@ def test_rows_are_gathered_on_the_sims_device(lib, sim):
         lib.cudaSetDevice(0)
     assert (lib.fake_launches(), lib.fake_on_other_device()) == (before[0] + 1, before[1])
     assert device.value == 1
+
+
+@pytest.mark.parametrize("training,norm_obs,norm_reward,needs", [
+    (1, 1, 1, "obs_mean obs_var ret_mean ret_var obs_mean_out obs_var_out ret_mean_out ret_var_out rewards_out"),
+    (1, 0, 0, "ret_mean ret_var ret_mean_out ret_var_out"),
+    (0, 1, 1, "obs_mean obs_var ret_var rewards_out"),
+    (0, 0, 0, "")])
+def test_normalisation_refuses_missing_statistics(lib, training, norm_obs, norm_reward, needs):
+    """arc_norm_step without a pointer that its kernels would follow."""
+    always = ("obs", "rewards", "dones", "returns", "returns_out", "work")
+    a = _NormArgs(rows=4, cols=3, training=training, norm_obs=norm_obs, norm_reward=norm_reward)
+    for name in (*always, *needs.split()) + (("obs_out", "terminal_obs", "terminal_out") if norm_obs else ()):
+        setattr(a, name, 4096)
+    assert lib.arc_norm_step(ctypes.byref(a), None) == 0
+    for name in (*always, *needs.split()):
+        b = _NormArgs.from_buffer_copy(a)
+        setattr(b, name, None)
+        assert lib.arc_norm_step(ctypes.byref(b), None) != 0, name
