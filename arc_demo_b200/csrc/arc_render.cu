@@ -723,8 +723,8 @@ __device__ F3 glow_along(const FrameK& fr, unsigned mask, F3 O, F3 D, float tdep
 template <class R>
 __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
     k_render(const VisK* __restrict__ vis, int nv, const FrameK* __restrict__ frames, Worlds<R> W,
-             const int* __restrict__ ids, int width, int height, int tiles_x, int n_tiles,
-             int samples, unsigned char* __restrict__ out)
+             const int* __restrict__ ids, int width, int height, int tiles_x, int samples,
+             unsigned char* __restrict__ out)
 {
     __shared__ alignas(FrameK) int frame_words[kFrameWords];
     const FrameK& fr = *reinterpret_cast<const FrameK*>(frame_words);  // up to ball
@@ -756,9 +756,7 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
         return fwd + scale(right, (wx - 0.5f * width) * sx) + scale(up, (wy - 0.5f * height) * sy);
     };
 
-    {
-    const int tile = blockIdx.x;
-    const int x0 = tile % tiles_x * kTileW, r0 = tile / tiles_x * kTileH;
+    const int tile = blockIdx.x, x0 = tile % tiles_x * kTileW, r0 = tile / tiles_x * kTileH;
     // cull the items' bounding spheres against the tile's frustum
     {
         const float wx0 = (float)x0, wx1 = (float)(x0 + kTileW);
@@ -1032,7 +1030,6 @@ __global__ void __launch_bounds__(kThreads, ARC_RENDER_MIN_BLOCKS)
     unsigned char* o = out + (((size_t)item * height + row) * width + px) * 3;
     for (int k = 0; k < 3; ++k)
         o[k] = (unsigned char)((acc[k] + samples / 2) / samples);
-    }
 }
 
 __device__ __forceinline__ double wrap_angle(double a)
@@ -1675,18 +1672,8 @@ int launch(arc_renderer* r, const SimView& sv, const Worlds<R>& W, const int* d_
     if (report(cudaGetLastError(), "frame setup"))
         return ARC_ERR_CUDA;
     const int tiles_x = (r->w + rd::kTileW - 1) / rd::kTileW, tiles_y = (r->h + rd::kTileH - 1) / rd::kTileH;
-    // a CTA copies its frame's record once for up to four tiles, fewer while
-    // that would leave the GPU less than eight waves of CTAs
-    const int n_tiles = tiles_x * tiles_y;
-    int dev = 0, sms = 0;
-    if (report(cudaGetDevice(&dev), "device") ||
-        report(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device"))
-        return ARC_ERR_CUDA;
-    const long long per = (long long)n_tiles * n / (8ll * ARC_RENDER_MIN_BLOCKS * sms);
-    const int each = 1; (void)per;
-    dim3 grid((n_tiles + each - 1) / each, n);
-    rd::k_render<R><<<grid, rd::kThreads, 0, st>>>(r->d_vis, r->nv, r->d_frames, W, d_ids, r->w, r->h, tiles_x,
-                                                   n_tiles, r->samples, d_rgb);
+    rd::k_render<R><<<dim3(tiles_x * tiles_y, n), rd::kThreads, 0, st>>>(r->d_vis, r->nv, r->d_frames, W, d_ids, r->w,
+                                                                         r->h, tiles_x, r->samples, d_rgb);
     return report(cudaGetLastError(), "render");
 }
 
