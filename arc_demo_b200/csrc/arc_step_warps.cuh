@@ -635,9 +635,8 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue, bool s
 }
 
 // One control step of a group's worlds (items first .. first + per_group - 1,
-// at most 32: worlds ids[item], or item itself without ids) by kThreads
-// threads, thread tid = lane j of warp `leg`, in the order of the operation
-// list `list`. On return the
+// at most 32: worlds ids[item], or item itself without ids) by the group's
+// warps, lane j of warp `leg` here, in the order of the operation list `list`. On return the
 // worlds' records, flags, time and unstable marks are written and every
 // thread of the CTA has passed the group's last barrier.
 //
@@ -651,10 +650,9 @@ inline GroupPlan group_plan(int n_items, int sms, bool alone, bool queue, bool s
 template <class Sync, class Mem>
 __device__ __forceinline__ void step_group(const Sync& sync, Mem& sm, const DevModel<F>& M, const Worlds<F>& W, const Actuation& A,
                                            F* __restrict__ spill, int spill_per_lane, int lane_cap,
-                                           const int* __restrict__ ids, int n_items, int first, int tid, int leg,
-                                           int j, int sub0, int sub1, F* __restrict__ tile_q, int per_group, int list)
+                                           const int* __restrict__ ids, int n_items, int first, int leg, int j,
+                                           int sub0, int sub1, F* __restrict__ tile_q, int per_group, int list)
 {
-    (void)tid;
     // a split group steps whole control steps with uncapped lists only
     const bool first_tile = Sync::kSplit || sub0 == 0, last_tile = Sync::kSplit || sub1 >= M.substeps;
     // what this warp has of the leg: the coxa (leg 0: and the torso), the femur
@@ -1130,7 +1128,7 @@ __device__ __forceinline__ void step_split(SplitSmem& sm, const DevModel<F>& M, 
 {
     const int tid = threadIdx.x % kThreads;
     step_group(SplitSync{(int)threadIdx.x / kThreads}, sm, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
-               blockIdx.x * per_group, tid, tid / kWorlds, tid % kWorlds, 0, M.substeps, nullptr, per_group, 0);
+               blockIdx.x * per_group, tid / kWorlds, tid % kWorlds, 0, M.substeps, nullptr, per_group, 0);
 }
 
 // The groups of a launch in CTAs of kAligned groups, one CTA per SM: slot g of
@@ -1168,7 +1166,7 @@ __device__ __forceinline__ void step_aligned(AlignedSmem& as, const DevModel<F>&
             sync.join(leg);
         const bool over = group >= whole;
         step_group(sync, as.step[slot], M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
-                   over ? whole * kWorlds + (group - whole) * rest_per : group * kWorlds, tid, leg, j, sub0, sub1,
+                   over ? whole * kWorlds + (group - whole) * rest_per : group * kWorlds, leg, j, sub0, sub1,
                    tile_q, over ? rest_per : kWorlds, over && tail ? (int)kListLatency : list);
         if (j == 0)
             sync.leave(leg);

@@ -43,7 +43,7 @@ k_step_warps64(const __grid_constant__ DevModel<double> M, Worlds<double> W, Act
 #pragma unroll 1
     for (int group = first; group < n_groups;) {
         wl::step_group(wl::CtaSync{}, sm.step, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
-                       group * per_group, tid, leg, j, 0, M.substeps, nullptr, per_group, list);
+                       group * per_group, leg, j, 0, M.substeps, nullptr, per_group, list);
         if (!queue)
             break;
         __syncthreads();

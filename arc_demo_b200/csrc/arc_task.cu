@@ -1083,8 +1083,9 @@ k_task_rows(TaskState S, TaskOut O, const int* __restrict__ ids, int first, int 
 //   kPhysics      the step alone (arc_sim_step, the separate env step, tiles
 //                 of substeps);
 //   kWithTask     each CTA steps a group of 32 worlds, then, before its next
-//                 group, runs the task layer on them (task_group); the ended worlds go to the ended-world list, which a separate
-//                 reset launch then takes;
+//                 group, runs the task layer on them (task_group); the ended
+//                 worlds go to the ended-world list, which a separate reset
+//                 launch then takes;
 //   kWithResets   the same, and the group's ended worlds are reset in the
 //                 kernel too, one after the other by the whole CTA.
 // The task functions are compiled once (not inlined) and called both from
@@ -1122,11 +1123,6 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
     ControlSmem& cs = *reinterpret_cast<ControlSmem*>(smem_raw);
     const int tid = threadIdx.x, leg = tid / wl::kWorlds, j = tid % wl::kWorlds;
     const int n_groups = (n_items + per_group - 1) / per_group;
-    auto world_of = [&](int item) {
-        const int w = item < n_items ? (ids ? ids[item] : item) : -1;
-        return w >= 0 && w < W.n ? w : -1;
-    };
-    (void)world_of;  // the physics-only form takes no task work
     // with a queue every group, the first included, is taken from it: a CTA
     // that becomes resident only when others leave finds the queue empty
     // instead of holding back a group of its own
@@ -1140,10 +1136,11 @@ k_control_step(const __grid_constant__ DevModel<float> M, const __grid_constant_
 #pragma unroll 1
     for (int group = first; group < n_groups;) {
         wl::step_group(wl::CtaSync{}, cs.step, M, W, A, spill, spill_per_lane, lane_cap, ids, n_items,
-                       group * per_group, tid, leg, j, sub0, sub1, tile_q, per_group, list);
+                       group * per_group, leg, j, sub0, sub1, tile_q, per_group, list);
         if constexpr (kMode != kPhysics) {
             // arc/task.py:155-259
-            const int world = world_of(group * wl::kWorlds + j);
+            const int at = group * wl::kWorlds + j, item = at < n_items ? (ids ? ids[at] : at) : -1;
+            const int world = item < W.n ? item : -1;
             __syncthreads();  // warp 0 has read the step's shared memory for the last time
             task_group<float, kTaskStepObs>(cs.task, M, W, P, S, O, A.actions32, world);
             if (tid == 0)
