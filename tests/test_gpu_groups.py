@@ -136,3 +136,52 @@ def test_split_groups_equal_whole_groups(fp64):
         s.close()
     assert np.array_equal(*states)
     assert longest > 2
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+def test_both_lists_of_a_split_leg_spill(fp64):
+    # bitwise, substep by substep. World i has the femur sphere of leg i % 4 in
+    # the corner of a pit: its floor and two walls are three contacts, one more
+    # than a split group's upper warps keep on chip, while the leg's tibia,
+    # inside the walls' columns, has as many in the same room of the spill
+    from oracle.oracle import World
+
+    n, steps, cell = 16, 3, 0.4
+    states, femurs, both = [], [0] * 4, [0] * 4
+    for record in (False, True):
+        s = Sim(n, substeps=1, fp64=fp64, cell=cell)
+        s.set_kernel(KERNEL_WARPS)
+        s._lib.arc_sim_world.restype = ctypes.POINTER(World)
+        s._lib.arc_sim_world.argtypes = [ctypes.c_void_p, ctypes.c_int]
+        s.reset(np.arange(n), np.arange(n, dtype=np.uint32), np.zeros(n))
+        state = s.get_state()
+        for i in range(n):
+            leg, sx, sy = i % 4, 1 - 2 * (i // 4 % 2), 1 - 2 * (i // 8)
+            w = s._lib.arc_sim_world(s.ptr, i).contents
+            ball = w.spheres[5 * leg + 1]
+            assert ball.body == 3 * leg + 2
+            rot = np.array(w.bodies[ball.body].rot.m).reshape(3, 3)
+            at = state[i, 13 * ball.body:][:3] + rot @ [ball.pos.x, ball.pos.y, ball.pos.z]
+            # its centre 0.3 radii from the walls at x = 0 and y = 0
+            shift = 0.3 * ball.radius * np.array([sx, sy]) - at[:2]
+            for b in range(13):
+                state[i, 13 * b: 13 * b + 2] += shift
+            heights = np.full((64, 64), at[2] + 0.05)
+            heights[(slice(32, None) if sy > 0 else slice(None, 32)), (slice(32, None) if sx > 0 else slice(None, 32))] \
+                = at[2] - 0.8 * ball.radius
+            s.set_terrain(i, heights, cell)
+        s.set_state(state)
+        s._check(s._lib.arc_sim_set_record_contacts(s.ptr, int(record)))
+        for _ in range(steps):
+            s.step(np.tile(s.default_angles, (n, 1)))
+            states.append((record, s.get_state()))
+            for i in range(n if record else 0):
+                w = s._lib.arc_sim_world(s.ptr, i).contents
+                bodies = [w.contacts[k].body for k in range(w.n_contacts)]
+                for leg in range(4):
+                    upper, lower = bodies.count(3 * leg + 2), bodies.count(3 * leg + 3)
+                    femurs[leg], both[leg] = max(femurs[leg], upper), max(both[leg], min(upper, lower))
+        s.close()
+    for a, b in zip((x for r, x in states if not r), (x for r, x in states if r)):
+        assert np.array_equal(a, b)
+    assert min(femurs) > 2 and min(both) > 2, (femurs, both)
