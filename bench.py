@@ -839,6 +839,9 @@ REF_BUILD = {"": "-O3 -march=x86-64-v3 -ffp-contract=fast -fno-math-errno -fno-t
              "_v4": "-O3 -march=x86-64-v4 -ffp-contract=fast -fno-math-errno -fno-trapping-math -fopenmp (AVX-512)"}
 
 
+NO_REFERENCE = "oracle/_ref/libarcsim_ref.so not built (needs the reference sources)"
+
+
 def reference_loop(n: int, seconds: float | None, steps: int | None, warmup: int, threads: int,
                    variant: str | None = None) -> dict:
     """The reference's OpenMP step/observe/heights (its csrc/, oracle/_ref) with
@@ -848,7 +851,7 @@ def reference_loop(n: int, seconds: float | None, steps: int | None, warmup: int
     from oracle.oracle import RefSim, fastest_ref_variant, ref_available
     from oracle.task_oracle import TaskConfig, TaskOracle
     if not ref_available():
-        raise RuntimeError("oracle/_ref/libarcsim_ref.so not built")
+        raise RuntimeError(NO_REFERENCE)
     variant = fastest_ref_variant() if variant is None else variant
     torch.set_num_threads(threads)
     sim = RefSim(n, threads=threads, variant=variant)
@@ -896,6 +899,9 @@ def cpu_baseline(seconds: float, full_n: int) -> dict:
     """The reference's path over every world of the workload (like for
     like), plus a 4,096-world sample and one thread on 1,024 worlds."""
     import torch
+    from oracle.oracle import ref_available
+    if not ref_available():
+        return {"unavailable": NO_REFERENCE}
     threads = os.cpu_count() or 1
     torch_threads = torch.get_num_threads()
     r = reference_loop(full_n, seconds, None, 1, threads)
@@ -923,6 +929,9 @@ def run_reference(args) -> dict | None:
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return None
+    from oracle.oracle import ref_available
+    if not ref_available():
+        return {"impl": "reference", "unavailable": NO_REFERENCE}
     threads = os.cpu_count() or 1
     n = args.worlds
     r = reference_loop(n, None, max(args.steps, 1), max(args.warmup, 0), threads)
