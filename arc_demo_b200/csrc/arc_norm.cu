@@ -4,8 +4,8 @@
 // Bound by memory and launches: the batch is read for its moments, and read
 // and written once to normalise it. As tensor operations the same step took
 // 55 launches (six FP64 copies of the batch among them) and 207 us of GPU
-// time at 10,007 x 195; here three launches and 25 us, with a batch in L2
-// (5.0, 6.9 and 13.3; the 40 MB read and written take 6 us at the copy rate, the
+// time at 10,007 x 195; here three launches and 30 us within a training step
+// (5.3, 7.1 and 17.9; with nothing else running 25; the 40 MB read and written take 6 us at the copy rate, the
 // rest is the FP64 arithmetic per element and launch latency):
 //   k_norm_moments  per block of rows and 256 columns: the column's mean and
 //                   sum of squared deviations from it, in FP64 and two passes

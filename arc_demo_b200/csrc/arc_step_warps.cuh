@@ -254,7 +254,7 @@ __device__ __forceinline__ int collide(P& b, const BodyK<F>& k, Ref body, const 
     // columns higher than the sphere's bottom at once: of the 9 columns that
     // a lane's spheres span in a substep 0.6 are, and testing one per
     // iteration cost a warp 22 iterations where 6 find them all (4,096
-    // worlds: 504 us against 527)
+    // worlds in CTAs of four warps: 504 us against 527)
     const bool wide = ix1 - ix0 > 1 || iy1 - iy0 > 1;
     int left = 1 | (ix1 > ix0 ? 2 : 0) | (iy1 > iy0 ? 4 : 0) | (ix1 > ix0 && iy1 > iy0 ? 8 : 0);
 #pragma unroll 1
@@ -402,10 +402,16 @@ enum : uint32_t { OP_END = 0, OP_INT, OP_JNT, OP_COL, OP_UPD, OP_DMP, OP_CVL, OP
 // the SM, of 47k cycles a substep). kListLatency fills that wait: legs 0 and
 // 1 solve their third joint and collide the femur before their damping
 // joint, leg 2 its third joint, leg 3, whose damping joint comes at once,
-// nothing. It pays while an SM holds one or two CTAs (4,096 worlds: 527 us
-// against 579; 8,000: 509 against 531); with three or four the other CTAs
-// fill the waits and the damping chain's earlier start wins (16,384 worlds:
-// 945 against 984 us), so kListThroughput leaves all of it for later.
+// nothing. It pays while an SM holds one or two CTAs of four warps (the step
+// of robots thrown about by random actions, 4,096 worlds: 405 us against 450;
+// 9,400: 508 against 533; FP64 with one, 4,096: 625 against 670, and not with
+// two, 8,000: 776 against 730); with more the other groups fill the waits and
+// the damping chain's earlier start wins (a control step of 65,536 standing
+// robots: 3.19 ms against 2.99 in aligned CTAs, 3.75 against 3.43 in CTAs of
+// one group), so kListThroughput leaves all of it for later. Most launches
+// that small are split and have lists of their own (below): kListLatency is
+// for those that cannot be (recorded contacts, tiles), for the small fused
+// ones and for the last groups of an aligned launch.
 #define ARC_LEG_HEAD(k)                                                                                        \
     ARC_OP(OP_INT, 1, 4, 0, 0), ARC_OP(OP_JNT, 0, 1, k, (k) + 1), ARC_OP(OP_JNT, 1, 2, 0, 0),                   \
         ARC_OP(OP_UPD, 1, 2, 0, 0)
@@ -498,19 +504,20 @@ struct CtaSync {
 };
 
 // AlignedSync: the CTA holds several groups that start their third joints
-// together. The step is bound by instruction fetch: its loop is larger than
-// the SM's instruction cache, and with four CTAs of one group each the 16
-// warps stream through it at 16 places (12 % of the fetches miss, and waiting
-// for instructions is the largest stall but the barriers: 1.4 of 7.8 cycles
-// per instruction at 16,384 worlds). Warps of the same leg run the same code
-// in the same order; where they run it at the same time they fetch it once. Once a substep is enough, and the third
-// joint is the best place for it (65,536 worlds 3.41 ms in CTAs of their
-// own, 3.64 four to a CTA without aligning, 3.24 aligned at leg 0's substep
-// start, 3.20 before the tibia's spheres, 3.16 before joint 3, 3.30 at both).
-// But warps that share a scheduler then have it to themselves in turns, so
-// each group's legs start at another warp (step_aligned): what the alignment
-// still gives is 2 % (65,536 worlds of another state: 2,694 us with leg k of
-// every group on one scheduler, 2,475 turned, 2,532 turned and not aligned).
+// together. The step's loop is larger than the SM's instruction cache, and in
+// four CTAs of one group each the 16 warps stream through it at 16 places.
+// Warps of the same leg run the same code in the same order; where they run
+// it at the same time they fetch it once (16,384 worlds: 97.6 % of the fetches
+// hit, not 94.4; waiting for instructions 0.35 per issue, not 0.52). A control
+// step of standing robots, in CTAs of one group / four to a CTA without the
+// aligning / aligned: 65,536 worlds 3,430 / 3,550 / 2,990 us, 16,384 of many
+// terrain sizes 984 / 1,030 / 853, FP64 16,384 2,100 / 2,020 / 1,790. Robots
+// thrown about by random actions differ too much to stay together: the step of
+// 65,536 takes 2,455 / 2,518 / 2,469 us. Once a substep is enough, and the third
+// joint is the best place for it (65,536 worlds 3.16 ms; at leg 0's substep
+// start 3.24, before the tibia's spheres 3.20, at both 3.30; not aligned 3.64).
+// Warps that share a scheduler then have it to themselves in turns, so each
+// group's legs start at another warp (step_aligned).
 //
 // Each group has four of the sixteen named barriers, one per neighbouring
 // pair of warps around the ring (0-1, 1-2, 2-3, 3-0). A pair's joint and
@@ -594,27 +601,26 @@ struct AlignedSmem {
 // How a launch over n_items worlds is split: worlds per group (one CTA's
 // lanes) and the operation list.
 //   Worlds per group. A group's time is that of the longest path over its
-// worlds' contacts, so with fewer groups than SMs smaller groups are faster:
-// 64 worlds take 353 us one per group and 408 us as two groups of 32, 1,000
-// worlds 404-418 us in groups of 7-14 and 443 us in groups of 32. Groups
-// beyond about half the SMs gain little more and crowd out what runs beside
-// the step, so the split stops there; and a launch that shares the GPU with
-// others (`alone` false) keeps groups of 32.
+// worlds' contacts, so with fewer groups than SMs smaller groups are faster,
+// up to about half as many groups as SMs (split groups, FP32: 64 worlds one
+// per group 272 us, as two groups of 32 283; 1,000 worlds in groups of 14 294,
+// of 32 305, of 7 on nearly every SM 324; FP64 399 and 408, then 438, 433 and
+// 533; in CTAs of four warps 64: 322 and 353, 1,000: 367 and 386). More also
+// crowd out what runs beside the step, so the split stops there; and a launch
+// that shares the GPU with others (`alone` false) keeps groups of 32.
 //   Operation list: kListLatency up to two groups per SM in FP32, up to one
-// in FP64, whose SMs hold two (4,096 worlds: 758 us against 848; 7,000:
-// 1,119 against 1,069).
+// in FP64, whose SMs hold two (the figures are at the lists above).
 //   Split groups (SplitSync) up to two groups per SM in FP32, one in FP64
-// (FP32, one group per CTA of four warps and split: 1 world 298 and 256 us, 64:
-// 320 and 272, 1,000: 367 and 293, 4,096: 405 and 350, 6,000: 456 and 441,
-// 9,400: 500 and 477; FP64, 1: 458 and 378, 4,096: 621 and 565), where a whole
-// control step runs in one launch, no list can reach the reference's cap and
-// nobody records contacts.
+// (FP32, CTAs of four warps and split: 1 world 292 and 257 us, 64: 322 and
+// 272, 1,000: 367 and 294, 4,096: 405 and 349, 6,000: 459 and 437, 9,400: 504
+// and 485; FP64, 1: 445 and 377, 4,096: 632 and 565), where a whole control
+// step runs in one launch, no list can reach the reference's cap and nobody
+// records contacts.
 //   Aligned CTAs (AlignedSync) take a work queue and a whole SM each, so not
-// beside others, and all that is more than split groups take (10,007 worlds:
-// 555 us in CTAs of their own, 546 aligned; 12,000: 584 and 565; 16,384: 950
-// and 672; FP64 7,000: 777 and 732; 9,400: 831 and 761). They run
-// kListThroughput (a control step of 65,536 standing robots 2,835 us, in
-// kListLatency 2,905; thrown-about ones, 2,472 and 2,425, like it less).
+// beside others, and all that is more than split groups take (a training step
+// of 10,007 standing robots: 843 us in CTAs of their own, 828 aligned; FP64,
+// thrown-about robots, 7,000: 781 and 733, 9,400: 832 and 762; larger ones at
+// AlignedSync). They run kListThroughput.
 struct GroupPlan {
     int per_group, groups, list;
     bool aligned, split;
@@ -1137,8 +1143,9 @@ __device__ __forceinline__ void step_split(SplitSmem& sm, const DevModel<F>& M, 
 //
 // What is left over from whole waves of slots runs on SMs that are emptying:
 // up to kAligned / 2 groups per SM it takes the latency list, and fewer worlds
-// than one group per SM are split into as many groups as SMs (20,000 worlds,
-// 33 groups more than one wave: 1,524 us without either, 1,458 with the list).
+// than one group per SM are split into as many groups as SMs (the step of
+// 20,000 thrown-about robots, 33 groups more than one wave: 1,160 us without
+// either, 1,145 with; 25,000: 1,260 and 1,231; 65,536: 2,505 and 2,469).
 __device__ __forceinline__ void step_aligned(AlignedSmem& as, const DevModel<F>& M, const Worlds<F>& W,
                                              const Actuation& A, F* __restrict__ spill, int spill_per_lane,
                                              int lane_cap, const int* __restrict__ ids, int n_items, int* queue,
@@ -1146,8 +1153,9 @@ __device__ __forceinline__ void step_aligned(AlignedSmem& as, const DevModel<F>&
 {
     // each group's legs start at another warp: warps 4 apart share a scheduler,
     // and with leg k of every group on the same one, that scheduler had the
-    // chain's four joints to issue at once while the others waited (16,384
-    // worlds 740 -> 674 us, 65,536 2,694 -> 2,475; FP64 16,384 1,505 -> 1,398)
+    // chain's four joints to issue at once while the others waited (thrown-about
+    // robots, 16,384 worlds 740 -> 674 us, 65,536 2,694 -> 2,475; FP64 16,384
+    // 1,505 -> 1,398)
     const int tid = threadIdx.x % kThreads, slot = threadIdx.x / kThreads, j = tid % kWorlds;
     const int leg = (tid / kWorlds + slot * (kWarps / kAligned)) % kWarps;
     const int grid = gridDim.x, whole = n_items / (kAligned * grid * kWorlds) * kAligned * grid;  // groups

@@ -7,9 +7,9 @@
 // k of each. Its bodies, anchors and contact records take twice the shared
 // memory of the FP32 step (109 KB per CTA), so two CTAs share an SM, and
 // each thread may use up to 255 registers; with more than one group per SM the
-// two run aligned in one CTA (wl::AlignedSync: 16,384 worlds 2,123 -> 1,839
-// us, and turned on the warps, from another state, 1,505 -> 1,400), with fewer
-// a group runs on eight warps (wl::SplitSync).
+// two run aligned in one CTA (wl::AlignedSync: a control step of 16,384
+// standing robots 2,100 -> 1,790 us), with fewer a group runs on eight warps
+// (wl::SplitSync).
 // The whole control step runs in one launch (no substep tiles).
 #define ARC_WARPS_FP64
 #include "arc_step_warps.cuh"

@@ -452,8 +452,8 @@ template <class R> struct TaskSmem {
 // lane, and divided twice; a warp per world keeps its offsets in registers
 // and has five samples in flight per lane (a thread per sample, with the
 // frame read from shared memory for each, took 70k cycles against 25k). Both
-// together: 65,536 worlds 205 -> 99 us, 4,096 48 -> 19 us, FP64 16,384 78 ->
-// 34 us; the observation alone of one world 42 -> 9 us.
+// together: 65,536 worlds 205 -> 98 us, 4,096 48 -> 18 us, FP64 16,384 78 ->
+// 33 us; the observation alone of one world 42 -> 9 us.
 template <class R, int kMode>
 __device__ __noinline__ void task_group(TaskSmem<R>& ts, const DevModel<R>& M, const Worlds<R>& W, const TaskParams& P,
                                         const TaskState& S, const TaskOut& O, const float* __restrict__ actions,
@@ -624,8 +624,8 @@ k_task(const __grid_constant__ DevModel<R> M, Worlds<R> W, const __grid_constant
 // one lane runs once costs most in fetching it: the task state and
 // observation of a new world by one thread took 46k cycles.) The reset of
 // the 470 worlds that end in a step of 65,536: 217 -> 33 us; of 26 in one of
-// 4,096: 200 -> 28 us; of 16,384 worlds at once 2,001 -> 543 us (268 MB of
-// terrain written: 41 us at the copy rate), bound by instruction issue (59 %
+// 4,096: 200 -> 26 us; of 16,384 worlds at once 2,001 -> 514 us (268 MB of
+// terrain written: 41 us at the copy rate), bound by instruction issue (57 %
 // of cycles) and the barriers between the phases.
 
 constexpr int kResetThreads = 128;
@@ -1091,12 +1091,14 @@ k_task_rows(TaskState S, TaskOut O, const int* __restrict__ ids, int first, int 
 // The task functions are compiled once (not inlined) and called both from
 // the fused forms and from the separate task kernels, so their outputs do
 // not depend on the form. The physics is inlined into each instantiation:
-// the physics-only one then holds no task code, gets the registers it needs
-// without spills (126, against 128 and spills when the task code shares the
-// kernel) and steps 6 % faster; the fused instantiations compile the same
+// the physics-only one then holds no task code and gets the registers it needs
+// without spills (127; one kernel for every form took 128 with spills and
+// stepped 6 % slower); the fused instantiations compile the same
 // physics source in another context and agree with it to FP32 rounding
-// rather than bit for bit. The ended-world list is filled in completion
-// order, as the separate task kernel fills it.
+// rather than bit for bit, and are 9-10 % slower (65,536 worlds, policy
+// included: 3.03 ms, 3.34 with the task, 3.31 with the resets too). The
+// ended-world list is filled in completion order, as the separate task kernel
+// fills it.
 static_assert(kResetThreads == wl::kThreads, "the fused form's CTA resets worlds");
 enum : int { kPhysics = 0, kWithTask = 1, kWithResets = 2 };
 

@@ -65,9 +65,9 @@ class DeviceVecEnv:
         self.sim.set_kernel(kernel, worlds_per_cta)
 
     def set_fused(self, mode: int) -> None:
-        """With the warp-per-leg kernel: 0 the step kernel, then the task,
-        heights and reset kernels; 1 the step and the task layer fused per
-        group of 32 worlds, the resets after; 2 the resets fused too (one
+        """With the warp-per-leg kernel: 0 the step kernel, then the task and
+        reset kernels; 1 the step and the task layer fused per group of 32
+        worlds, the resets after; 2 the resets fused too (one
         launch per control step). Forms 1 and 2 agree with form 0 to FP32
         rounding (their physics is compiled into their own kernel)."""
         self.sim._check(self.gpu.lib.arc_env_set_fused(self.sim.ptr, int(mode)))

@@ -57,11 +57,11 @@ RENDER_METRIC = "frames/s at 640x360, 4 samples per pixel"
 RENDER_WORLDS = 256
 RENDER_W, RENDER_H, RENDER_SAMPLES = 640, 360, 4
 # Work and DRAM traffic of k_render per frame of this workload, from one ncu
-# capture of a 16-frame launch: 786.8 M warp instructions, 1.58 MB read +
-# 76.73 MB written, over 16 frames. The kernel is bound by instruction issue
+# capture of a 16-frame launch: 683.1 M warp instructions, 1.65 MB read +
+# 61.00 MB written, over 16 frames. The kernel is bound by instruction issue
 # (4 warp instructions per SM per cycle).
-RENDER_WARP_INST_PER_FRAME = 786.831e6 / 16
-RENDER_DRAM_BYTES_PER_FRAME = (1.5777e6 + 76.7283e6) / 16
+RENDER_WARP_INST_PER_FRAME = 683.050e6 / 16
+RENDER_DRAM_BYTES_PER_FRAME = (1.6502e6 + 60.9956e6) / 16
 
 
 def parse():
@@ -241,7 +241,7 @@ def autotune(env, torch, stream,
     return best, table
 
 
-FORMS = {0: "step kernel, then task, heights and reset kernels",
+FORMS = {0: "step kernel, then task and reset kernels",
          1: "step and task layer fused per group of 32 worlds, then the reset kernel",
          2: "step, task layer and resets fused: one launch per control step"}
 
@@ -253,8 +253,8 @@ def autotune_parts(env, torch, stream, one_step,
     form). Ranges 1: the policy, then env.step() as one CUDA graph; 2, 4, 8: the
     worlds in that many ranges on their own streams (DeviceVecEnv.step_parts),
     each range's policy then its step. Forms (DeviceVecEnv.set_fused): 0 the
-    step kernel, then the task, heights and reset kernels; 1 the step and the
-    task layer fused per group of 32 worlds, then the reset kernel; 2 the
+    step kernel, then the task and reset kernels; 1 the step and the task
+    layer fused per group of 32 worlds, then the reset kernel; 2 the
     resets fused too."""
     table = {}
     stream.synchronize()
@@ -450,7 +450,7 @@ def run_ours(args) -> dict | None:
             plain = {"ms_per_step": round(plain_ms, 3), "env_steps_per_s": round(n / plain_ms * 1e3),
                      "step_kernel_ms": round(plain_kernel_ms, 3), "step_order": plain_order,
                      "loop": "the same policy and env.step() graph with the plain per-world kernel (one thread "
-                             "per world) and the separate task, heights and reset kernels; the loop and the "
+                             "per world) and the separate task and reset kernels; the loop and the "
                              "kernel each in the faster of the two step orders"}
             apply_candidate(env, best_wpc)
 
@@ -490,8 +490,8 @@ def run_ours(args) -> dict | None:
     form = form if cand.startswith("warps") else 0  # the fused forms need the warp-per-leg kernel
     # our launches per control step and range: the step order's two kernels
     # (with the warp-per-leg kernel), then the step, task and reset kernels
-    # (form 0), the fused step and the reset kernel (1), the fused step alone (2); the ranges' merge; the memset of the ended-world count
-    # is not a kernel
+    # (form 0), the fused step and the reset kernel (1), the fused step alone
+    # (2); the ranges' merge; the memset of the ended-world count is no kernel
     per_part = {0: 3, 1: 2, 2: 1}[form] + (2 if cand.startswith(("warps", "tile")) else 0)
     launches = (per_part * parts + (1 if parts > 1 else 0)) * K
     out = {
@@ -691,7 +691,7 @@ def leg_uneven_ou(torch, n=4096, steps=300, warmup=20) -> dict:
             "latency_ms": {"p50": round(float(np.percentile(lat, 50)), 4),
                            "p99": round(float(np.percentile(lat, 99)), 4), "max": round(float(lat.max()), 4)},
             "ended_in_last_step": ended,
-            "loop": "OU actions on the device, then DeviceVecEnv.step() (one CUDA graph: step, task, heights, "
+            "loop": "OU actions on the device, then DeviceVecEnv.step() (one CUDA graph: step, task, "
                     "reset of ended worlds)"}
 
 
@@ -791,7 +791,7 @@ def leg_fp64(torch, n, steps=6, warmup=3) -> dict:
             "control_step_ms": round(step_ms / steps, 4),
             "env_steps_per_s_control_step": round(n * steps / (step_ms * 1e-3), 1),
             "note": "actions fixed (uniform random); every kernel from the same states 3 steps after a reset; "
-                    "control step = step, task, heights, reset in one graph"}
+                    "control step = step, task, reset in one graph"}
 
 
 def leg_serving(seconds=3.0, clients=8, rates=(200.0, 50.0), tick_cap=131072) -> dict:

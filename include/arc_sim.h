@@ -310,10 +310,9 @@ int arc_env_step_ids(arc_sim *s, const int *d_ids, int n_ids, void *stream);
 
 /* How the env's control step (arc_env_step, arc_env_step_part,
  * arc_env_step_host, arc_env_step_ids) runs with the warp-per-leg kernel:
- * 0 (the default) the step kernel, then the task, heights and reset kernels;
- * 1 each group of 32 worlds stepped and then given its rewards,
- * observations and heights in the same kernel, the ended worlds reset by the
- * reset kernel after it; 2 the ended worlds reset in that kernel too (one
+ * 0 (the default) the step kernel, then the task and reset kernels; 1 each
+ * group of 32 worlds stepped and then given its rewards and observations in
+ * the same kernel, the ended worlds reset by the reset kernel after it; 2 the ended worlds reset in that kernel too (one
  * launch per control step). The task layer's results are the same in all
  * three; the physics of forms 1 and 2 is compiled into their own kernel and
  * agrees with form 0's to FP32 rounding (form 0, the fastest, keeps the
