@@ -198,7 +198,8 @@ int arc_sim_step_ids(arc_sim *s, const int *d_ids, int n_ids, const double *d_ta
 int arc_sim_observe_ids(const arc_sim *s, const int *d_ids, int n_ids, double *root, double *rot, double *joints,
                         double *contacts, int *flags, void *stream);
 /* on != 0: the warp-per-leg kernel runs one wave of resident CTAs that take
- * groups of 32 worlds from a device work queue, instead of one CTA per group */
+ * groups of 32 worlds from a device work queue, instead of one CTA per group
+ * (and large launches CTAs of several groups that run aligned, one per SM) */
 int arc_sim_set_work_queue(arc_sim *s, int on);
 /* Substep tiling of the FP32 warp-per-leg kernel: tile in 1 .. substeps - 1 runs
  * each control step as launches of `tile` substeps, the state going through
